@@ -37,7 +37,7 @@ UNITS = [
     ('mpsw_tiles.cpp', ['--fmad=false', '-x', 'cu']),
 ]
 HEADERS = ['mpsw_internal.h', 'mpsw_kernels.cuh', 'mpsw_launch.h', 'mpsw_launch.cuh', 'mpsw_members.cuh',
-           'mpsw_fused.cuh', 'mpsw_setup.h', 'mpsw_tiles.h', 'mpsw_engine.h']
+           'mpsw_fused.cuh', 'mpsw_stage.h', 'mpsw_stage.cuh', 'mpsw_setup.h', 'mpsw_tiles.h', 'mpsw_engine.h']
 
 
 def _nvcc():

@@ -408,6 +408,7 @@ void Engine::free_device_mesh() {
   mesh_built = false;
   fused = FusedDev();
   fused_K = 0;
+  st64 = st32 = StageDev();
 }
 
 // Halo tiles of the fused FP32 member stages (meshes with at most 6 edges per cell and 10
@@ -450,6 +451,35 @@ void Engine::build_fused() {
   cuda_check(Launch<float, double>::fused_prepare(fused), "fused stage shared-memory limit");
   fused.ok = true;
   fused_K = K;
+}
+
+// Halo tiles of the nonlinear stage, while the tiles' blobs (2.7 times the mesh: halo entities are
+// packed with every tile that reads them) stay in the 126 MB L2 between stages: 2.3 KB a cell in
+// FP64, 1.2 KB in FP32.  Measured us a stage, tiles against grid-wide passes: level 3 5.1 / 16.6
+// (FP64) 3.9 / 12.6 (FP32), level 5 7.4 / 18.6 and 5.5 / 14.5, level 6 21.7 / 25.7 and 12.9 / 18.0;
+// level 7, beyond the line, 93.7 / 66.8 and 63.2 / 49.9.  Tiles own as many cells as give each of
+// the 148 SMs one, on meshes for which that is fewer than the layers' caps allow.
+// MPSW_STAGE_TILES=0 keeps the passes.
+void Engine::build_stage() {
+  constexpr size_t kL2 = (size_t)110 << 20;
+  st64 = st32 = StageDev();
+  const char *off = getenv("MPSW_STAGE_TILES");
+  if ((off && atoi(off) == 0) || (size_t)nC * 1200 > kL2) return;
+  const int share = std::max(8, (nC + 147) / 148);
+  StageSetHost t;
+  if (!build_stage_tiles(bm, share < 60 ? share : 128, &t).empty()) return;
+  const int *cnt = up<int>(t.cnt, mesh_bufs);
+  for (int p = 0; p < 2; p++) {
+    const std::vector<unsigned char> &blob = p ? t.blob32 : t.blob64;
+    if (blob.size() > kL2) continue;
+    StageDev &d = p ? st32 : st64;
+    d.ntiles = t.ntiles;
+    d.cnt = cnt;
+    d.blob_off = up<long long>(p ? t.off32 : t.off64, mesh_bufs);
+    d.blob = up<unsigned char>(blob, mesh_bufs);
+  }
+  cuda_check(Launch<double, double>::stage_prepare(), "nonlinear stage shared-memory limit");
+  cuda_check(Launch<float, double>::stage_prepare(), "nonlinear stage shared-memory limit");
 }
 
 RefMesh Engine::ref_mesh() {
@@ -518,6 +548,7 @@ void Engine::build_device_mesh() {
   d_perm[2] = up<int>(bm.perm_v, mesh_bufs);
   cuda_check(cudaGetDevice(&mesh_device), "cudaGetDevice");
   build_fused();
+  build_stage();
   noalloc_prepare_device();
   mesh_built = true;
   mesh_dirty = false;
@@ -663,8 +694,31 @@ void Engine::fwd_diag(const double *u, const double *h, const Diag<double> &d, c
   if (ph.visc4 > 0) L64::del4_vc(m64, 1, d.dsq_u, d.dsq_vort, d.dsq_div, stream);
 }
 
+// One nonlinear stage: a kernel over halo tiles that writes the linearisation point to `out`, or
+// where the mesh has no tiles the grid-wide passes, which leave it in d.
+//
+// Beside the members of an overlapped sweep the tiles are taken only while they are at most two a
+// SM: their blocks hold half an SM's registers each, and on larger meshes cost the member kernels
+// more than the passes do (level 6, 8 FP64 members: sweep pair 6.5 ms with tiles, 6.0 without;
+// level 5, 64 FP32 members: 6.7 against 6.85 ms).
+bool Engine::stage_tiled() const { return st64.ntiles > 0 && (!beside_members || st64.ntiles <= 2 * 148); }
+
+static StageBaseOut base_out(const Diag<double> &d) {  // (u is the stage's input itself)
+  StageBaseOut o{};
+  o.d[SO_HE] = d.he; o.d[SO_V] = d.v; o.d[SO_GPT] = d.gpt; o.d[SO_GPN] = d.gpn; o.d[SO_PE] = d.pe;
+  o.d[SO_VORT] = d.vort; o.d[SO_HV] = d.hv; o.d[SO_KE] = d.ke;
+  o.on = 1;
+  return o;
+}
+
 void Engine::fwd_stage(const double *u, const double *h, const Diag<double> &d, const Phys<double> &ph,
-                       const RK<double, double> &rku, const RK<double, double> &rkh, double *tu, double *th) {
+                       const RK<double, double> &rku, const RK<double, double> &rkh, double *tu, double *th,
+                       const StageBaseOut &out) {
+  if (stage_tiled()) {
+    L64::stage(st64, StageArgs<double, double>{u, h, 0.0, ph, rku, rkh, tu, th, out, m64.e_sc2, m64.e_sc4, m64.e_usrc},
+               stream);
+    return;
+  }
   L64::fwd_vertex(m64, u, h, 0.0, d, stream);
   L64::fwd_cell(m64, d_cnb, u, h, 0.0, d, rkh, th, stream);
   L64::fwd_edge_diag(m64, u, h, 0.0, d, ph, stream);
@@ -836,7 +890,10 @@ void Engine::rk4(int nsteps) {  // src/mpas_sw_module.f90:528-635
       const double *hi = k == 0 ? h0 : sp_h[k - 1];
       RK<double, double> ru{u0, k == 0 ? u0 : acc_u, k == 3 ? u0 : acc_u, k < 3 ? sp_u[k] : nullptr, c[k], w[k], 0.0, ph.tc1};
       RK<double, double> rh{h0, k == 0 ? h0 : acc_h, k == 3 ? h0 : acc_h, k < 3 ? sp_h[k] : nullptr, c[k], w[k], 0.0, 0};
-      fwd_stage(ui, hi, stage[0], ph, ru, rh, k == 3 ? dv("tend_u") : nullptr, k == 3 ? dv("tend_h") : nullptr);
+      StageBaseOut so{};
+      if (adv) so.d[SO_HE] = stage[0].he;
+      so.on = adv;
+      fwd_stage(ui, hi, stage[0], ph, ru, rh, k == 3 ? dv("tend_u") : nullptr, k == 3 ? dv("tend_h") : nullptr, so);
       // after the stage: its h_edge is in stage[0], the next provisional h in sp_h[k] and, in
       // stage 4, the new h in h0
       if (adv)
@@ -904,6 +961,12 @@ void Engine::forward(int prec, int nsteps) {
       const float *ui = s32_u[k], *hi = s32_h[k];
       RK<float, double> ru{u0, k == 0 ? u0 : acc_u, k == 3 ? u0 : acc_u, k < 3 ? s32_u[k + 1] : nullptr, c[k], w[k], 0.f, ph.tc1};
       RK<float, double> rh{h0, k == 0 ? h0 : acc_h, k == 3 ? h0 : acc_h, k < 3 ? s32_h[k + 1] : nullptr, c[k], w[k], offf, 0};
+      if (st32.ntiles > 0) {
+        L32::stage(st32, StageArgs<float, double>{ui, hi, offf, ph, ru, rh, nullptr, nullptr, StageBaseOut{}, m32.e_sc2,
+                                                 m32.e_sc4, m32.e_usrc},
+                   stream);
+        continue;
+      }
       L32::fwd_vertex(m32, ui, hi, offf, d32, stream);
       L32::fwd_cell(m32, d_cnb, ui, hi, offf, d32, rh, nullptr, stream);
       L32::fwd_edge_diag(m32, ui, hi, offf, d32, ph, stream);
@@ -947,7 +1010,8 @@ void Engine::rk4_tlm(int nsteps) {  // src/mpas_sw_module.f90:637-781
       const double *hi = k == 0 ? h0 : sp_h[k - 1];
       RK<double, double> ru{u0, k == 0 ? u0 : acc_u, k == 3 ? u0 : acc_u, k < 3 ? sp_u[k] : nullptr, c[k], w[k], 0.0, ph.tc1};
       RK<double, double> rh{h0, k == 0 ? h0 : acc_h, k == 3 ? h0 : acc_h, k < 3 ? sp_h[k] : nullptr, c[k], w[k], 0.0, 0};
-      fwd_stage(ui, hi, stage[0], ph, ru, rh, k == 3 ? dv("tend_u") : nullptr, k == 3 ? dv("tend_h") : nullptr);
+      fwd_stage(ui, hi, stage[0], ph, ru, rh, k == 3 ? dv("tend_u") : nullptr, k == 3 ? dv("tend_h") : nullptr,
+                base_out(stage[0]));
       const Base<double> bs = base_of(stage[0], ui);
       const double *uti = k == 0 ? ut0 : tp_u[k - 1];
       const double *hti = k == 0 ? ht0 : tp_h[k - 1];
@@ -1023,7 +1087,7 @@ void Engine::rk4_adj() {  // src/mpas_sw_module.f90:783-1002
     const double *hi = k == 0 ? h0 : sp_h[k - 1];
     RK<double, double> ru{u0, k == 0 ? u0 : acc_u, acc_u, k < 3 ? sp_u[k] : nullptr, c[k], w[k], 0.0, ph.tc1};
     RK<double, double> rh{h0, k == 0 ? h0 : acc_h, acc_h, k < 3 ? sp_h[k] : nullptr, c[k], w[k], 0.0, 0};
-    fwd_stage(ui, hi, stage[k + 1], ph, ru, rh, nullptr, nullptr);
+    fwd_stage(ui, hi, stage[k + 1], ph, ru, rh, nullptr, nullptr, base_out(stage[k + 1]));
   }
   cuda_check(cudaMemcpyAsync(u2, ph.tc1 ? u0 : acc_u, sizeof(double) * nE, cudaMemcpyDeviceToDevice, stream), "u(2)");
   cuda_check(cudaMemcpyAsync(h2, acc_h, sizeof(double) * nC, cudaMemcpyDeviceToDevice, stream), "h(2)");

@@ -72,6 +72,8 @@ struct Window {
   std::vector<long long> bin_cost;
   std::vector<int> bin_split;
   long long forward_steps = 0;  // trajectory steps recomputed by the last adjoint sweep
+  int store_now = 0;          // precisions the forward being launched stores (bit 0 FP64, bit 1 FP32)
+  Phys<double> forward_phys{}; // physics of the forward sweep that wrote the checkpoints
   int store_mode = -1;        // -1 automatic, else a mask of the precisions to store
   double store_budget = 0;    // bytes for automatic mode (0: 40% of free device memory)
   // member buffers per precision (0 FP64, 1 FP32), allocated for the largest B seen
@@ -132,6 +134,9 @@ struct Engine {
   FusedDev fused;              // halo tiles and coefficients of the fused member stages
   int fused_K = 0;             // owned cells per tile of `fused` (0: not built)
   void build_fused();
+  StageDev st64, st32;         // halo tiles of the nonlinear stage, FP64 and FP32 stencils
+  void build_stage();
+  bool beside_members = false; // the nonlinear stages being launched run beside member kernels
 
   // work
   std::vector<void *> work;
@@ -195,7 +200,9 @@ struct Engine {
   void tracers_download(const double *src, const double *tend);
   void fwd_diag(const double *u, const double *h, const Diag<double> &d, const Phys<double> &ph);
   void fwd_stage(const double *u, const double *h, const Diag<double> &d, const Phys<double> &ph,
-                 const RK<double, double> &rku, const RK<double, double> &rkh, double *tu, double *th);
+                 const RK<double, double> &rku, const RK<double, double> &rkh, double *tu, double *th,
+                 const StageBaseOut &out);
+  bool stage_tiled() const;
   void tl_diag_run(const Base<double> &bs, const double *ut, const double *ht, const Diag<double> &d,
                    const Phys<double> &ph);
   void check_launch(const char *what);
@@ -233,8 +240,8 @@ struct Engine {
   void window_store_alloc(int nsteps);
   void window_store_free(int prec);
   void window_capture_state(cudaStream_t s);
-  void window_forward();
-  void window_ensure();
+  void window_forward(int stores);
+  void window_ensure(int prec);
   void window_tl(int prec, int B, double *du, double *dh, cudaStream_t s);
   void window_ad(int prec, int B, double *au, double *ah, cudaStream_t s);
   void window_final(double *u, double *h, cudaStream_t s);

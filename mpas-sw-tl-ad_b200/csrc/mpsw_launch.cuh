@@ -12,6 +12,7 @@
 #include "mpsw_launch.h"
 #include "mpsw_fused.cuh"
 #include "mpsw_members.cuh"
+#include "mpsw_stage.cuh"
 
 namespace mpsw {
 
@@ -186,6 +187,17 @@ void Launch<R, A>::fwd_edge_tend(const MeshDev<R> &m, const R *u, const R *h, R 
   g_launches++;
   if (sizeof(R) == 4 && !d.v) throw std::invalid_argument("FP32 fwd_edge_tend needs the PV-flux rows in d.v");
   MPSW_BDISPATCH(m, launch_k(k_fwd_edge_tend<R, A, NB::e2>, launch_cfg(m.nE), s, m, u, h, off, d, ph, rk, tend_u));
+}
+template <typename R, typename A>
+void Launch<R, A>::stage(const StageDev &ts, const StageArgs<R, A> &a, cudaStream_t s) {
+  g_launches++;
+  const size_t smem = stage_smem<R>(a.ph.visc2 > R(0) || a.ph.visc4 > R(0), a.ph.visc4 > R(0));
+  launch_k(k_stage<R, A>, LaunchCfg{ts.ntiles, kStageThreads, smem}, s, ts, a);
+}
+template <typename R, typename A>
+cudaError_t Launch<R, A>::stage_prepare() {
+  return cudaFuncSetAttribute((const void *)k_stage<R, A>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)stage_smem<R>(true, true));
 }
 template <typename R, typename A>
 void Launch<R, A>::tracer_stage(const MeshDev<R> &m, const int *c_nb, int nT, const R *u, const R *he,

@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 
 #include "mpsw_internal.h"
+#include "mpsw_stage.h"
 
 namespace mpsw {
 
@@ -53,6 +54,9 @@ struct Launch {
   static void del4_vc(const MeshDev<R> &m, int B, const R *dsq_u, R *dsq_vort, R *dsq_div, cudaStream_t s);
   static void fwd_edge_tend(const MeshDev<R> &m, const R *u, const R *h, R off, const Diag<R> &d,
                             const Phys<R> &ph, const RK<R, A> &rk, R *tend_u, cudaStream_t s);
+  // a whole nonlinear stage on halo tiles (mpsw_stage.cuh), and its shared-memory limit
+  static void stage(const StageDev &ts, const StageArgs<R, A> &a, cudaStream_t s);
+  static cudaError_t stage_prepare();
   static void tend_h(const MeshDev<R> &m, const R *u, const R *he, R *out, cudaStream_t s);
   static void tracer_stage(const MeshDev<R> &m, const int *c_nb, int nT, const R *u, const R *he, const R *tr_in,
                            R *tr0, const R *h0, const R *h_next, R *tend, R *acc, R *tr_next, R c, R w, int first,

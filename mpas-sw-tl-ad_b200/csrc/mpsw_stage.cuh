@@ -1,0 +1,184 @@
+// One nonlinear RK stage as one kernel over halo tiles (layout and arithmetic: mpsw_stage.h).
+//
+// A single trajectory is bound by latency: run as four grid-wide passes (vertices, cells, edge
+// diagnostics, edge tendencies) a stage cost 4.5 us a pass on the level-5 mesh whatever the
+// pass computed, launch, ramp-up and a chain of index -> value loads from L2.  Here a block
+// computes the whole stage for its tile: the passes become phases separated by block barriers,
+// their indirect loads go to shared memory, and the halo is recomputed (about 1.7 times the owned
+// edges) instead of exchanged through another launch.  The blob is mesh data, which no kernel
+// writes, so fetching it runs before the wait for the previous stage and overlaps that stage; the
+// next stage's blocks are let in at once for the same reason.
+#pragma once
+
+#include "mpsw_fused.cuh"
+#include "mpsw_stage.h"
+
+namespace mpsw {
+
+// Records of a tile in shared memory, after the work values: rows of a section's capacity, so that
+// every address but the entity's is a constant.
+template <typename R>
+struct StageShared {
+  static constexpr int row(int cap, int vals) { return 16 * cap * (1 + (vals * (int)sizeof(R) + 15) / 16); }
+  static constexpr int V = 0, CM = V + row(kCapVA, kValsV), CX = CM + row(kCapCM, kValsCM),
+                       CK = CX + row(kCapCM, kValsCX), CO = CK + row(kCapCK, kValsCK), END = CO + row(kCapCO, 0);
+  // chunk rows of the sections, in the order V CM CX CK CO
+  static constexpr int rows(int vals) { return 1 + (vals * (int)sizeof(R) + 15) / 16; }
+  static constexpr int RV = rows(kValsV), RCM = RV + rows(kValsCM), RCX = RCM + rows(kValsCX),
+                       RCK = RCX + rows(kValsCK), RCO = RCK + 1;
+  static_assert(RCO <= 32, "one lane of a warp copies each chunk row");
+};
+template <typename R>
+inline size_t stage_smem(bool visc, bool del4) {
+  return (size_t)stage_work((int)sizeof(R), visc, del4) + StageShared<R>::END;
+}
+
+__device__ __forceinline__ unsigned smem_addr(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
+
+template <typename R, typename A>
+__global__ void __launch_bounds__(kStageThreads, 2) k_stage(StageDev ts, StageArgs<R, A> a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ __align__(8) unsigned long long arrived;
+  using S = StageShared<R>;
+  constexpr int NT = kStageThreads;
+  const int tid = threadIdx.x;
+  const bool del4 = a.ph.visc4 > R(0), visc = del4 || a.ph.visc2 > R(0);
+  unsigned char *const w = smem_raw, *const rec = smem_raw + stage_work((int)sizeof(R), visc, del4);
+  int n[kStageCounts], off[kStageSections];
+#pragma unroll
+  for (int k = 0; k < kStageCounts; k++) n[k] = __ldg(ts.cnt + (size_t)blockIdx.x * kStageCounts + k);
+  stage_layout(n, (int)sizeof(R), off);
+  const unsigned char *g = ts.blob + __ldg(ts.blob_off + blockIdx.x);
+  if (tid < 32) {  // one bulk copy per chunk row of the records
+    const int ncx = visc ? n[S_CM] : n[S_CO];
+    if (tid == 0) {
+      asm volatile("mbarrier.init.shared.b64 [%0], 1;" ::"r"(smem_addr(&arrived)) : "memory");
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+      const int bytes = 16 * (S::RV * n[S_VA] + (S::RCM - S::RV) * n[S_CM] + (S::RCX - S::RCM) * ncx +
+                              (S::RCK - S::RCX) * n[S_CK] + n[S_CO]);
+      asm volatile("mbarrier.arrive.expect_tx.shared.b64 _, [%0], %1;" ::"r"(smem_addr(&arrived)), "r"(bytes)
+                   : "memory");
+    }
+    __syncwarp();
+    if (tid < S::RCO) {
+      const int k = tid < S::RV ? 0 : tid < S::RCM ? 1 : tid < S::RCX ? 2 : tid < S::RCK ? 3 : 4;
+      const int first = k == 0 ? 0 : k == 1 ? S::RV : k == 2 ? S::RCM : k == 3 ? S::RCX : S::RCK;
+      const int cnt = k == 0 ? n[S_VA] : k == 1 || k == 2 ? n[S_CM] : k == 3 ? n[S_CK] : n[S_CO];
+      const int cap = k == 0 ? kCapVA : k == 1 || k == 2 ? kCapCM : k == 3 ? kCapCK : kCapCO;
+      const int dst = k == 0 ? S::V : k == 1 ? S::CM : k == 2 ? S::CX : k == 3 ? S::CK : S::CO;
+      const int src = k == 0 ? off[SB_V] : k == 1 ? off[SB_CM] : k == 2 ? off[SB_CX] : k == 3 ? off[SB_CK] : off[SB_CO];
+      asm volatile(
+          "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+              smem_addr(rec + dst + 16 * cap * (tid - first))),
+          "l"(g + src + 16 * cnt * (tid - first)), "r"(16 * (k == 2 ? ncx : cnt)), "r"(smem_addr(&arrived))
+          : "memory");
+    }
+  }
+  auto sec = [&](int o) { return reinterpret_cast<const StageChunk *>(rec + o); };
+  EdgeRec<R> er;
+  if (tid < n[S_EM]) stage_rec(reinterpret_cast<const StageChunk *>(g + off[SB_E]), n[S_EM], tid, &er);
+  const int *ids = reinterpret_cast<const int *>(g + off[SB_GE]), *idc = reinterpret_cast<const int *>(g + off[SB_GC]);
+  int ge[2] = {0, 0}, gc = 0;
+  if (tid < n[S_EA]) ge[0] = __ldg(ids + tid);
+  if (tid + NT < n[S_EA]) ge[1] = __ldg(ids + tid + NT);
+  if (tid < n[S_CA]) gc = __ldg(idc + tid);
+  // owned edges belong to the first threads, owned cells to the last (top counts from the end)
+  const int top = NT - 1 - tid;
+  const bool edge = tid < n[S_EO], cell = top < n[S_CO];
+  const int own = edge ? ge[0] : cell ? __ldg(idc + top) : -1;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  // the state on the tile (each value once: past L1) and what the thread's owned entity adds to
+  A x0 = A(0), acc = A(0);
+  {
+    R u0 = R(0), u1 = R(0), h = R(0);  // in flight together
+    if (tid < n[S_EA]) u0 = __ldcg(a.u + ge[0]);
+    if (tid + NT < n[S_EA]) u1 = __ldcg(a.u + ge[1]);
+    if (tid < n[S_CA]) h = __ldcg(a.h + gc);
+    if (edge || cell) {
+      const RK<R, A> &rk = edge ? a.rku : a.rkh;
+      if (rk.next) x0 = __ldcg(rk.x0 + own);
+      if (rk.acc_out) acc = __ldcg(rk.acc_in + own);
+    }
+    if (tid < n[S_EA]) stage_val<R>(w, W_U + tid, 0) = u0;
+    if (tid + NT < n[S_EA]) stage_val<R>(w, W_U + tid + NT, 0) = u1;
+    if (tid < n[S_CA]) stage_val<R>(w, W_H + tid, 0) = h;
+  }
+  __syncthreads();  // (also: the barrier's initialisation is visible)
+  {
+    unsigned ok = 0;  // the copies were issued a stage ago; a bound all the same
+    for (int i = 0; i < (1 << 20) && !ok; i++)
+      asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared.b64 p, [%1], 0;\nselp.u32 %0, 1, 0, p;\n}"
+                   : "=r"(ok)
+                   : "r"(smem_addr(&arrived))
+                   : "memory");
+    if (__syncthreads_or(!ok)) {
+      if (a.ph.bad) *a.ph.bad = 1;
+      return;
+    }
+  }
+  // phase 1: vertices; from the next warp on, ke cells (with viscosity also the other divergences)
+  const int nv32 = stage_up32(n[S_VA]);
+  if (tid < n[S_VA]) {
+    VertexRec<R> r;
+    stage_rec(sec(S::V), kCapVA, tid, &r);
+    const int gv = a.out.on && tid < n[S_VO] ? __ldg(reinterpret_cast<const int *>(g + off[SB_GV]) + tid) : -1;
+    stage_vertex(r, w, a, tid, gv, visc);
+  } else if (tid >= nv32) {
+    for (int i = tid - nv32; i < (visc ? n[S_CM] : n[S_CK]); i += NT - nv32) {
+      CellMRec<R> m;
+      stage_rec(sec(S::CM), kCapCM, i, &m);
+      if (i < n[S_CK]) {
+        CellKRec<R> r;
+        stage_rec(sec(S::CK), kCapCK, i, &r);
+        stage_ke(r, m.v[6], m.v[7], w, a, i, a.out.on && i < n[S_CO] ? __ldg(idc + i) : -1);
+      }
+      if (visc) {
+        CellXRec<R> r;
+        stage_rec(sec(S::CX), kCapCM, i, &r);
+        stage_div(r, m.v[7], w, i);
+      }
+    }
+  }
+  __syncthreads();
+  // phase 2: tangential velocity of the pv_edge layer; pv_cell on the last threads
+  R v = R(0);
+  if (tid < n[S_EM]) {
+    v = stage_perp(er, w);
+  } else if (top < n[S_CM]) {
+    CellMRec<R> r;
+    stage_rec(sec(S::CM), kCapCM, top, &r);
+    stage_pvcell(r, w, top);
+  }
+  __syncthreads();
+  // phase 3: pv_edge; thickness of the owned cells on the last threads
+  if (tid < n[S_EM]) {
+    stage_edge(er, w, a, tid, a.out.on && edge ? own : -1, v, del4);
+  } else if (cell) {
+    CellMRec<R> m;
+    CellXRec<R> r;
+    stage_rec(sec(S::CM), kCapCM, top, &m);
+    stage_rec(sec(S::CX), kCapCM, top, &r);
+    stage_thick(r, sec(S::CO)[top], m.v[6], m.v[7], w, a, top, own, x0, acc);
+  }
+  __syncthreads();
+  if (del4) {
+    if (tid < n[S_VA]) {
+      VertexRec<R> r;
+      stage_rec(sec(S::V), kCapVA, tid, &r);
+      stage_del4_vertex(r, w, tid, n[S_EM]);
+    } else if (tid - nv32 >= 0 && tid - nv32 < n[S_CK]) {
+      const int i = tid - nv32;
+      CellXRec<R> r;
+      CellMRec<R> m;
+      stage_rec(sec(S::CX), kCapCM, i, &r);
+      stage_rec(sec(S::CM), kCapCM, i, &m);
+      stage_del4_cell(r, m.v[7], w, i, n[S_EM]);
+    }
+    __syncthreads();
+  }
+  // phase 4
+  if (edge) stage_tend(er, w, a, tid, own, x0, acc);
+}
+
+}  // namespace mpsw

@@ -1,0 +1,352 @@
+// Nonlinear RK stage on halo tiles: the tile's data layout and the per-entity arithmetic of each
+// phase (mpsw_stage.cuh runs the phases in a thread block, one kernel per stage; a host loop can
+// run the same functions).
+//
+// A tile owns a run of cells of the internal order, the edges whose lower-numbered cell it owns
+// and the vertices whose lowest-numbered cell it owns.  Its local spaces are numbered in nested
+// layers (owned first, then what the owned tendencies need), so that every phase works on a
+// prefix.  All of the mesh a stage reads for the tile is packed into one blob of records, one per
+// entity.  Values are combined in the reference's order, entity by entity
+// (src/mpas_sw_dyncore.f90:95-361, 468-637), so FP64 results do not depend on the tiling.
+#pragma once
+
+#include <cmath>
+#include <cstddef>
+
+#include "mpsw_internal.h"
+
+namespace mpsw {
+
+// Prefix sizes of a tile's local spaces: owned edges | edges whose pv_edge is formed (owned and
+// their edgesOnEdge) | edges whose u is read; owned cells | cells of owned edges (and owned) |
+// cells whose pv_cell is formed | cells whose h is read; owned vertices | all vertices.
+enum StageCount { S_EO, S_EM, S_EA, S_CO, S_CK, S_CM, S_CA, S_VO, S_VA, kStageCounts };
+
+// Most entities of each layer (the builder shortens a tile until it fits): the values that the
+// phases exchange then have fixed places in shared memory, and neighbour lists hold byte offsets
+// into them, so a gather is one unpack and one load.  The pv_edge layer is also at most the
+// threads of a block, which keep one edge's record in registers through the phases.
+constexpr int kStageThreads = 448;
+constexpr int kCapEM = 384, kCapEA = 672, kCapCO = 96, kCapCK = 128, kCapCM = 192, kCapCA = 256, kCapVA = 400;
+
+// A tile fits when its layers do, and when the kinds of entities a phase forms side by side get
+// threads of their own, in whole warps: vertices and ke cells, edges and pv_cell cells, edges and
+// owned cells.
+MPSW_HD inline int stage_up32(int x) { return (x + 31) & ~31; }
+MPSW_HD inline bool stage_fits(const int *n) {
+  return n[S_EM] <= kCapEM && n[S_EA] <= kCapEA && n[S_CO] <= kCapCO && n[S_CK] <= kCapCK && n[S_CM] <= kCapCM &&
+         n[S_CA] <= kCapCA && n[S_VA] <= kCapVA && stage_up32(n[S_VA]) + n[S_CK] <= kStageThreads &&
+         stage_up32(n[S_EM]) + stage_up32(n[S_CM]) <= kStageThreads &&
+         stage_up32(n[S_EM]) + stage_up32(n[S_CO]) <= kStageThreads;
+}
+
+// Values exchanged between the phases: offsets in values from the start of the work area.
+enum StageWork {
+  W_U = 0,
+  W_H = W_U + kCapEA,
+  W_PVV = W_H + kCapCA,
+  W_PC = W_PVV + kCapVA,
+  W_KE = W_PC + kCapCM,
+  W_HS = W_KE + kCapCK,
+  W_PE = W_HS + kCapCK,
+  W_HE = W_PE + kCapEM,
+  W_VORT = W_HE + kCapEM,  // from here: with viscosity
+  W_DIV = W_VORT + kCapVA,
+  W_DSQ = W_DIV + kCapCM,  // from here: with del4
+  W_V4 = W_DSQ + kCapEM,
+  W_C4 = W_V4 + kCapVA,
+  W_END = W_C4 + kCapCK
+};
+MPSW_HD inline int stage_work(int r, bool visc, bool del4) { return r * (del4 ? W_END : visc ? W_DSQ : W_VORT); }
+
+// A blob: per entity a record of 16-byte chunks, stored chunk by chunk ([chunk][n]), first chunk(s)
+// the neighbour list as byte offsets into the work arrays, then values in the stencils' precision.
+//   vertices:       edges[3] cells[3]; sign dcEdge [3], kites [3], area, 1 / area, f
+//   pv_cell cells:  vertices[6]; kites [6], area, 1 / area
+//   the same cells: edges[6] in the scatter order; sign dvEdge [6]
+//   ke cells:       edges[6] in the cell's order; (dcEdge / 4) dvEdge [6], h_s
+//   owned cells:    cells across [6]
+//   pv_edge edges:  c1 c2 v1 v2 as local indices, edgesOnEdge[10]; weights [10], dc, dv, 1 / dc, 1 / dv
+// The edge records come last and go to registers; what is before them goes to shared memory.
+// Slots past a list weigh zero and point at the entity itself (cells) or at value 0.
+enum StageSection { SB_V, SB_CM, SB_CX, SB_CK, SB_CO, SB_E, SB_GE, SB_GC, SB_GV, kStageSections };
+
+MPSW_HD inline int stage_chunks(int vals, int r) { return (vals * r + 15) / 16; }
+constexpr int kValsV = 9, kValsCM = 8, kValsCX = 6, kValsCK = 7, kValsE = 14;
+
+// Byte offsets of a blob's sections for values of `r` bytes; returns the blob's size.
+MPSW_HD inline int stage_layout(const int *n, int r, int *off) {
+  int o = 0;
+  off[SB_V] = o; o += 16 * n[S_VA] * (1 + stage_chunks(kValsV, r));
+  off[SB_CM] = o; o += 16 * n[S_CM] * (1 + stage_chunks(kValsCM, r));
+  off[SB_CX] = o; o += 16 * n[S_CM] * (1 + stage_chunks(kValsCX, r));
+  off[SB_CK] = o; o += 16 * n[S_CK] * (1 + stage_chunks(kValsCK, r));
+  off[SB_CO] = o; o += 16 * n[S_CO];
+  off[SB_E] = o; o += 16 * n[S_EM] * (2 + stage_chunks(kValsE, r));
+  off[SB_GE] = o; o += (4 * n[S_EA] + 15) / 16 * 16;
+  off[SB_GC] = o; o += (4 * n[S_CA] + 15) / 16 * 16;
+  off[SB_GV] = o; o += (4 * n[S_VO] + 15) / 16 * 16;
+  return o;
+}
+
+// 16 bytes of a record
+struct alignas(16) StageChunk {
+  unsigned w[4];
+};
+// entry k of a neighbour list held in chunks
+MPSW_HD inline int stage_at(const StageChunk *c, int k) {
+  const unsigned w = c[k >> 3].w[(k & 7) >> 1];
+  return (int)((k & 1) ? w >> 16 : w & 0xFFFFu);
+}
+// A record in registers: L chunks of lists and NV values.
+template <typename R, int L, int NV>
+struct StageRec {
+  static constexpr int kChunks = (NV * (int)sizeof(R) + 15) / 16;
+  StageChunk list[L];
+  union {
+    StageChunk raw[kChunks > 0 ? kChunks : 1];
+    R v[(kChunks > 0 ? kChunks : 1) * 16 / sizeof(R)];
+  };
+  MPSW_HD StageRec() {}
+  MPSW_HD int at(int k) const { return stage_at(list, k); }
+};
+// the record of entity i, from a section's first chunk; n: records a chunk row holds
+template <typename R, int L, int NV>
+MPSW_HD inline void stage_rec(const StageChunk *p, int n, int i, StageRec<R, L, NV> *r) {
+#pragma unroll
+  for (int k = 0; k < L; k++) r->list[k] = p[k * n + i];
+#pragma unroll
+  for (int k = 0; k < StageRec<R, L, NV>::kChunks; k++) r->raw[k] = p[(L + k) * n + i];
+}
+template <typename R>
+using VertexRec = StageRec<R, 1, kValsV>;
+template <typename R>
+using CellMRec = StageRec<R, 1, kValsCM>;
+template <typename R>
+using CellXRec = StageRec<R, 1, kValsCX>;
+template <typename R>
+using CellKRec = StageRec<R, 1, kValsCK>;
+template <typename R>
+using EdgeRec = StageRec<R, 2, kValsE>;
+
+// value at byte offset b of the work array that starts at value `first`
+template <typename R>
+MPSW_HD inline R &stage_val(unsigned char *w, int first, int b) {
+  return *reinterpret_cast<R *>(w + first * (int)sizeof(R) + b);
+}
+
+// Where a stage's linearisation point goes (any may be null): u, h_edge, v, gradPVt, gradPVn,
+// pv_edge on edges, vorticity, h_vertex on vertices, ke on cells, in FP64 and / or rounded to FP32.
+struct StageBaseOut {
+  double *d[9];
+  float *f[9];
+  int on;  // any of them
+};
+enum StageBaseField { SO_U, SO_HE, SO_V, SO_GPT, SO_GPN, SO_PE, SO_VORT, SO_HV, SO_KE };
+
+// One stage: input state, RK bookkeeping, optional tendencies and linearisation point.
+template <typename R, typename A>
+struct StageArgs {
+  const R *u, *h;  // h is stored relative to off
+  R off;
+  Phys<R> ph;
+  RK<R, A> rku, rkh;
+  R *tend_u, *tend_h;
+  StageBaseOut out;
+  const R *sc2, *sc4, *usrc;  // edge scalings of del2 / del4, wind source
+};
+
+MPSW_HD inline void stage_put(const StageBaseOut &o, int f, int g, double x) {
+  if (o.d[f]) o.d[f][g] = x;
+  if (o.f[f]) o.f[f][g] = (float)x;
+}
+
+// The functions below form entity i of a tile from its record; w: the work area; g: the internal
+// index where the tile owns the entity, else -1.
+
+// ---- phase 1: vertices (:208-219, :282-292) ----------------------------------------------------
+template <typename R, typename A>
+MPSW_HD inline void stage_vertex(const VertexRec<R> &r, unsigned char *w, const StageArgs<R, A> &a, int i, int g,
+                                 bool visc) {
+  R circ = R(0), hv = R(0);
+#pragma unroll
+  for (int k = 0; k < VDEG; k++) circ = circ + r.v[k] * stage_val<R>(w, W_U, r.at(k));
+  const R area = r.v[6], ra = r.v[7];
+  const R vort = div_r(circ, area, ra);
+#pragma unroll
+  for (int k = 0; k < VDEG; k++) hv = hv + (stage_val<R>(w, W_H, r.at(3 + k)) + a.off) * r.v[3 + k];
+  hv = div_r(hv, area, ra);
+  stage_val<R>(w, W_PVV + i, 0) = (r.v[8] + vort) / hv;
+  if (visc) stage_val<R>(w, W_VORT + i, 0) = vort;
+  if (g >= 0) {
+    stage_put(a.out, SO_VORT, g, vort);
+    stage_put(a.out, SO_HV, g, hv);
+  }
+}
+
+// RK bookkeeping of one value (src/mpas_sw_module.f90:590-611); x0 / acc: rk.x0 and rk.acc_in there
+template <typename R, typename A>
+MPSW_HD inline void stage_rk(const RK<R, A> &rk, int g, R t, A x0, A acc) {
+  if (rk.next) rk.next[g] = rk.frozen ? R(x0) : R((x0 - A(rk.off)) + rk.c * A(t));
+  if (rk.acc_out && !rk.frozen) rk.acc_out[g] = acc + rk.w * A(t);
+}
+
+// ---- phase 1: kinetic energy (:245-256) ----------------------------------------------------------
+template <typename R, typename A>
+MPSW_HD inline void stage_ke(const CellKRec<R> &r, R area, R ra, unsigned char *w, const StageArgs<R, A> &a, int i,
+                             int g) {
+  R ke = R(0);
+#pragma unroll
+  for (int k = 0; k < 6; k++) {
+    const R u = stage_val<R>(w, W_U, r.at(k));
+    ke = ke + r.v[k] * (u * u);
+  }
+  ke = div_r(ke, area, ra);
+  stage_val<R>(w, W_KE + i, 0) = ke;
+  stage_val<R>(w, W_HS + i, 0) = r.v[6];
+  if (g >= 0) stage_put(a.out, SO_KE, g, ke);
+}
+// divergence, where viscosity needs it (:222-242)
+template <typename R>
+MPSW_HD inline void stage_div(const CellXRec<R> &r, R ra, unsigned char *w, int i) {
+  R div = R(0);
+#pragma unroll
+  for (int k = 0; k < 6; k++) div = div + r.v[k] * stage_val<R>(w, W_U, r.at(k));
+  stage_val<R>(w, W_DIV + i, 0) = div * ra;
+}
+// ---- phase 3: thickness tendency of an owned cell and its RK update (:468-482) ---------------------
+template <typename R, typename A>
+MPSW_HD inline void stage_thick(const CellXRec<R> &r, const StageChunk &across, R area, R ra, unsigned char *w,
+                                const StageArgs<R, A> &a, int i, int g, A x0, A acc) {
+  const R hc = stage_val<R>(w, W_H + i, 0) + a.off;
+  R th = R(0);
+#pragma unroll
+  for (int k = 0; k < 6; k++) {
+    const R he = R(0.5) * (hc + (stage_val<R>(w, W_H, stage_at(&across, k)) + a.off));
+    th = th - (stage_val<R>(w, W_U, r.at(k)) * r.v[k]) * he;
+  }
+  th = div_r(th, area, ra);
+  if (a.tend_h) a.tend_h[g] = th;
+  stage_rk(a.rkh, g, th, x0, acc);
+}
+
+// ---- phase 2: tangential velocity (:259-267), pv_cell (:324-340) -----------------------------------
+template <typename R>
+MPSW_HD inline R stage_perp(const EdgeRec<R> &r, unsigned char *w) {
+  R v = R(0);
+#pragma unroll
+  for (int j = 0; j < 10; j++) v = v + r.v[j] * stage_val<R>(w, W_U, r.at(4 + j));
+  return v;
+}
+template <typename R>
+MPSW_HD inline void stage_pvcell(const CellMRec<R> &r, unsigned char *w, int i) {
+  R pc = R(0);
+#pragma unroll
+  for (int k = 0; k < 6; k++) {
+    const R pv = stage_val<R>(w, W_PVV, r.at(k));
+    if constexpr (sizeof(R) == 4) pc = pc + (r.v[k] * r.v[7]) * pv;
+    else pc = pc + div_r(r.v[k] * pv, r.v[6], r.v[7]);
+  }
+  stage_val<R>(w, W_PC + i, 0) = pc;
+}
+
+// ---- phase 3: gradients of pv (:296-301), pv_edge (:305-320, :344-359), h_edge (:95-105) and
+// delsq_u (:539-551); v: the tangential velocity of phase 2 --------------------------------------------
+template <typename R, typename A>
+MPSW_HD inline void stage_edge(const EdgeRec<R> &r, unsigned char *w, const StageArgs<R, A> &a, int i, int g, R v,
+                               bool del4) {
+  const int c1 = r.at(0), c2 = r.at(1), v1 = r.at(2), v2 = r.at(3);
+  const R dc = r.v[10], dv = r.v[11], rc = r.v[12], rv = r.v[13], u = stage_val<R>(w, W_U + i, 0);
+  const R pv1 = stage_val<R>(w, W_PVV, v1), pv2 = stage_val<R>(w, W_PVV, v2);
+  const R gpt = div_r(pv2 - pv1, dv, rv);
+  R pe = R(0);
+  pe = pe + R(0.5) * pv1;
+  pe = pe + R(0.5) * pv2;
+  pe = pe - ((a.ph.apvm * v) * a.ph.dt) * gpt;
+  const R gpn = div_r(stage_val<R>(w, W_PC, c2) - stage_val<R>(w, W_PC, c1), dc, rc);
+  pe = pe - ((a.ph.apvm * u) * a.ph.dt) * gpn;
+  const R he = R(0.5) * ((stage_val<R>(w, W_H, c1) + a.off) + (stage_val<R>(w, W_H, c2) + a.off));
+  stage_val<R>(w, W_PE + i, 0) = pe;
+  stage_val<R>(w, W_HE + i, 0) = sizeof(R) == 4 ? u * he : he;  // FP32 stencils keep the thickness flux
+  if (del4)
+    stage_val<R>(w, W_DSQ + i, 0) = div_r(stage_val<R>(w, W_DIV, c2) - stage_val<R>(w, W_DIV, c1), dc, rc) -
+                                    div_r(stage_val<R>(w, W_VORT, v2) - stage_val<R>(w, W_VORT, v1), dv, rv);
+  if (g >= 0) {
+    stage_put(a.out, SO_U, g, u);
+    stage_put(a.out, SO_HE, g, he);
+    stage_put(a.out, SO_V, g, v);
+    stage_put(a.out, SO_GPT, g, gpt);
+    stage_put(a.out, SO_GPN, g, gpn);
+    stage_put(a.out, SO_PE, g, pe);
+  }
+}
+
+// ---- del4 (:554-589): delsq_vorticity on the vertices, delsq_divergence on the cells of owned
+// edges; entities whose neighbours lie outside the pv_edge layer are read by no owned edge -------
+template <typename R>
+MPSW_HD inline void stage_del4_vertex(const VertexRec<R> &r, unsigned char *w, int i, int nem) {
+  R circ = R(0);
+#pragma unroll
+  for (int k = 0; k < VDEG; k++) {
+    if (r.at(k) >= nem * (int)sizeof(R)) return;
+    circ = circ + r.v[k] * stage_val<R>(w, W_DSQ, r.at(k));
+  }
+  stage_val<R>(w, W_V4 + i, 0) = circ * r.v[7];
+}
+template <typename R>
+MPSW_HD inline void stage_del4_cell(const CellXRec<R> &r, R ra, unsigned char *w, int i, int nem) {
+  R div = R(0);
+#pragma unroll
+  for (int k = 0; k < 6; k++) {
+    if (r.at(k) >= nem * (int)sizeof(R)) return;
+    div = div + r.v[k] * stage_val<R>(w, W_DSQ, r.at(k));
+  }
+  stage_val<R>(w, W_C4 + i, 0) = div * ra;
+}
+
+// ---- phase 4: normal-velocity tendency of an owned edge (:485-637) and its RK update -----------
+template <typename R, typename A>
+MPSW_HD inline void stage_tend(const EdgeRec<R> &r, unsigned char *w, const StageArgs<R, A> &a, int i, int g, A x0,
+                               A acc) {
+  const R pee = stage_val<R>(w, W_PE + i, 0);
+  R q = R(0);
+#pragma unroll
+  for (int j = 0; j < 10; j++) {
+    const int e = r.at(4 + j);
+    const R wpv = R(0.5) * (pee + stage_val<R>(w, W_PE, e));
+    if constexpr (sizeof(R) == 4) q = q + (r.v[j] * stage_val<R>(w, W_HE, e)) * wpv;
+    else q = q + ((r.v[j] * stage_val<R>(w, W_U, e)) * wpv) * stage_val<R>(w, W_HE, e);
+  }
+  const int c1 = r.at(0), c2 = r.at(1), v1 = r.at(2), v2 = r.at(3);
+  const R dc = r.v[10], dv = r.v[11], rc = r.v[12], rv = r.v[13];
+  const R h1 = stage_val<R>(w, W_H, c1), h2 = stage_val<R>(w, W_H, c2);
+  const R s1 = stage_val<R>(w, W_HS, c1), s2 = stage_val<R>(w, W_HS, c2);
+  R grav;
+  if constexpr (sizeof(R) == 8) grav = R(GRAVITY) * ((((h2 + a.off) + s2) - (h1 + a.off)) - s1);
+  else grav = R(GRAVITY) * ((h2 - h1) + (s2 - s1));  // difference the offset-free values first
+  const R ke1 = stage_val<R>(w, W_KE, c1), ke2 = stage_val<R>(w, W_KE, c2);
+  R tu = q - div_r((ke2 - ke1) + grav, dc, rc);
+  if (a.ph.visc2 > R(0)) {
+    R ud = div_r(stage_val<R>(w, W_DIV, c2) - stage_val<R>(w, W_DIV, c1), dc, rc) -
+           div_r(stage_val<R>(w, W_VORT, v2) - stage_val<R>(w, W_VORT, v1), dv, rv);
+    ud = (a.sc2[g] * a.ph.visc2) * ud;
+    tu = tu + ud;
+  }
+  if (a.ph.visc4 > R(0)) {
+    R ud = div_r(stage_val<R>(w, W_C4, c2) - stage_val<R>(w, W_C4, c1), dc, rc) -
+           div_r(stage_val<R>(w, W_V4, v2) - stage_val<R>(w, W_V4, v1), dv, rv);
+    ud = (a.sc4[g] * a.ph.visc4) * ud;
+    tu = tu - ud;
+  }
+  const R hee = R(0.5) * ((h1 + a.off) + (h2 + a.off));
+  if (a.ph.wind) tu = tu + (a.usrc[g] / R(RHO_REF)) / hee;
+  if (a.ph.drag) {
+    const R kee = R(0.5) * (ke1 + ke2);
+    tu = tu - ((R(1.0e-3) * stage_val<R>(w, W_U + i, 0)) * sqrt(R(2) * kee)) / hee;
+  }
+  if (a.ph.bad && !(tu - tu == R(0))) *a.ph.bad = 1;  // NaN or infinite
+  if (a.tend_u) a.tend_u[g] = tu;
+  stage_rk(a.rku, g, tu, x0, acc);
+}
+
+}  // namespace mpsw

@@ -382,4 +382,168 @@ std::string build_tiles(const BuiltMesh &m, size_t budget, int kmax, int M, bool
   return "";
 }
 
+// ---- tiles of the nonlinear stage (mpsw_stage.h) ------------------------------------------------
+namespace {
+
+// Layers of the tile owning cells [c0, c1): the tangent-linear layers, with the owned vertices
+// first among the vertices.
+void stage_spaces(const Builder &b, const BuiltMesh &m, int c0, int c1, Space &E, Space &C, Space &V, int *n) {
+  for (int c = c0; c < c1; c++)
+    for (int k = 0; k < b.cn(c); k++) {
+      const int v = b.cvs(c, k);
+      if (std::min(b.vc(v, 0), std::min(b.vc(v, 1), b.vc(v, 2))) == c) V.add(v);
+    }
+  n[S_VO] = V.close();
+  int cnt[kTileCounts];
+  tile_spaces(b, m, c0, c1, false, E, C, V, cnt);
+  n[S_EO] = cnt[E_OWN]; n[S_EM] = cnt[E_MID]; n[S_EA] = cnt[E_ALL];
+  n[S_CO] = cnt[C_OWN]; n[S_CK] = cnt[C_KE]; n[S_CM] = cnt[C_MID]; n[S_CA] = cnt[C_ALL];
+  n[S_VA] = cnt[V_ALL];
+}
+
+// Every neighbour a phase reads is in the layer it is formed on.
+bool stage_valid(const Builder &b, const BuiltMesh &m, const Space &E, const Space &C, const Space &V, const int *n) {
+  auto in = [](int x, int hi) { return x >= 0 && x < hi; };
+  for (int v : V.list)
+    for (int k = 0; k < VDEG; k++)
+      if (!in(E.local(b.ves(v, k)), n[S_EA]) || !in(C.local(b.vc(v, k)), n[S_CA])) return false;
+  for (int i = 0; i < n[S_CM]; i++) {
+    const int c = C.list[i];
+    for (int k = 0; k < b.cn(c); k++) {
+      if (!in(E.local(b.ces(c, k)), n[S_EA]) || !in(V.local(b.cvs(c, k)), n[S_VA])) return false;
+      if (i < n[S_CK] && !in(E.local(m.c_eoc[(size_t)k * m.nC + c]), n[S_EA])) return false;
+      if (i < n[S_CO] && !in(C.local(b.cnb(c, k)), n[S_CA])) return false;
+    }
+  }
+  for (int i = 0; i < n[S_EM]; i++) {
+    const int e = E.list[i];
+    const bool own = i < n[S_EO];
+    for (int c : {m.e_c1[e], m.e_c2[e]}) {
+      if (!in(C.local(c), own ? n[S_CK] : n[S_CM])) return false;
+      if (own)  // del4: delsq_u on every edge of the cell
+        for (int k = 0; k < b.cn(c); k++)
+          if (!in(E.local(b.ces(c, k)), n[S_EM])) return false;
+    }
+    for (int v : {m.e_v1[e], m.e_v2[e]}) {
+      if (!in(V.local(v), n[S_VA])) return false;
+      if (own)
+        for (int k = 0; k < VDEG; k++)
+          if (!in(E.local(b.ves(v, k)), n[S_EM])) return false;
+    }
+    for (int j = 0; j < m.e_n[e]; j++)
+      if (!in(E.local(b.eoe(e, j)), own ? n[S_EM] : n[S_EA])) return false;
+  }
+  return true;
+}
+
+// One tile's blob with values of type R (stage_layout).
+template <typename R>
+void stage_pack(const Builder &b, const BuiltMesh &m, const Space &E, const Space &C, const Space &V, const int *n,
+                std::vector<unsigned char> *blob) {
+  int off[kStageSections];
+  const int size = stage_layout(n, (int)sizeof(R), off);
+  const size_t base = blob->size();
+  blob->resize(base + (size_t)size, 0);
+  unsigned char *p = blob->data() + base;
+  // entry k of entity i's list, and value k after `lists` list chunks, in a section of cnt records
+  auto list = [&](int sec, int cnt, int i, int k, int x) {
+    reinterpret_cast<uint16_t *>(p + off[sec] + 16 * ((k >> 3) * cnt + i))[k & 7] = (uint16_t)(x * (int)sizeof(R));
+  };
+  constexpr int per = 16 / (int)sizeof(R);
+  auto val = [&](int sec, int cnt, int lists, int i, int k, R x) {
+    reinterpret_cast<R *>(p + off[sec] + 16 * ((lists + k / per) * cnt + i))[k % per] = x;
+  };
+  const int nv = n[S_VA], ncm = n[S_CM], nck = n[S_CK], nco = n[S_CO], nem = n[S_EM];
+  for (int i = 0; i < nv; i++) {
+    const int v = V.list[i];
+    for (int k = 0; k < VDEG; k++) {
+      const size_t s = (size_t)k * m.nV + v;
+      list(SB_V, nv, i, k, E.local(m.v_es[s]));
+      list(SB_V, nv, i, 3 + k, C.local(m.v_c[s]));
+      val(SB_V, nv, 1, i, k, R(m.v_esg[s]) * R(m.e_dc[m.v_es[s]]));
+      val(SB_V, nv, 1, i, 3 + k, R(m.v_k[s]));
+    }
+    val(SB_V, nv, 1, i, 6, R(m.v_area[v]));
+    val(SB_V, nv, 1, i, 7, R(1) / R(m.v_area[v]));
+    val(SB_V, nv, 1, i, 8, R(m.v_f[v]));
+  }
+  for (int i = 0; i < ncm; i++) {
+    const int c = C.list[i];
+    for (int k = 0; k < kCellSlots; k++) {
+      const size_t s = (size_t)k * m.nC + c;
+      if (i < nco) list(SB_CO, nco, i, k, k < b.cn(c) ? C.local(b.cnb(c, k)) : i);
+      if (k >= b.cn(c)) continue;  // padded: value 0 with coefficient 0
+      list(SB_CM, ncm, i, k, V.local(m.c_vs[s]));
+      val(SB_CM, ncm, 1, i, k, R(m.c_vk[s]));
+      list(SB_CX, ncm, i, k, E.local(m.c_es[s]));
+      val(SB_CX, ncm, 1, i, k, R(m.c_esg[s]) * R(m.e_dv[m.c_es[s]]));
+      if (i < nck) {
+        const int e = m.c_eoc[s];
+        list(SB_CK, nck, i, k, E.local(e));
+        val(SB_CK, nck, 1, i, k, (R(0.25) * R(m.e_dc[e])) * R(m.e_dv[e]));
+      }
+    }
+    val(SB_CM, ncm, 1, i, 6, R(m.c_area[c]));
+    val(SB_CM, ncm, 1, i, 7, R(1) / R(m.c_area[c]));
+    if (i < nck) val(SB_CK, nck, 1, i, 6, R(m.c_hs[c]));
+  }
+  for (int i = 0; i < nem; i++) {
+    const int e = E.list[i];
+    list(SB_E, nem, i, 0, C.local(m.e_c1[e]));
+    list(SB_E, nem, i, 1, C.local(m.e_c2[e]));
+    list(SB_E, nem, i, 2, V.local(m.e_v1[e]));
+    list(SB_E, nem, i, 3, V.local(m.e_v2[e]));
+    for (int j = 0; j < kEoeSlots; j++) {
+      const bool has = j < m.e_n[e];  // a padded slot weighs nothing
+      list(SB_E, nem, i, 4 + j, has ? E.local(b.eoe(e, j)) : i);
+      val(SB_E, nem, 2, i, j, has ? R(m.e_w[(size_t)j * m.nE + e]) : R(0));
+    }
+    val(SB_E, nem, 2, i, 10, R(m.e_dc[e]));
+    val(SB_E, nem, 2, i, 11, R(m.e_dv[e]));
+    val(SB_E, nem, 2, i, 12, R(1) / R(m.e_dc[e]));
+    val(SB_E, nem, 2, i, 13, R(1) / R(m.e_dv[e]));
+  }
+  std::memcpy(p + off[SB_GE], E.list.data(), 4 * E.list.size());
+  std::memcpy(p + off[SB_GC], C.list.data(), 4 * C.list.size());
+  std::memcpy(p + off[SB_GV], V.list.data(), 4 * (size_t)n[S_VO]);
+}
+
+}  // namespace
+
+std::string build_stage_tiles(const BuiltMesh &m, int kmax, StageSetHost *o) {
+  if (kmax < 1) return "tile size must be positive";
+  for (int c = 0; c < m.nC; c++)
+    if (m.c_n[c] > kCellSlots) return "stage tiles need at most 6 edges per cell";
+  for (int e = 0; e < m.nE; e++)
+    if (m.e_n[e] > kEoeSlots) return "stage tiles need at most 10 edgesOnEdge";
+  for (const std::vector<double> *x : {&m.e_dc, &m.e_dv, &m.c_area, &m.v_area})
+    for (double d : *x)
+      if (!(d > 1e-50 && d < 1e50)) return "a mesh metric outside the range div_r serves";
+  Builder b(m);
+  *o = StageSetHost();
+  int stamp = 0;
+  for (int c0 = 0; c0 < m.nC;) {
+    int K = std::min(kmax, m.nC - c0), n[kStageCounts];
+    for (;; K = std::max(1, K - (K + 4) / 5)) {  // shorten the run while its halo is too large
+      Space E(b.se, b.le, stamp), C(b.sc, b.lc, stamp), V(b.sv, b.lv, stamp);
+      stamp++;
+      stage_spaces(b, m, c0, c0 + K, E, C, V, n);
+      if (!stage_fits(n)) {
+        if (K == 1) return "one cell's halo exceeds a tile";
+        continue;
+      }
+      if (!stage_valid(b, m, E, C, V, n)) return fail(o->ntiles, "a phase of the stage would read outside its tile");
+      o->cnt.insert(o->cnt.end(), n, n + kStageCounts);
+      o->off64.push_back((long long)o->blob64.size());
+      o->off32.push_back((long long)o->blob32.size());
+      stage_pack<double>(b, m, E, C, V, n, &o->blob64);
+      stage_pack<float>(b, m, E, C, V, n, &o->blob32);
+      break;
+    }
+    o->ntiles++;
+    c0 += K;
+  }
+  return "";
+}
+
 }  // namespace mpsw

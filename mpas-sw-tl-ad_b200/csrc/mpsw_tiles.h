@@ -19,6 +19,7 @@
 
 #include "mpsw_internal.h"
 #include "mpsw_setup.h"
+#include "mpsw_stage.h"
 
 namespace mpsw {
 
@@ -54,5 +55,19 @@ struct TileSetHost {
 // `kmax` cells.  Returns an empty string or the problem found (a cell whose halo alone exceeds
 // the budget, or a phase that would read outside its tile).
 std::string build_tiles(const BuiltMesh &m, size_t budget, int kmax, int M, bool adjoint, TileSetHost *out);
+
+// Tiles of the nonlinear stage (mpsw_stage.h).
+struct StageSetHost {
+  int ntiles = 0;
+  std::vector<int> cnt;                                  // [ntiles][kStageCounts]
+  std::vector<long long> off64, off32;                   // [ntiles] byte offset of each tile's blob
+  std::vector<unsigned char> blob64, blob32;
+};
+
+// Build the nonlinear stage's tiles with at most kmax owned cells each (fewer where a layer would
+// exceed its cap, stage_fits), for a mesh with at most 6 edges per cell and 10 edgesOnEdge.
+// Returns an empty string or what keeps the mesh from being tiled (the stage then runs as
+// grid-wide passes).
+std::string build_stage_tiles(const BuiltMesh &m, int kmax, StageSetHost *out);
 
 }  // namespace mpsw

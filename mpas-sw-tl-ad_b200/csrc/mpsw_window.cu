@@ -311,15 +311,16 @@ void Engine::window_free_trajectory() {
 // stages' diagnostics and provisional states are left in sd[k] / su[k] (su[0] is the step's
 // start state); in precision 1 their base fields are rounded to FP32 (sd32, su32), and with
 // store_step >= 0 they are written to that step's slots of the valid stores.  hook(k) runs
-// after each stage.
+// after each stage.  base: the stages' linearisation points are wanted in sd / sd32 (a sweep that
+// recomputes them).
 template <typename Hook>
-static void traj_step(Engine &E, bool in_place, int prec, Hook &&hook, int store_step = -1) {
+static void traj_step(Engine &E, bool in_place, int prec, bool base, Hook &&hook, int store_step = -1) {
   Window &W = E.win;
   const Phys<double> ph = E.phys();
   double w[4], c[4];
   rk_coeffs(ph.dt, w, c);
   double *u0 = W.x_u, *h0 = W.x_h;
-  const bool st64 = store_step >= 0 && W.st[0].mem, st32 = store_step >= 0 && W.st[1].mem;
+  const bool st64 = store_step >= 0 && (W.store_now & 1), st32 = store_step >= 0 && (W.store_now & 2);
   for (int k = 0; k < 4; k++) {
     W.su[0] = u0;
     const double *ui = W.su[k];
@@ -328,18 +329,25 @@ static void traj_step(Engine &E, bool in_place, int prec, Hook &&hook, int store
                           k < 3 ? W.su[k + 1] : nullptr, c[k], w[k], 0.0, ph.tc1};
     RK<double, double> rh{h0, k == 0 ? h0 : E.acc_h, (k == 3 && in_place) ? h0 : E.acc_h,
                           k < 3 ? W.sh[k + 1] : nullptr, c[k], w[k], 0.0, 0};
-    E.fwd_stage(ui, hi, W.sd[k], ph, ru, rh, nullptr, nullptr);
-    if (prec == 1 || st64 || st32) {
+    const Diag<double> &d = W.sd[k];
+    const Diag<float> &f = W.sd32[k];
+    double *const own64[] = {nullptr, d.he, d.v, d.gpt, d.gpn, d.pe, d.vort, d.hv, d.ke};
+    float *const own32[] = {W.su32[k], f.he, f.v, f.gpt, f.gpn, f.pe, f.vort, f.hv, f.ke};
+    StageBaseOut out{};
+    for (int i = 0; i < 9; i++) {
+      out.d[i] = st64 ? store_field<double>(W.st[0], store_step, k, i) : base && prec == 0 ? own64[i] : nullptr;
+      out.f[i] = st32 ? store_field<float>(W.st[1], store_step, k, i) : base && prec == 1 ? own32[i] : nullptr;
+    }
+    out.on = st64 || st32 || base;
+    E.fwd_stage(ui, hi, d, ph, ru, rh, nullptr, nullptr, out);
+    if (!E.stage_tiled() && (prec == 1 || st64 || st32)) {  // the grid-wide passes left them in sd
       ConvList L{};
-      const Diag<double> &d = W.sd[k];
-      const Diag<float> &f = W.sd32[k];
       const double *src[] = {ui, d.he, d.v, d.gpt, d.gpn, d.pe, d.vort, d.hv, d.ke};
-      float *dst[] = {W.su32[k], f.he, f.v, f.gpt, f.gpn, f.pe, f.vort, f.hv, f.ke};
       const long long n[] = {E.nE, E.nE, E.nE, E.nE, E.nE, E.nE, E.nV, E.nV, E.nC};
       for (int i = 0; i < 9; i++) {
         L.src[i] = src[i];
-        L.dst[i] = st32 ? store_field<float>(W.st[1], store_step, k, i) : prec == 1 ? dst[i] : nullptr;
-        L.dst64[i] = st64 ? store_field<double>(W.st[0], store_step, k, i) : nullptr;
+        L.dst[i] = out.f[i];
+        L.dst64[i] = st64 ? out.d[i] : nullptr;
         L.n[i] = n[i];
       }
       L.count = 9;
@@ -479,36 +487,58 @@ static void window_forward_done(Engine &E) {
   cuda_check(cudaMemcpyAsync(W.fin_u, W.x_u, sizeof(double) * E.nE, cudaMemcpyDeviceToDevice, E.stream), "final");
   cuda_check(cudaMemcpyAsync(W.fin_h, W.x_h, sizeof(double) * E.nC, cudaMemcpyDeviceToDevice, E.stream), "final");
   cuda_check(cudaGetLastError(), "window forward");
-  for (int p = 0; p < 2; p++) W.st[p].valid = W.st[p].mem ? W.nsteps : 0;
+  for (int p = 0; p < 2; p++)
+    if ((W.store_now >> p) & 1) W.st[p].valid = W.nsteps;
   W.pending = false;
+  W.forward_phys = E.phys();
 }
 
-// Forward over the window from the captured start state, checkpointing every `every` steps
-// and, when stores are allocated, writing every stage's linearisation point to them (the
+// Forward over the window from the start state in x_u, x_h, checkpointing every `every` steps and
+// writing every stage's linearisation point to the stores of the precisions in `stores` (the
 // whole window is then one CUDA graph, since every step writes different slots).
-void Engine::window_forward() {
+void Engine::window_forward(int stores) {
   Window &W = win;
   const int nsteps = W.nsteps;
-  if (W.st[0].mem || W.st[1].mem) {
-    GraphKey key = graph_key(6, 0, nsteps, W.st[0].mem, W.st[1].mem);
+  W.store_now = stores;
+  if (stores) {
+    GraphKey key = graph_key(6, stores, nsteps, W.st[0].mem, W.st[1].mem);
     key.n2 = W.every;
     run_graph(key, [&]() {
       for (int n = 0; n < nsteps; n++) {
         window_checkpoint(*this, n);
-        traj_step(*this, true, 0, [](int) {}, n);
+        traj_step(*this, true, 0, false, [](int) {}, n);
       }
     });
   } else {
     for (int n = 0; n < nsteps; n++) {
       window_checkpoint(*this, n);
-      run_graph(graph_key(1, 0, 1, nullptr, nullptr), [&]() { traj_step(*this, true, 0, [](int) {}); });
+      run_graph(graph_key(1, 0, 1, nullptr, nullptr), [&]() { traj_step(*this, true, 0, false, [](int) {}); });
     }
   }
   window_forward_done(*this);
 }
 
-void Engine::window_ensure() {
-  if (win.pending) window_forward();
+// The forward sweep, for a sweep of precision prec (-1: for the final state).  The store written is
+// that of the precision that asks first; a window that later sweeps in the other one as well runs
+// the forward again for its store, from the first checkpoint and with the physics of the first run.
+void Engine::window_ensure(int prec) {
+  Window &W = win;
+  const int have = (W.st[0].mem ? 1 : 0) | (W.st[1].mem ? 2 : 0), want = prec >= 0 ? have & (1 << prec) : have & 1 ? 1 : have;
+  if (W.pending) {
+    window_forward(want);
+  } else if (want && prec >= 0 && W.st[prec].valid < W.nsteps) {
+    cuda_check(cudaMemcpyAsync(W.x_u, W.ck_u[0], sizeof(double) * nE, cudaMemcpyDeviceToDevice, stream), "copy");
+    cuda_check(cudaMemcpyAsync(W.x_h, W.ck_h[0], sizeof(double) * nC, cudaMemcpyDeviceToDevice, stream), "copy");
+    const Phys<double> now = phys_cache;
+    phys_cache = W.forward_phys;
+    try {
+      window_forward(want);
+    } catch (...) {
+      phys_cache = now;
+      throw;
+    }
+    phys_cache = now;
+  }
 }
 
 // Members per chunk of the fused stage kernels for B members of precision R (0: the split member
@@ -612,12 +642,18 @@ static void window_tl_impl(Engine &E, int prec, int B, double *user_u, double *u
     key.p3 = W.st[prec].mem;
     key.n2 = ((long long)W.nsteps << 20) | W.every;
     StableBaseScope stable(true);  // the members read only stored stages
+    E.beside_members = true;
+    struct Reset {
+      bool &b;
+      ~Reset() { b = false; }
+    } reset{E.beside_members};
+    W.store_now = 1 << prec;
     E.run_graph(key, [&]() {
       cuda_check(cudaEventRecord(E.ev_fork, E.stream), "event record");
       cuda_check(cudaStreamWaitEvent(E.side, E.ev_fork, 0), "event wait");
       for (int n = 0; n < W.nsteps; n++) {
         window_checkpoint(E, n);
-        traj_step(E, true, 0, [](int) {}, n);
+        traj_step(E, true, 0, false, [](int) {}, n);
         cuda_check(cudaEventRecord(E.ev_step, E.stream), "event record");
         cuda_check(cudaStreamWaitEvent(E.side, E.ev_step, 0), "event wait");
         for (int k = 0; k < 4; k++)
@@ -627,7 +663,12 @@ static void window_tl_impl(Engine &E, int prec, int B, double *user_u, double *u
       cuda_check(cudaStreamWaitEvent(E.stream, E.ev_join, 0), "event wait");
     });
     window_forward_done(E);
-  } else if (W.st[prec].valid >= W.nsteps) {
+    members_copy(E, B, user_u, user_h, du, dh);
+    cuda_check(cudaGetLastError(), "window_tl");
+    return;
+  }
+  E.window_ensure(prec);
+  if (W.st[prec].valid >= W.nsteps) {
     // stored linearisation points: the whole sweep is one graph of member kernels
     GraphKey key = E.graph_key(4, prec, B, du, dh);
     key.p3 = W.st[prec].mem;
@@ -639,7 +680,6 @@ static void window_tl_impl(Engine &E, int prec, int B, double *user_u, double *u
           tl_member_stage<R>(E, prec, B, du, dh, mb, ph, w, c, k, stored_base<R>(W, prec, n, k), E.stream, n == 0);
     });
   } else {
-    E.window_ensure();
     cuda_check(cudaMemcpyAsync(W.x_u, W.ck_u[0], sizeof(double) * E.nE, cudaMemcpyDeviceToDevice, E.stream), "copy");
     cuda_check(cudaMemcpyAsync(W.x_h, W.ck_h[0], sizeof(double) * E.nC, cudaMemcpyDeviceToDevice, E.stream), "copy");
     // recompute each step's stages; the member work of stage k runs right after stage k (the
@@ -647,7 +687,7 @@ static void window_tl_impl(Engine &E, int prec, int B, double *user_u, double *u
     const GraphKey key = E.graph_key(2, prec, B, du, dh);
     for (int n = 0; n < W.nsteps; n++)
       E.run_graph(key, [&]() {
-        traj_step(E, true, prec, [&](int k) {
+        traj_step(E, true, prec, true, [&](int k) {
           tl_member_stage<R>(E, prec, B, du, dh, mb, ph, w, c, k, base_for<R>(W, k), E.stream, true);
         });
       });
@@ -747,12 +787,12 @@ static void window_ad_impl(Engine &E, int prec, int B, double *user_u, double *u
     cuda_check(cudaMemcpyAsync(dh_, sh_, sizeof(double) * E.nC, cudaMemcpyDeviceToDevice, E.stream), "copy");
   };
   auto advance = [&](int k) {  // k nonlinear steps of the state in x_u, x_h
-    for (int i = 0; i < k; i++) E.run_graph(E.graph_key(1, 0, 1, nullptr, nullptr), [&]() { traj_step(E, true, 0, [](int) {}); });
+    for (int i = 0; i < k; i++) E.run_graph(E.graph_key(1, 0, 1, nullptr, nullptr), [&]() { traj_step(E, true, 0, false, [](int) {}); });
     W.forward_steps += k;
   };
   auto adjoint_step = [&]() {  // the adjoint of the step that starts at x_u, x_h
     E.run_graph(E.graph_key(3, prec, B, au, ah), [&]() {
-      traj_step(E, false, prec, [](int) {});
+      traj_step(E, false, prec, true, [](int) {});
       ad_member_step<R>(E, prec, B, au, ah, mb, ph, w, c, [&](int k) { return base_for<R>(W, k); });
     });
   };
@@ -840,7 +880,7 @@ void Engine::window_ad(int prec, int B, double *au, double *ah, cudaStream_t s) 
   if (mesh_dirty) throw EngineError(MPSW_ERR_STATE, "mesh changed since mpsw_window_init");
   if (prec != 0 && prec != 1) throw EngineError(MPSW_ERR_ARG, "precision must be 0 or 1");
   join(s, stream, true);
-  window_ensure();
+  window_ensure(prec);
   TuneScope scope(tuning(prec, B));
   nonfinite_clear();  // after the autotuner, whose timings run on arbitrary buffer contents
   if (prec == 0) window_ad_impl<double>(*this, prec, B, au, ah);
@@ -852,7 +892,7 @@ void Engine::window_ad(int prec, int B, double *au, double *ah, cudaStream_t s) 
 void Engine::window_final(double *u, double *h, cudaStream_t s) {
   if (!win.nsteps) throw EngineError(MPSW_ERR_STATE, "mpsw_window_init has not been called");
   join(s, stream, true);
-  window_ensure();
+  window_ensure(-1);
   cuda_check(cudaMemcpyAsync(u, win.fin_u, sizeof(double) * nE, cudaMemcpyDeviceToDevice, stream), "final u");
   cuda_check(cudaMemcpyAsync(h, win.fin_h, sizeof(double) * nC, cudaMemcpyDeviceToDevice, stream), "final h");
   join(s, stream, false);
@@ -990,7 +1030,7 @@ static double time_kernel_impl(Engine &E, int which, int prec, int B, int iters,
 double Engine::time_kernel(int which, int prec, int B, int iters) {
   if (!win.nsteps) throw EngineError(MPSW_ERR_STATE, "mpsw_window_init has not been called");
   if (which < 0 || which > 9 || B < 1 || iters < 1) throw EngineError(MPSW_ERR_ARG, "bad kernel timing request");
-  window_ensure();
+  window_ensure(prec);
   TuneScope scope(tuned_for(prec, B));  // the launch choices the sweeps use
   return prec == 1 ? time_kernel_impl<float>(*this, which, prec, B, iters, true)
                    : time_kernel_impl<double>(*this, which, prec, B, iters, true);
