@@ -22,6 +22,11 @@ void convert_d2f_off(long long n, const double *src, double off, float *dst, cud
   launch_k(k_convert_off, launch_cfg(n), s, n, src, off, dst);
 }
 
+void members_resize(long long n, int Bd, double *dst, int Bs, const double *src, cudaStream_t s) {
+  g_launches++;
+  launch_k(k_members_resize, launch_cfg(n * Bd), s, n, Bd, dst, Bs, src);
+}
+
 void convert_list(const ConvList &L, long long max_n, cudaStream_t s) {
   g_launches++;
   launch_k(k_convert_list, launch_cfg(max_n), s, L);

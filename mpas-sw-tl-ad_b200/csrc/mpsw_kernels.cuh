@@ -417,6 +417,14 @@ __global__ void k_convert(long long n, const S *__restrict__ src, D *dst) {
   MPSW_GRID_LOOP(t, n) dst[t] = D(src[t]);
 }
 
+static __global__ void k_members_resize(long long n, int Bd, double *dst, int Bs, const double *__restrict__ src) {
+  MPSW_GRID_LOOP(t, n * Bd) {
+    const long long i = t / Bd;
+    const int b = (int)(t - i * Bd);
+    dst[t] = b < Bs ? src[i * Bs + b] : 0.0;
+  }
+}
+
 // Rounds up to kConvMax double arrays to float in one launch (linearisation point of a stage).
 // dst = float(src - off): reduced-precision h relative to a reference depth
 static __global__ void k_convert_off(long long n, const double *src, double off, float *dst) {

@@ -106,6 +106,8 @@ struct Launch {
 
 void convert_d2f(long long n, const double *src, float *dst, cudaStream_t s);
 void convert_d2f_off(long long n, const double *src, double off, float *dst, cudaStream_t s);
+// rows of Bd doubles from rows of Bs: the first min(Bd, Bs) copied, the rest zero
+void members_resize(long long n, int Bd, double *dst, int Bs, const double *src, cudaStream_t s);
 void convert_list(const ConvList &L, long long max_n, cudaStream_t s);
 void convert_f2d(long long n, const float *src, double *dst, cudaStream_t s);
 

@@ -28,6 +28,16 @@ namespace {
 
 using L64 = Launch<double, double>;
 
+// Members a sweep of B members runs with: counts that are no multiple of a thread's vector width
+// would move one member at a time, so the engine's own buffers hold a few zero members more.
+// Level 6, 6 steps, ms a tangent-linear / adjoint pair: FP32 members 28 -> 6.09, 32 -> 5.79; 36 ->
+// 7.63, 40 -> 7.43; 12 -> 3.80, 16 -> 3.98; 13 one at a time 6.22, padded 4.13.  FP64 3 -> 3.75, 4 -> 3.24; 10 ->
+// 6.21, 12 -> 6.06; 5 -> 4.62, 6 -> 4.79, 8 -> 4.88 (5 and 6 stay).
+int padded_members(int prec, int B) {
+  if (prec == 1) return B <= 2 ? B : B <= 4 ? 4 : (B + 7) / 8 * 8;
+  return B <= 2 || B == 5 || B == 6 ? B : (B + 3) / 4 * 4;
+}
+
 template <typename R>
 struct MemberBufs {
   Diag<R> d{};
@@ -618,18 +628,26 @@ static void tl_member_stage(Engine &E, int prec, int B, double *du, double *dh, 
   Launch<R, double>::tl_edge_tend(m, B, bs, uti, hti, d, ph, rut, nullptr, st);
 }
 
-// Copy B members' FP64 states between a caller's buffers and the engine's (internal order).
-static void members_copy(Engine &E, int B, double *dst_u, double *dst_h, const double *src_u, const double *src_h) {
-  cuda_check(cudaMemcpyAsync(dst_u, src_u, sizeof(double) * E.nE * B, cudaMemcpyDeviceToDevice, E.stream), "members");
-  cuda_check(cudaMemcpyAsync(dst_h, src_h, sizeof(double) * E.nC * B, cudaMemcpyDeviceToDevice, E.stream), "members");
+// Copy members' FP64 states between a caller's buffers and the engine's (internal order): rows of
+// Bd members from rows of Bs, zeros past the source's.
+static void members_copy(Engine &E, int Bd, double *dst_u, double *dst_h, int Bs, const double *src_u,
+                         const double *src_h) {
+  if (Bd != Bs) {
+    members_resize(E.nE, Bd, dst_u, Bs, src_u, E.stream);
+    members_resize(E.nC, Bd, dst_h, Bs, src_h, E.stream);
+    return;
+  }
+  cuda_check(cudaMemcpyAsync(dst_u, src_u, sizeof(double) * E.nE * Bd, cudaMemcpyDeviceToDevice, E.stream), "members");
+  cuda_check(cudaMemcpyAsync(dst_h, src_h, sizeof(double) * E.nC * Bd, cudaMemcpyDeviceToDevice, E.stream), "members");
 }
 
 template <typename R>
-static void window_tl_impl(Engine &E, int prec, int B, double *user_u, double *user_h) {
+static void window_tl_impl(Engine &E, int prec, int Bu, double *user_u, double *user_h) {
+  const int B = padded_members(prec, Bu);
   Window &W = E.win;
   MemberBufs<R> *mb = members<R>(E, prec, B, E.stream);
   double *du = W.ms[prec].x_u, *dh = W.ms[prec].x_h;
-  members_copy(E, B, du, dh, user_u, user_h);
+  members_copy(E, B, du, dh, Bu, user_u, user_h);
   const Phys<double> ph64 = E.phys();
   const Phys<R> ph = phys_as<R>(ph64);
   double w[4], c[4];
@@ -663,7 +681,7 @@ static void window_tl_impl(Engine &E, int prec, int B, double *user_u, double *u
       cuda_check(cudaStreamWaitEvent(E.stream, E.ev_join, 0), "event wait");
     });
     window_forward_done(E);
-    members_copy(E, B, user_u, user_h, du, dh);
+    members_copy(E, Bu, user_u, user_h, B, du, dh);
     cuda_check(cudaGetLastError(), "window_tl");
     return;
   }
@@ -692,7 +710,7 @@ static void window_tl_impl(Engine &E, int prec, int B, double *user_u, double *u
         });
       });
   }
-  members_copy(E, B, user_u, user_h, du, dh);
+  members_copy(E, Bu, user_u, user_h, B, du, dh);
   cuda_check(cudaGetLastError(), "window_tl");
 }
 
@@ -743,12 +761,13 @@ static void ad_member_step(Engine &E, int prec, int B, double *au, double *ah, M
 }
 
 template <typename R>
-static void window_ad_impl(Engine &E, int prec, int B, double *user_u, double *user_h) {
+static void window_ad_impl(Engine &E, int prec, int Bu, double *user_u, double *user_h) {
+  const int B = padded_members(prec, Bu);
   Window &W = E.win;
   MemberBufs<R> *mb = members<R>(E, prec, B, E.stream);
   double *au = W.ms[prec].x_u, *ah = W.ms[prec].x_h;
   W.forward_steps = 0;
-  members_copy(E, B, au, ah, user_u, user_h);
+  members_copy(E, B, au, ah, Bu, user_u, user_h);
   const MeshDev<R> &m = mesh_for<R>(E);
   const Phys<double> ph64 = E.phys();
   const Phys<R> ph = phys_as<R>(ph64);
@@ -777,7 +796,7 @@ static void window_ad_impl(Engine &E, int prec, int B, double *user_u, double *u
       for (int n = W.nsteps - 1; n >= 0; n--)
         ad_member_step<R>(E, prec, B, au, ah, mb, ph, w, c, [&](int k) { return stored_base<R>(W, prec, n, k); });
     });
-    members_copy(E, B, user_u, user_h, au, ah);
+    members_copy(E, Bu, user_u, user_h, B, au, ah);
     cuda_check(cudaGetLastError(), "window_ad");
     return;
   }
@@ -823,7 +842,7 @@ static void window_ad_impl(Engine &E, int prec, int B, double *user_u, double *u
       rev(a, m, s, su, sh);
     };
     rev(0, W.nsteps, W.snaps, W.ck_u[0], W.ck_h[0]);
-    members_copy(E, B, user_u, user_h, au, ah);
+    members_copy(E, Bu, user_u, user_h, B, au, ah);
     cuda_check(cudaGetLastError(), "window_ad");
     return;
   }
@@ -842,7 +861,7 @@ static void window_ad_impl(Engine &E, int prec, int B, double *user_u, double *u
       adjoint_step();  // recomputes this step's four stages, then their adjoints
     }
   }
-  members_copy(E, B, user_u, user_h, au, ah);
+  members_copy(E, Bu, user_u, user_h, B, au, ah);
   cuda_check(cudaGetLastError(), "window_ad");
 }
 
@@ -866,7 +885,7 @@ void Engine::window_tl(int prec, int B, double *du, double *dh, cudaStream_t s) 
   if (mesh_dirty) throw EngineError(MPSW_ERR_STATE, "mesh changed since mpsw_window_init");
   if (prec != 0 && prec != 1) throw EngineError(MPSW_ERR_ARG, "precision must be 0 or 1");
   join(s, stream, true);
-  TuneScope scope(tuning(prec, B));
+  TuneScope scope(tuning(prec, padded_members(prec, B)));
   nonfinite_clear();  // after the autotuner, whose timings run on arbitrary buffer contents
   if (prec == 0) window_tl_impl<double>(*this, prec, B, du, dh);
   else window_tl_impl<float>(*this, prec, B, du, dh);
@@ -881,7 +900,7 @@ void Engine::window_ad(int prec, int B, double *au, double *ah, cudaStream_t s) 
   if (prec != 0 && prec != 1) throw EngineError(MPSW_ERR_ARG, "precision must be 0 or 1");
   join(s, stream, true);
   window_ensure(prec);
-  TuneScope scope(tuning(prec, B));
+  TuneScope scope(tuning(prec, padded_members(prec, B)));
   nonfinite_clear();  // after the autotuner, whose timings run on arbitrary buffer contents
   if (prec == 0) window_ad_impl<double>(*this, prec, B, au, ah);
   else window_ad_impl<float>(*this, prec, B, au, ah);
@@ -1031,6 +1050,7 @@ double Engine::time_kernel(int which, int prec, int B, int iters) {
   if (!win.nsteps) throw EngineError(MPSW_ERR_STATE, "mpsw_window_init has not been called");
   if (which < 0 || which > 9 || B < 1 || iters < 1) throw EngineError(MPSW_ERR_ARG, "bad kernel timing request");
   window_ensure(prec);
+  B = padded_members(prec, B);
   TuneScope scope(tuned_for(prec, B));  // the launch choices the sweeps use
   return prec == 1 ? time_kernel_impl<float>(*this, which, prec, B, iters, true)
                    : time_kernel_impl<double>(*this, which, prec, B, iters, true);
@@ -1149,7 +1169,7 @@ int mpsw_window_tuning(mpsw_handle *h, int precision, int B, int *v_block) {
   return mpsw::guarded(h, [&](mpsw::Engine &e) {
     if (!v_block) throw mpsw::EngineError(MPSW_ERR_ARG, "null output");
     if (precision != 0 && precision != 1) throw mpsw::EngineError(MPSW_ERR_ARG, "precision must be 0 or 1");
-    const mpsw::TuneTable *t = e.tuned_for(precision, B);
+    const mpsw::TuneTable *t = e.tuned_for(precision, mpsw::padded_members(precision, B));
     for (int k = 0; k < mpsw::K_TUNED; k++) {
       v_block[2 * k] = t ? t->k[k].v : 0;
       v_block[2 * k + 1] = t ? t->k[k].block : 0;
@@ -1163,7 +1183,7 @@ int mpsw_window_fused(mpsw_handle *h, int precision, int B, int *members_per_blo
     if (B < 1) throw mpsw::EngineError(MPSW_ERR_ARG, "B must be positive");
     e.prepare();
     *members_per_block =
-        precision == 1 ? mpsw::fused_members<float>(e, B, mpsw::phys_as<float>(e.phys())) : 0;
+        precision == 1 ? mpsw::fused_members<float>(e, mpsw::padded_members(precision, B), mpsw::phys_as<float>(e.phys())) : 0;
     *tile_cells = *members_per_block ? e.fused_K : 0;
   });
 }
