@@ -13,6 +13,8 @@
 #include <cmath>
 #include <cctype>
 #include <cstring>
+#include <system_error>
+#include <thread>
 #include <map>
 #include <memory>
 #include <stdexcept>
@@ -198,19 +200,26 @@ void Engine::need_device() {
   for (cudaEvent_t *ev : {&ev_fork, &ev_step, &ev_join})
     cuda_check(cudaEventCreateWithFlags(ev, cudaEventDisableTiming), "cudaEventCreate");
   cuda_check(cudaMalloc(&d_bad, sizeof(int)), "cudaMalloc flag");
+  cuda_check(cudaMallocHost(&h_bad, sizeof(int)), "cudaMallocHost flag");
   cuda_check(cudaMemsetAsync(d_bad, 0, sizeof(int), stream), "clear flag");
 }
 
 Engine::~Engine() {
   if (stream) cudaStreamSynchronize(stream);
-  for (auto &v : vars)
+  copies_pending = false;
+  for (auto &v : vars) {
+    unpin(v);
     if (v.dev) cudaFree(v.dev);
+  }
+  cudaFree(d_transfer);
+  if (d_mean) cudaFree(d_mean);
   free_device_mesh();
   for (void *p : work) cudaFree(p);
   if (trc) cudaFree(trc);
   window_free();
   if (l2_flush) cudaFree(l2_flush);
   if (d_bad) cudaFree(d_bad);
+  if (h_bad) cudaFreeHost(h_bad);
   for (cudaEvent_t ev : {ev_fork, ev_step, ev_join})
     if (ev) cudaEventDestroy(ev);
   if (side) cudaStreamDestroy(side);
@@ -259,6 +268,7 @@ void Engine::allocate_group(int g) {
     long long n = 1;
     for (auto x : v.dims) n *= x;
     v.count = n;
+    unpin(v);
     if (v.is_int) v.hi.assign(n, 0); else v.hr.assign(n, 0.0);
     v.allocated = true;
     v.host_valid = true;
@@ -283,41 +293,111 @@ const std::vector<int> &Engine::perm_of(int ent) const {
   return ent == 1 ? bm.perm_c : ent == 2 ? bm.perm_e : bm.perm_v;
 }
 
+// Host mirrors that cross more than once are page-locked, so the copies are plain DMA; the
+// renumbering (and the split of the interleaved time levels) runs on the device.
+void Engine::pin(Var &v) {
+  if (v.pinned || ++v.crossings < 3 || v.hr.empty()) return;
+  if (cudaHostRegister(v.hr.data(), sizeof(double) * v.hr.size(), cudaHostRegisterDefault) == cudaSuccess) v.pinned = true;
+  else (void)cudaGetLastError();  // pageable copies work too
+}
+void Engine::unpin(Var &v) {
+  if (!v.pinned) return;
+  copies_done();
+  cudaHostUnregister(v.hr.data());
+  v.pinned = false;
+}
+// wait for the copies that still read or write host mirrors
+void Engine::copies_done() {
+  if (!copies_pending) return;
+  cuda_check(cudaStreamSynchronize(stream), "host copies");
+  copies_pending = false;
+}
+double *Engine::transfer_buffer(size_t n) {
+  if (n > d_transfer_n) {
+    if (d_transfer) cuda_check(cudaStreamSynchronize(stream), "transfer buffer");
+    cudaFree(d_transfer);
+    d_transfer = nullptr;
+    d_transfer_n = 0;
+    cuda_check(cudaMalloc(&d_transfer, sizeof(double) * n), "cudaMalloc transfer buffer");
+    d_transfer_n = n;
+  }
+  return d_transfer;
+}
+
 void Engine::upload(Var &v) {
   if (!v.ent || (v.dev && v.dev_valid)) return;
   if (!v.dev) v.dev = (double *)dalloc(sizeof(double) * v.count);
   if (!mesh_built) throw EngineError(MPSW_ERR_STATE, "mesh not initialised (call sw_mpas_init_block)");
-  const auto &p = perm_of(v.ent);
-  const long long n = (long long)p.size();
-  staging.resize(v.count);
-  for (long long i = 0; i < n; i++)
-    for (int l = 0; l < v.lead; l++) staging[(size_t)l * n + p[i]] = v.hr[(size_t)l + (size_t)v.lead * i];
-  cuda_check(cudaMemcpyAsync(v.dev, staging.data(), sizeof(double) * v.count, cudaMemcpyHostToDevice, stream), "upload");
-  cuda_check(cudaStreamSynchronize(stream), "upload sync");
+  pin(v);
+  double *t = transfer_buffer(v.count);
+  copies_pending = true;
+  cuda_check(cudaMemcpyAsync(t, v.hr.data(), sizeof(double) * v.count, cudaMemcpyHostToDevice, stream), "upload");
+  var_to_internal((int)perm_of(v.ent).size(), v.lead, d_perm[v.ent - 1], t, v.dev, stream);
+  cuda_check(cudaGetLastError(), "upload");
   v.dev_valid = true;
 }
 
-void Engine::download(Var &v) {
+// Start the copy of v's device value into its mirror; copies_done() finishes it.
+void Engine::download_start(Var &v) {
   if (!v.ent || v.host_valid) return;
-  const auto &p = perm_of(v.ent);
-  const long long n = (long long)p.size();
-  staging.resize(v.count);
-  cuda_check(cudaMemcpyAsync(staging.data(), v.dev, sizeof(double) * v.count, cudaMemcpyDeviceToHost, stream), "download");
-  cuda_check(cudaStreamSynchronize(stream), "download sync");
-  for (long long i = 0; i < n; i++)
-    for (int l = 0; l < v.lead; l++) v.hr[(size_t)l + (size_t)v.lead * i] = staging[(size_t)l * n + p[i]];
+  pin(v);
+  double *t = transfer_buffer(v.count);
+  copies_pending = true;
+  var_to_reference((int)perm_of(v.ent).size(), v.lead, d_perm[v.ent - 1], v.dev, t, stream);
+  cuda_check(cudaGetLastError(), "download");
+  cuda_check(cudaMemcpyAsync(v.hr.data(), t, sizeof(double) * v.count, cudaMemcpyDeviceToHost, stream), "download");
   v.host_valid = true;
 }
+void Engine::download(Var &v) {
+  if (!v.ent || v.host_valid) return;
+  v.host_valid = false;
+  download_start(v);
+  copies_done();
+}
 
-void Engine::set_var(const char *name, const void *src, long long count) {
+// memcpy / memcmp of large arrays over a few threads
+template <typename F>
+static void in_parts(size_t bytes, F &&f) {
+  constexpr size_t kPart = (size_t)2 << 20;
+  const int parts = (int)std::min<size_t>(4, bytes / kPart);
+  if (parts < 2) {
+    f(0, 0, bytes);
+    return;
+  }
+  std::vector<std::thread> ts;
+  const size_t step = (bytes / parts + 63) / 64 * 64;
+  auto part = [&](int i) { f(i, i * step, i + 1 < parts ? (i + 1) * step : bytes); };
+  int i = 1;
+  try {
+    for (; i < parts; i++) ts.emplace_back(part, i);
+  } catch (const std::system_error &) {  // no more threads: the rest here
+  }
+  for (; i < parts; i++) part(i);
+  part(0);
+  for (auto &t : ts) t.join();
+}
+static void copy_bytes(void *dst, const void *src, size_t bytes) {
+  in_parts(bytes, [=](int, size_t a, size_t b) { std::memcpy((char *)dst + a, (const char *)src + a, b - a); });
+}
+static bool same_bytes(const void *x, const void *y, size_t bytes) {
+  bool eq[4] = {true, true, true, true};
+  in_parts(bytes, [&](int i, size_t a, size_t b) { eq[i] = !std::memcmp((const char *)x + a, (const char *)y + a, b - a); });
+  return eq[0] && eq[1] && eq[2] && eq[3];
+}
+
+void Engine::set_var(const char *name, const void *src, long long count, bool if_changed) {
   Var &v = var(name);
   if (!v.allocated) throw EngineError(MPSW_ERR_STATE, std::string(name) + " is not allocated");
   if (count != v.count) throw EngineError(MPSW_ERR_ARG, std::string(name) + ": element count mismatch");
   if (!src && count) throw EngineError(MPSW_ERR_ARG, "null source buffer");
+  copies_done();
   if (v.is_int) {
+    if (if_changed && same_bytes(v.hi.data(), src, sizeof(int) * count)) return;
     std::memcpy(v.hi.data(), src, sizeof(int) * count);
   } else {
-    std::memcpy(v.hr.data(), src, sizeof(double) * count);
+    // (the mirror holds what was last exchanged with the caller)
+    if (if_changed && same_bytes(v.hr.data(), src, sizeof(double) * count)) return;
+    copy_bytes(v.hr.data(), src, sizeof(double) * count);
     v.nonzero = std::any_of(v.hr.begin(), v.hr.end(), [](double x) { return x != 0.0; });
   }
   v.host_valid = true;
@@ -325,18 +405,26 @@ void Engine::set_var(const char *name, const void *src, long long count) {
   if (v.mesh) mesh_dirty = true;
 }
 
-void Engine::get_var(const char *name, void *dst, long long count) {
-  Var &v = var(name);
-  if (!v.allocated) throw EngineError(MPSW_ERR_STATE, std::string(name) + " is not allocated");
-  if (count != v.count) throw EngineError(MPSW_ERR_ARG, std::string(name) + ": element count mismatch");
-  if (!dst && count) throw EngineError(MPSW_ERR_ARG, "null destination buffer");
-  if (v.ent && !v.host_valid) {
-    if (v.lazy_diag) materialize_pending();
-    download(v);
+void Engine::get_vars(int n, const char *const *names, void *const *dst, const long long *counts) {
+  for (int i = 0; i < n; i++) {
+    Var &v = var(names[i]);
+    if (!v.allocated) throw EngineError(MPSW_ERR_STATE, std::string(names[i]) + " is not allocated");
+    if (counts[i] != v.count) throw EngineError(MPSW_ERR_ARG, std::string(names[i]) + ": element count mismatch");
+    if (!dst[i] && counts[i]) throw EngineError(MPSW_ERR_ARG, "null destination buffer");
   }
-  if (v.is_int) std::memcpy(dst, v.hi.data(), sizeof(int) * count);
-  else std::memcpy(dst, v.hr.data(), sizeof(double) * count);
+  for (int i = 0; i < n; i++) {
+    Var &v = var(names[i]);
+    if (v.ent && !v.host_valid && v.lazy_diag) materialize_pending();
+  }
+  for (int i = 0; i < n; i++) download_start(var(names[i]));
+  copies_done();
+  for (int i = 0; i < n; i++) {
+    Var &v = var(names[i]);
+    if (v.is_int) std::memcpy(dst[i], v.hi.data(), sizeof(int) * counts[i]);
+    else copy_bytes(dst[i], v.hr.data(), sizeof(double) * counts[i]);
+  }
 }
+void Engine::get_var(const char *name, void *dst, long long count) { get_vars(1, &name, &dst, &count); }
 
 void Engine::mark_written(Var &v, bool maybe_nonzero) {
   v.dev_valid = true;
@@ -662,10 +750,10 @@ void Engine::nonfinite_clear() {
 }
 void Engine::nonfinite_check(const char *what) {
   if (!d_bad) return;
-  int v = 0;
-  cuda_check(cudaMemcpyAsync(&v, d_bad, sizeof(int), cudaMemcpyDeviceToHost, stream), "read non-finite flag");
+  cuda_check(cudaMemcpyAsync(h_bad, d_bad, sizeof(int), cudaMemcpyDeviceToHost, stream), "read non-finite flag");
   cuda_check(cudaStreamSynchronize(stream), what);
-  if (v)
+  copies_pending = false;
+  if (*h_bad)
     throw EngineError(MPSW_ERR_NONFINITE, std::string(what) +
                                               ": a tendency became non-finite (NaN or Inf); the state or the "
                                               "members are corrupt or the time step is unstable");
@@ -745,6 +833,7 @@ void Engine::tl_diag_run(const Base<double> &bs, const double *ut, const double 
 void Engine::check_launch(const char *what) {
   cuda_check(cudaGetLastError(), what);
   cuda_check(cudaStreamSynchronize(stream), what);
+  copies_pending = false;
 }
 
 // Lazily computed diagnostics of the state left by the last routine (the reference's final
@@ -913,7 +1002,7 @@ void Engine::rk4(int nsteps) {  // src/mpas_sw_module.f90:528-635
   finish_levels({"u", "h"});
   L64::recon(m64, 1, ph.sphere, u0, dv("uReconstructX"), dv("uReconstructY"), dv("uReconstructZ"),
              dv("uReconstructZonal"), dv("uReconstructMeridional"), stream);
-  check_launch("sw_rk4");
+  cuda_check(cudaGetLastError(), "sw_rk4");
   for (const char *n : {"u", "h", "tend_u", "tend_h"}) mark_written(var(n), true);
   mark_recon(0);
   mark_diag(0, true);
@@ -946,11 +1035,11 @@ void Engine::forward(int prec, int nsteps) {
   rk_coeffs(ph64.dt, w, c);
   double *u0 = dv("u"), *h0 = dv("h");
   // reference depth: the mean of h(1), rounded to a whole metre (exact in FP32)
-  staging.resize(nC);
-  cuda_check(cudaMemcpyAsync(staging.data(), h0, sizeof(double) * nC, cudaMemcpyDeviceToHost, stream), "h download");
-  cuda_check(cudaStreamSynchronize(stream), "h download");
+  if (!d_mean) cuda_check(cudaMalloc(&d_mean, sizeof(double) * (kSumParts + 1)), "cudaMalloc mean");
+  sum_of(nC, h0, d_mean, stream);
   double sum = 0;
-  for (int i = 0; i < nC; i++) sum += staging[i];
+  cuda_check(cudaMemcpyAsync(&sum, d_mean, sizeof(double), cudaMemcpyDeviceToHost, stream), "h mean");
+  cuda_check(cudaStreamSynchronize(stream), "h mean");
   const double off = nC ? std::round(sum / nC) : 0.0;
   const float offf = (float)off;
   using L32 = Launch<float, double>;
@@ -980,7 +1069,7 @@ void Engine::forward(int prec, int nsteps) {
   finish_levels({"u", "h"});
   L64::recon(m64, 1, ph64.sphere, u0, dv("uReconstructX"), dv("uReconstructY"), dv("uReconstructZ"),
              dv("uReconstructZonal"), dv("uReconstructMeridional"), stream);
-  check_launch("forward");
+  cuda_check(cudaGetLastError(), "forward");
   for (const char *n : {"u", "h"}) mark_written(var(n), true);
   mark_recon(0);
   mark_diag(0, true);
@@ -1004,7 +1093,7 @@ void Engine::rk4_tlm(int nsteps) {  // src/mpas_sw_module.f90:637-781
   double w[4], c[4];
   rk_coeffs(ph.dt, w, c);
   double *u0 = dv("u"), *h0 = dv("h"), *ut0 = dv("u_tl"), *ht0 = dv("h_tl");
-  for (int step = 0; step < nsteps; step++) {
+  auto step = [&]() {
     for (int k = 0; k < 4; k++) {
       const double *ui = k == 0 ? u0 : sp_u[k - 1];
       const double *hi = k == 0 ? h0 : sp_h[k - 1];
@@ -1023,13 +1112,14 @@ void Engine::rk4_tlm(int nsteps) {  // src/mpas_sw_module.f90:637-781
       if (ph.visc4 > 0) L64::del4_vc(m64, 1, tl_diag.dsq_u, tl_diag.dsq_vort, tl_diag.dsq_div, stream);
       L64::tl_edge_tend(m64, 1, bs, uti, hti, tl_diag, ph, rut, k == 3 ? dv("tend_u_tl") : nullptr, stream);
     }
-  }
+  };
+  for (int n = 0; n < nsteps; n++) run_graph(graph_key(10, 0, 1, u0, ut0), step);
   finish_levels({"u", "h", "u_tl", "h_tl"});
   L64::recon(m64, 1, ph.sphere, u0, dv("uReconstructX"), dv("uReconstructY"), dv("uReconstructZ"),
              dv("uReconstructZonal"), dv("uReconstructMeridional"), stream);
   L64::recon(m64, 1, ph.sphere, ut0, dv("uReconstructX_tl"), dv("uReconstructY_tl"), dv("uReconstructZ_tl"),
              dv("uReconstructZonal_tl"), dv("uReconstructMeridional_tl"), stream);
-  check_launch("sw_rk4_tlm");
+  cuda_check(cudaGetLastError(), "sw_rk4_tlm");
   for (const char *n : {"u", "h", "tend_u", "tend_h", "u_tl", "h_tl", "tend_u_tl", "tend_h_tl"}) mark_written(var(n), true);
   mark_recon(0);
   mark_recon(1);
@@ -1058,12 +1148,12 @@ AdSeeds<double> Engine::seeds(bool *any) {
 void Engine::zero_ad_seeds() {
   for (int i = 0; i < 19; i++) {
     Var &v = var((std::string(kDiagNames[i]) + "_ad").c_str());
-    cuda_check(cudaMemsetAsync(v.dev, 0, sizeof(double) * v.count, stream), "memset");
+    if (v.nonzero || !v.dev_valid) cuda_check(cudaMemsetAsync(v.dev, 0, sizeof(double) * v.count, stream), "memset");
     mark_written(v, false);
   }
   for (const char *n : {"tend_u_ad", "tend_h_ad"}) {
     Var &v = var(n);
-    cuda_check(cudaMemsetAsync(v.dev, 0, sizeof(double) * v.count, stream), "memset");
+    if (v.nonzero || !v.dev_valid) cuda_check(cudaMemsetAsync(v.dev, 0, sizeof(double) * v.count, stream), "memset");
     mark_written(v, false);
   }
 }
@@ -1082,6 +1172,7 @@ void Engine::rk4_adj() {  // src/mpas_sw_module.f90:783-1002
   rk_coeffs(ph.dt, w, c);
   double *u0 = dv("u"), *h0 = dv("h"), *u2 = dv("u", 1), *h2 = dv("h", 1);
   // forward sweep, keeping the diagnostics of every stage (:815-878)
+  run_graph(graph_key(11, 0, 1, u0, h0), [&]() {
   for (int k = 0; k < 4; k++) {
     const double *ui = k == 0 ? u0 : sp_u[k - 1];
     const double *hi = k == 0 ? h0 : sp_h[k - 1];
@@ -1093,6 +1184,7 @@ void Engine::rk4_adj() {  // src/mpas_sw_module.f90:783-1002
   cuda_check(cudaMemcpyAsync(h2, acc_h, sizeof(double) * nC, cudaMemcpyDeviceToDevice, stream), "h(2)");
   L64::recon(m64, 1, ph.sphere, u0, dv("uReconstructX"), dv("uReconstructY"), dv("uReconstructZ"),
              dv("uReconstructZonal"), dv("uReconstructMeridional"), stream);
+  });
   double *ua = dv("u_ad"), *ha = dv("h_ad");
   // adjoint of the output reconstruction and diagnostics at x(2) (:887-905)
   if (recon_seeds_nonzero())
@@ -1112,6 +1204,9 @@ void Engine::rk4_adj() {  // src/mpas_sw_module.f90:783-1002
   // tendency adjoint of stage 4 (:913-914), with any seed left in tend_*_ad
   const double *stu = var("tend_u_ad").nonzero ? dv("tend_u_ad") : nullptr;
   const double *sth = var("tend_h_ad").nonzero ? dv("tend_h_ad") : nullptr;
+  GraphKey key = graph_key(12, 0, 1, ua, ha);
+  key.n2 = (stu ? 1 : 0) | (sth ? 2 : 0);
+  run_graph(key, [&]() {
   L64::ad_tinit(m64, 1, ua, ha, ph.tc1 ? nullptr : stu, sth, ph.tc1 ? 0.0 : w[3], w[3], tu_[0], th_[0], stream);
   AdSeeds<double> none{};
   for (int k = 3; k >= 0; k--) {  // :912-970
@@ -1133,8 +1228,9 @@ void Engine::rk4_adj() {  // src/mpas_sw_module.f90:783-1002
   }
   cuda_check(cudaMemsetAsync(dv("u_ad", 1), 0, sizeof(double) * nE, stream), "memset");
   cuda_check(cudaMemsetAsync(dv("h_ad", 1), 0, sizeof(double) * nC, stream), "memset");
+  });
   zero_ad_seeds();
-  check_launch("sw_rk4_adj");
+  cuda_check(cudaGetLastError(), "sw_rk4_adj");
   for (const char *n : {"u", "h", "u_ad", "h_ad"}) mark_written(var(n), true);
   mark_recon(0);
   mark_diag(0, true);
@@ -1291,6 +1387,17 @@ int mpsw_var_info(mpsw_handle *h, const char *name, int *rank, long long dims[4]
 
 int mpsw_set_var(mpsw_handle *h, const char *name, const void *src, long long count) {
   return mpsw::guarded(h, [&](mpsw::Engine &e) { e.set_var(name, src, count); });
+}
+
+int mpsw_update_var(mpsw_handle *h, const char *name, const void *src, long long count) {
+  return mpsw::guarded(h, [&](mpsw::Engine &e) { e.set_var(name, src, count, true); });
+}
+
+int mpsw_get_vars(mpsw_handle *h, int n, const char *const *names, void *const *dst, const long long *counts) {
+  return mpsw::guarded(h, [&](mpsw::Engine &e) {
+    if (n < 0 || (n && (!names || !dst || !counts))) throw mpsw::EngineError(MPSW_ERR_ARG, "null argument");
+    e.get_vars(n, names, dst, counts);
+  });
 }
 
 int mpsw_get_var(mpsw_handle *h, const char *name, void *dst, long long count) {

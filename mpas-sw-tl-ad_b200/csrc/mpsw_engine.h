@@ -37,6 +37,8 @@ struct Var {
   double *dev = nullptr;  // [lead][n] internal order (state, diagnostics, tendencies)
   bool allocated = false, host_valid = true, dev_valid = true;
   bool nonzero = false;    // may hold nonzero values (adjoint seeds are skipped when false)
+  bool pinned = false;     // hr is page-locked
+  int crossings = 0;       // transfers so far
   bool lazy_diag = false;  // device value is produced on demand from the level-1 state
 };
 
@@ -173,7 +175,17 @@ struct Engine {
   const std::vector<int> &perm_of(int ent) const;
   void upload(Var &v);
   void download(Var &v);
-  void set_var(const char *name, const void *src, long long count);
+  void pin(Var &v);
+  void unpin(Var &v);
+  void copies_done();
+  double *transfer_buffer(size_t n);
+  bool copies_pending = false;   // copies from or to host mirrors not yet waited for
+  double *d_transfer = nullptr;  // a variable in the reference layout on its way in or out
+  size_t d_transfer_n = 0;
+  double *d_mean = nullptr;
+  void download_start(Var &v);
+  void set_var(const char *name, const void *src, long long count, bool if_changed = false);
+  void get_vars(int n, const char *const *names, void *const *dst, const long long *counts);
   void get_var(const char *name, void *dst, long long count);
   void mark_written(Var &v, bool maybe_nonzero);
   template <typename T, typename S>
@@ -206,6 +218,7 @@ struct Engine {
   void tl_diag_run(const Base<double> &bs, const double *ut, const double *ht, const Diag<double> &d,
                    const Phys<double> &ph);
   void check_launch(const char *what);
+  int *h_bad = nullptr;  // its page-locked copy
   int *d_bad = nullptr;  // non-finite flag of the tendency kernels (Phys::bad)
   void nonfinite_clear();
   void nonfinite_check(const char *what);

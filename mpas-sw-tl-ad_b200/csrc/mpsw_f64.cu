@@ -27,6 +27,20 @@ void members_resize(long long n, int Bd, double *dst, int Bs, const double *src,
   launch_k(k_members_resize, launch_cfg(n * Bd), s, n, Bd, dst, Bs, src);
 }
 
+void var_to_internal(int n, int lead, const int *perm, const double *src, double *dst, cudaStream_t s) {
+  g_launches++;
+  launch_k(k_var_in, launch_cfg((long long)n * lead), s, n, lead, perm, src, dst);
+}
+void var_to_reference(int n, int lead, const int *perm, const double *src, double *dst, cudaStream_t s) {
+  g_launches++;
+  launch_k(k_var_out, launch_cfg((long long)n * lead), s, n, lead, perm, src, dst);
+}
+void sum_of(long long n, const double *x, double *out, cudaStream_t s) {
+  g_launches += 2;
+  launch_k(k_sum, LaunchCfg{kSumParts, 256, 0}, s, n, x, out + 1);
+  launch_k(k_sum, LaunchCfg{1, 256, 0}, s, (long long)kSumParts, (const double *)(out + 1), out);
+}
+
 void convert_list(const ConvList &L, long long max_n, cudaStream_t s) {
   g_launches++;
   launch_k(k_convert_list, launch_cfg(max_n), s, L);

@@ -417,6 +417,36 @@ __global__ void k_convert(long long n, const S *__restrict__ src, D *dst) {
   MPSW_GRID_LOOP(t, n) dst[t] = D(src[t]);
 }
 
+static __global__ void k_var_in(int n, int lead, const int *__restrict__ perm, const double *__restrict__ src,
+                                double *dst) {
+  MPSW_GRID_LOOP(t, (long long)n * lead) {
+    const int i = (int)(t / lead), l = (int)(t - (long long)i * lead);
+    dst[(size_t)l * n + perm[i]] = src[t];
+  }
+}
+static __global__ void k_var_out(int n, int lead, const int *__restrict__ perm, const double *__restrict__ src,
+                                 double *dst) {
+  MPSW_GRID_LOOP(t, (long long)n * lead) {
+    const int i = (int)(t / lead), l = (int)(t - (long long)i * lead);
+    dst[t] = src[(size_t)l * n + perm[i]];
+  }
+}
+// one partial sum a block, over a fixed split (blocks of 256 threads)
+static __global__ void k_sum(long long n, const double *__restrict__ x, double *out) {
+  __shared__ double s[256];
+  pdl_begin();
+  const long long part = (n + gridDim.x - 1) / gridDim.x, a = part * blockIdx.x, b = a + part < n ? a + part : n;
+  double v = 0.0;
+  for (long long i = a + threadIdx.x; i < b; i += 256) v += x[i];
+  s[threadIdx.x] = v;
+  __syncthreads();
+  for (int k = 128; k > 0; k >>= 1) {
+    if ((int)threadIdx.x < k) s[threadIdx.x] += s[threadIdx.x + k];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) out[blockIdx.x] = s[0];
+}
+
 static __global__ void k_members_resize(long long n, int Bd, double *dst, int Bs, const double *__restrict__ src) {
   MPSW_GRID_LOOP(t, n * Bd) {
     const long long i = t / Bd;

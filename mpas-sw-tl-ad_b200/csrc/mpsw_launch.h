@@ -108,6 +108,12 @@ void convert_d2f(long long n, const double *src, float *dst, cudaStream_t s);
 void convert_d2f_off(long long n, const double *src, double off, float *dst, cudaStream_t s);
 // rows of Bd doubles from rows of Bs: the first min(Bd, Bs) copied, the rest zero
 void members_resize(long long n, int Bd, double *dst, int Bs, const double *src, cudaStream_t s);
+// a module variable's values, [lead] fastest in the reference layout, to and from [lead][n] internal order
+void var_to_internal(int n, int lead, const int *perm, const double *src, double *dst, cudaStream_t s);
+void var_to_reference(int n, int lead, const int *perm, const double *src, double *dst, cudaStream_t s);
+// sum of n values into out[0] (out: kSumParts + 1 values), the same whatever the launch
+constexpr int kSumParts = 148;
+void sum_of(long long n, const double *x, double *out, cudaStream_t s);
 void convert_list(const ConvList &L, long long max_n, cudaStream_t s);
 void convert_f2d(long long n, const float *src, double *dst, cudaStream_t s);
 

@@ -116,6 +116,7 @@ __global__ void k_tc_cell(TcArgs t) {
 void Engine::test_case(int tc) {
   if (!allocated[0]) throw EngineError(MPSW_ERR_STATE, "var_allocation has not been called");
   if (tc != 1 && tc != 2 && tc != 5 && tc != 6) throw EngineError(MPSW_ERR_ARG, "test case must be 1, 2, 5 or 6");
+  copies_done();  // host mirrors are written below
   need_device();
   const double a = sc("a");
   // the unit-sphere mesh scaled by the Earth radius (:173-186 and the same lines of each case)

@@ -77,7 +77,7 @@ class MpasSwModule:
         names = [lib.mpsw_var_name(i).decode() for i in range(lib.mpsw_var_count())]
         d['_canon'] = {n.lower(): n for n in names}
         d['_arr'] = {}         # lower name -> ndarray (Fortran order)
-        d['_synced'] = {}      # lower name -> copy of the content last exchanged with the engine
+        d['_synced'] = set()   # lower names of allocated arrays sent only when their content changed
         d['_stale'] = set()    # lower names to refresh from the engine on next access
         d['_mesh_dirty'] = set()
 
@@ -122,22 +122,18 @@ class MpasSwModule:
     def _push(self, key, force=False):
         d = self.__dict__
         arr = d['_arr'][key]
-        last = d['_synced'].get(key)
-        if not force and last is not None and np.array_equal(last, arr):
-            return
-        ptr = arr.ctypes.data_as(ctypes.c_void_p)
-        d['_h'].call('mpsw_set_var', d['_canon'][key].encode(), ptr, arr.size)
-        if last is not None or key in _TRACKED:
-            d['_synced'][key] = arr.copy(order='F')
+        # the engine keeps what was last exchanged and compares with it
+        routine = 'mpsw_update_var' if key in d['_synced'] and not force else 'mpsw_set_var'
+        d['_h'].call(routine, d['_canon'][key].encode(), ctypes.c_void_p(arr.ctypes.data), arr.size)
 
-    def _pull(self, key):
+    def _pull(self, *keys):
         d = self.__dict__
-        arr = d['_arr'][key]
-        d['_h'].call('mpsw_get_var', d['_canon'][key].encode(), arr.ctypes.data_as(ctypes.c_void_p),
-                     arr.size)
-        d['_stale'].discard(key)
-        if key in d['_synced']:
-            d['_synced'][key] = arr.copy(order='F')
+        n = len(keys)
+        arrs = [d['_arr'][k] for k in keys]
+        d['_h'].call('mpsw_get_vars', n, (ctypes.c_char_p * n)(*[d['_canon'][k].encode() for k in keys]),
+                     (ctypes.c_void_p * n)(*[a.ctypes.data for a in arrs]),
+                     (ctypes.c_longlong * n)(*[a.size for a in arrs]))
+        d['_stale'].difference_update(keys)
 
     def _push_mesh(self, everything=False):
         d = self.__dict__
@@ -163,10 +159,7 @@ class MpasSwModule:
                 if k.lower() in d['_arr']:
                     d['_stale'].add(k.lower())
             raise
-        for k in eager:
-            k = k.lower()
-            if k in d['_arr']:
-                self._pull(k)
+        self._pull(*[k.lower() for k in eager if k.lower() in d['_arr']])
         for k in lazy:
             k = k.lower()
             if k in d['_arr']:
@@ -188,7 +181,7 @@ class MpasSwModule:
             d['_arr'][lname] = np.zeros(shape, dtype=np.int32 if is_int.value else np.float64, order='F')
             d['_stale'].discard(lname)
             if lname in _TRACKED:
-                d['_synced'][lname] = d['_arr'][lname].copy(order='F')
+                d['_synced'].add(lname)
             else:
                 d['_mesh_dirty'].add(lname)
 

@@ -28,6 +28,8 @@ SIGNATURES = {
                                ctypes.POINTER(_c_int), ctypes.POINTER(_c_int)]),
     'mpsw_set_var': (_c_int, [_vp, _cp, _vp, _ll]),
     'mpsw_get_var': (_c_int, [_vp, _cp, _vp, _ll]),
+    'mpsw_update_var': (_c_int, [_vp, _cp, _vp, _ll]),
+    'mpsw_get_vars': (_c_int, [_vp, _c_int, ctypes.POINTER(_cp), ctypes.POINTER(_vp), ctypes.POINTER(_ll)]),
     'mpsw_var_allocation': (_c_int, [_vp]),
     'mpsw_var_allocation_tlm': (_c_int, [_vp]),
     'mpsw_var_allocation_adj': (_c_int, [_vp]),
