@@ -497,6 +497,7 @@ void Engine::free_device_mesh() {
   fused = FusedDev();
   fused_K = 0;
   st64 = st32 = StageDev();
+  rows = RowTab();
 }
 
 // Halo tiles of the fused FP32 member stages (meshes with at most 6 edges per cell and 10
@@ -570,6 +571,26 @@ void Engine::build_stage() {
   cuda_check(Launch<float, double>::stage_prepare(), "nonlinear stage shared-memory limit");
 }
 
+// Tables of the FP32 member-row passes, for meshes whose lists are those of a closed hexagon /
+// pentagon mesh (MPSW_ROWS=0: none, the members then take the general passes).
+void Engine::build_row_tables() {
+  rows = RowTab();
+  const char *off = getenv("MPSW_ROWS");
+  RowTabHost h;
+  if ((off && atoi(off) == 0) || !build_rows(bm, &h).empty()) return;
+  auto &o = mesh_bufs;
+  rows.c_nb = up<int>(h.c_nb, o); rows.c_sp = up<int>(h.c_sp, o); rows.c_va = up<int>(h.c_va, o);
+  rows.c_vb = up<int>(h.c_vb, o); rows.e_q = up<int>(h.e_q, o); rows.e_o1 = up<int>(h.e_o1, o);
+  rows.e_o2 = up<int>(h.e_o2, o); rows.e_t = up<int>(h.e_t, o); rows.e_kr = up<float>(h.e_kr, o);
+  auto F = [&](const std::vector<double> &x) { return up<float>(x, o); };
+  rows.c_g1 = F(h.c_g1); rows.c_g2 = F(h.c_g2); rows.c_g3 = F(h.c_g3); rows.c_n1 = F(h.c_n1); rows.c_n2 = F(h.c_n2);
+  rows.c_m = F(h.c_m); rows.c_t = F(h.c_t); rows.c_q = F(h.c_q); rows.c_r = F(h.c_r); rows.c_ka = F(h.c_ka);
+  rows.c_kb = F(h.c_kb); rows.c_kk = F(h.c_kk); rows.c_r2 = F(h.c_r2); rows.c_r3 = F(h.c_r3); rows.c_ra = F(h.c_ra);
+  rows.e_d = F(h.e_d); rows.e_r4 = F(h.e_r4); rows.e_k = F(h.e_k); rows.e_i1 = F(h.e_i1); rows.e_i2 = F(h.e_i2);
+  rows.e_ke = F(h.e_ke); rows.e_lap = F(h.e_lap); rows.e_lapT = F(h.e_lapT); rows.e_lap0 = F(h.e_lap0);
+  rows.ok = true;
+}
+
 RefMesh Engine::ref_mesh() {
   RefMesh r;
   r.nC = nC; r.nE = nE; r.nV = nV; r.maxEdges = mE; r.maxEdges2 = mE2; r.vd = vd;
@@ -637,6 +658,7 @@ void Engine::build_device_mesh() {
   cuda_check(cudaGetDevice(&mesh_device), "cudaGetDevice");
   build_fused();
   build_stage();
+  build_row_tables();
   noalloc_prepare_device();
   mesh_built = true;
   mesh_dirty = false;

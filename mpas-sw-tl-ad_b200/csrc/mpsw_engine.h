@@ -138,6 +138,8 @@ struct Engine {
   void build_fused();
   StageDev st64, st32;         // halo tiles of the nonlinear stage, FP64 and FP32 stencils
   void build_stage();
+  RowTab rows;                 // tables of the FP32 member-row passes
+  void build_row_tables();
   bool beside_members = false; // the nonlinear stages being launched run beside member kernels
 
   // work

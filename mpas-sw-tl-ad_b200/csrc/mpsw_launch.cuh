@@ -12,6 +12,7 @@
 #include "mpsw_launch.h"
 #include "mpsw_fused.cuh"
 #include "mpsw_members.cuh"
+#include "mpsw_rows.cuh"
 #include "mpsw_stage.cuh"
 
 namespace mpsw {
@@ -487,6 +488,100 @@ void Launch<R, A>::ad_fused(const FusedDev &f, int M, const MeshDev<R> &m, int B
                                           (int)g_stable_base));
   } else {
     throw std::invalid_argument("fused stages run FP32 members only");
+  }
+}
+// ---- member-row passes ---------------------------------------------------------------------------
+// Forming the coefficients costs the same for any member count, so few members take the general
+// passes.  ms a sweep pair (8 steps; level 6: 6 steps), row passes against general ones: 64 members
+// level 4 1.48 / 2.23, level 5 2.7 / 3.1, level 6 8.7 / 10.0; 24 members level 5 2.09 / 2.47, level 6
+// 5.03 / 5.21; 16 members level 4 1.25 / 1.30, level 5 1.89 / 2.11, but level 6 3.98 / 3.88 and its
+// adjoint with recomputed stages, where nothing hides the staging, 14.3 / 13.2; 8 members level 5
+// 1.94 / 1.75.
+template <typename R, typename A>
+bool Launch<R, A>::rows_ok(const RowTab &t, int nE, int B, const Phys<R> &ph, bool adjoint) {
+  if (!std::is_same<R, float>::value || !t.ok || B % 4 || B > 512 || !stage_enabled()) return false;
+  if (B < 16 || (B < 24 && (long long)nE * B > 1000000)) return false;
+  return !adjoint || !(ph.visc2 > R(0) || ph.visc4 > R(0) || ph.wind || ph.drag);
+}
+// Members per thread (8 where the count allows) and block of row pass k; words: staged a entity.
+inline int row_width(KernelId k, int B) {
+  int v = tuned_v(k) >= 4 ? tuned_v(k) : 8;
+  while (B % v || v > 8) v >>= 1;
+  return B / v > 128 ? 8 : v;
+}
+// tiles: neighbouring tiles a block takes (while that leaves enough blocks to fill the SMs).
+inline LaunchCfg row_cfg(KernelId k, int n, int B, int v, int words, int tiles) {
+  const int tpe = B / v;
+  int block = tuned_block(k) ? tuned_block(k) : 64;
+  if (block < tpe) block = tpe <= 64 ? 64 : 128;
+  while (block > tpe && (size_t)words * 4 * (block / tpe) > 48 * 1024) block >>= 1;
+  const int epb = block / tpe;
+  int g = (n + epb - 1) / epb;
+  if (g >= 2048) g = (g + tiles - 1) / tiles;
+  return {g, epb * tpe, (size_t)words * 4 * epb};
+}
+#define MPSW_ROWV(v, ...)                                \
+  if ((v) == 8) { constexpr int VV = 8; __VA_ARGS__; }   \
+  else { constexpr int VV = 4; __VA_ARGS__; }
+
+template <typename R, typename A>
+void Launch<R, A>::row_tl(int part, const MeshDev<R> &m, const RowTab &t, int B, const Base<R> &bs, const R *ut,
+                          const R *ht, const Diag<R> &d, const Phys<R> &ph, const RK<R, A> &rku, const RK<R, A> &rkh,
+                          cudaStream_t s) {
+  if constexpr (std::is_same<R, float>::value && std::is_same<A, double>::value) {
+    g_launches++;
+    const int early = (int)g_stable_base;
+    const bool visc = ph.visc2 > 0.f || ph.visc4 > 0.f;
+    if (part == 0) {
+      const int v = row_width(K_TL_CELL, B);
+      const LaunchCfg c = row_cfg(K_TL_CELL, m.nC, B, v, kRowTlCellW, 1);
+      MPSW_ROWV(v, launch_k(k_row_tl_cell<VV>, c, s, m, t, B, bs, ut, ht, d.pc, d.ke, (int)ph.drag, rkh, early));
+    } else if (part == 1) {
+      const int v = row_width(K_TL_EDGE_DIAG, B);
+      const LaunchCfg c = row_cfg(K_TL_EDGE_DIAG, m.nE, B, v, kRowTlEdgeW, 2);
+      const float apt = ph.apvm * ph.dt;
+      if (visc) {
+        MPSW_ROWV(v, launch_k(k_row_tl_edge<VV, 1>, c, s, m, t, B, bs, ut, ht, (const float *)d.pc, d.pe, d.he, d.dsq_u, apt, early));
+      } else {
+        MPSW_ROWV(v, launch_k(k_row_tl_edge<VV, 0>, c, s, m, t, B, bs, ut, ht, (const float *)d.pc, d.pe, d.he, (float *)nullptr, apt, early));
+      }
+    } else {
+      const int v = row_width(K_TL_EDGE_TEND, B);
+      const LaunchCfg c = row_cfg(K_TL_EDGE_TEND, m.nE, B, v, kRowTlTendW, 2);
+      if (visc || ph.wind || ph.drag) {
+        MPSW_ROWV(v, launch_k(k_row_tl_tend<VV, 1>, c, s, m, B, bs, ut, ht, d, (const float *)d.he, ph, rku, early));
+      } else {
+        MPSW_ROWV(v, launch_k(k_row_tl_tend<VV, 0>, c, s, m, B, bs, ut, ht, d, (const float *)d.he, ph, rku, early));
+      }
+    }
+  } else {
+    throw std::invalid_argument("row passes run FP32 members only");
+  }
+}
+template <typename R, typename A>
+void Launch<R, A>::row_ad(int part, const MeshDev<R> &m, const RowTab &t, int B, const Base<R> &bs, const Phys<R> &ph,
+                          const AdIn<R> &in, const AdWork<R> &w, const AdOut<R, A> &out, cudaStream_t s) {
+  if constexpr (std::is_same<R, float>::value && std::is_same<A, double>::value) {
+    g_launches++;
+    const int early = (int)g_stable_base;
+    const float apt = ph.apvm * ph.dt;
+    if (part == 0) {
+      const int v = row_width(K_AD_EDGE, B);
+      const LaunchCfg c = row_cfg(K_AD_EDGE, m.nE, B, v, kRowAdEdgeW, 2);
+      MPSW_ROWV(v, launch_k(k_row_ad_edge<VV>, c, s, m, t, B, bs, apt, in, w, early));
+    } else if (part == 1) {
+      const int v = row_width(K_AD_CELL, B);
+      const LaunchCfg c = row_cfg(K_AD_CELL, m.nC, B, v, kRowAdCellW, 1);
+      MPSW_ROWV(v, launch_k(k_row_ad_cell<VV>, c, s, m, t, B, bs, apt, in, w, early));
+    } else {
+      const int v = row_width(K_AD_FINAL, B);
+      LaunchCfg c = row_cfg(K_AD_FINAL, m.nE, B, v, kRowAdFinalW, 2);
+      const int cell_blocks = row_cfg(K_AD_FINAL, m.nC, B, v, kRowAdFinalW, 2).grid;
+      c.grid += cell_blocks;
+      MPSW_ROWV(v, launch_k(k_row_ad_final<VV>, c, s, m, t, B, bs, apt, w, out, ph.bad, cell_blocks, early));
+    }
+  } else {
+    throw std::invalid_argument("row passes run FP32 members only");
   }
 }
 template <typename R, typename A>

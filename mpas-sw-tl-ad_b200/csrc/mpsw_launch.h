@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 
 #include "mpsw_internal.h"
+#include "mpsw_rows.h"
 #include "mpsw_stage.h"
 
 namespace mpsw {
@@ -83,6 +84,16 @@ struct Launch {
   // one kernel of ad_stage (0 edge, 1 cell, 2 vertex, 3 final), for timing
   static void ad_part(int which, const MeshDev<R> &m, int B, const Base<R> &bs, const Phys<R> &ph,
                       const AdIn<R> &in, const AdWork<R> &w, const AdOut<R, A> &out, cudaStream_t s);
+  // Row passes of FP32 members (mpsw_rows.cuh): a tangent-linear stage is parts 0 cells, 1 edges, 2
+  // tendencies (with del4 viscosity del4_vc between 1 and 2; d.he holds the thickness flux), an
+  // adjoint stage parts 0 edges, 1 cells, 2 final.  rows_ok: tables built and enough members (the
+  // adjoint passes serve the default physics).
+  static bool rows_ok(const RowTab &t, int nE, int B, const Phys<R> &ph, bool adjoint);
+  static void row_tl(int part, const MeshDev<R> &m, const RowTab &t, int B, const Base<R> &bs, const R *ut,
+                     const R *ht, const Diag<R> &d, const Phys<R> &ph, const RK<R, A> &rku, const RK<R, A> &rkh,
+                     cudaStream_t s);
+  static void row_ad(int part, const MeshDev<R> &m, const RowTab &t, int B, const Base<R> &bs, const Phys<R> &ph,
+                     const AdIn<R> &in, const AdWork<R> &w, const AdOut<R, A> &out, cudaStream_t s);
   // Fused member stages (FP32 members only; mpsw_fused.cuh): one kernel for a whole
   // tangent-linear or adjoint stage, M = 4 or 8 members per block.  The physics must be the
   // default (no viscosity, drag or wind) and the seeds empty; fused_ok() tells.
