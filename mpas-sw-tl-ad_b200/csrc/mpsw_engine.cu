@@ -544,8 +544,8 @@ void Engine::build_fused() {
 
 // Halo tiles of the nonlinear stage, while the tiles' blobs (2.7 times the mesh: halo entities are
 // packed with every tile that reads them) stay in the 126 MB L2 between stages: 2.3 KB a cell in
-// FP64, 1.2 KB in FP32.  Measured us a stage, tiles against grid-wide passes: level 3 5.1 / 16.6
-// (FP64) 3.9 / 12.6 (FP32), level 5 7.4 / 18.6 and 5.5 / 14.5, level 6 21.7 / 25.7 and 12.9 / 18.0;
+// FP64, 1.2 KB in FP32.  Measured us a stage, tiles against grid-wide passes: level 3 4.3 / 16.6
+// (FP64) 3.9 / 12.6 (FP32), level 5 6.8 / 18.6 and 4.9 / 14.5, level 6 19.1 / 25.7 and 12.1 / 18.0;
 // level 7, beyond the line, 93.7 / 66.8 and 63.2 / 49.9.  Tiles own as many cells as give each of
 // the 148 SMs one, on meshes for which that is fewer than the layers' caps allow.
 // MPSW_STAGE_TILES=0 keeps the passes.

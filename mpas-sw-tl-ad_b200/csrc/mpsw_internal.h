@@ -15,7 +15,6 @@
 // and the connectivity word is a broadcast.
 #pragma once
 
-#include <cmath>
 #include <cstddef>
 #include <cstdint>
 
@@ -175,25 +174,6 @@ struct AdOut {
 #else
 #define MPSW_HD
 #endif
-
-// a / b for a divisor whose reciprocal r = 1 / b (rounded to nearest) is at hand.  FP64: the
-// correctly rounded quotient, bit for bit what a / b gives, by Markstein's corrections (P.
-// Markstein, IBM J. Res. Dev. 34, 1990): a faithful q from one residual step, then q + (a - b q) r
-// rounds to nearest, for divisors within 1e-50 .. 1e50.  Quotients near the ends of the exponent
-// range, where a residual could be inexact, infinities and NaN take the division itself.  Five multiply-adds in place of a division
-// of some hundred cycles.  FP32 stencils multiply by the reciprocal.
-template <typename R>
-MPSW_HD inline R div_r(R a, R b, R r) {
-  if constexpr (sizeof(R) == 4) {
-    return a * r;
-  } else {
-    const R q0 = a * r;
-    const R m = q0 < R(0) ? -q0 : q0;
-    if (!(m > R(1e-200) && m < R(1e200))) return a == R(0) ? q0 : a / b;
-    const R q1 = fma(fma(-b, q0, a), r, q0);
-    return fma(fma(-b, q1, a), r, q1);
-  }
-}
 
 // Prefix sizes of a tile's local spaces; the meaning of each layer for the tangent-linear and
 // the adjoint stage is given in mpsw_tiles.h.

@@ -131,12 +131,12 @@ __global__ void __launch_bounds__(kStageThreads, 2) k_stage(StageDev ts, StageAr
       if (i < n[S_CK]) {
         CellKRec<R> r;
         stage_rec(sec(S::CK), kCapCK, i, &r);
-        stage_ke(r, m.v[6], m.v[7], w, a, i, a.out.on && i < n[S_CO] ? __ldg(idc + i) : -1);
+        stage_ke(r, m.v[6], w, a, i, a.out.on && i < n[S_CO] ? __ldg(idc + i) : -1);
       }
       if (visc) {
         CellXRec<R> r;
         stage_rec(sec(S::CX), kCapCM, i, &r);
-        stage_div(r, m.v[7], w, i);
+        stage_div(r, m.v[6], w, i);
       }
     }
   }
@@ -159,7 +159,7 @@ __global__ void __launch_bounds__(kStageThreads, 2) k_stage(StageDev ts, StageAr
     CellXRec<R> r;
     stage_rec(sec(S::CM), kCapCM, top, &m);
     stage_rec(sec(S::CX), kCapCM, top, &r);
-    stage_thick(r, sec(S::CO)[top], m.v[6], m.v[7], w, a, top, own, x0, acc);
+    stage_thick(r, sec(S::CO)[top], m.v[6], w, a, top, own, x0, acc);
   }
   __syncthreads();
   if (del4) {
@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(kStageThreads, 2) k_stage(StageDev ts, StageAr
       CellMRec<R> m;
       stage_rec(sec(S::CX), kCapCM, i, &r);
       stage_rec(sec(S::CM), kCapCM, i, &m);
-      stage_del4_cell(r, m.v[7], w, i, n[S_EM]);
+      stage_del4_cell(r, m.v[6], w, i, n[S_EM]);
     }
     __syncthreads();
   }

@@ -450,6 +450,7 @@ void stage_pack(const Builder &b, const BuiltMesh &m, const Space &E, const Spac
     reinterpret_cast<uint16_t *>(p + off[sec] + 16 * ((k >> 3) * cnt + i))[k & 7] = (uint16_t)(x * (int)sizeof(R));
   };
   constexpr int per = 16 / (int)sizeof(R);
+  auto divisor = [](double x) { return sizeof(R) == 4 ? R(1) / R(x) : R(x); };
   auto val = [&](int sec, int cnt, int lists, int i, int k, R x) {
     reinterpret_cast<R *>(p + off[sec] + 16 * ((lists + k / per) * cnt + i))[k % per] = x;
   };
@@ -463,9 +464,8 @@ void stage_pack(const Builder &b, const BuiltMesh &m, const Space &E, const Spac
       val(SB_V, nv, 1, i, k, R(m.v_esg[s]) * R(m.e_dc[m.v_es[s]]));
       val(SB_V, nv, 1, i, 3 + k, R(m.v_k[s]));
     }
-    val(SB_V, nv, 1, i, 6, R(m.v_area[v]));
-    val(SB_V, nv, 1, i, 7, R(1) / R(m.v_area[v]));
-    val(SB_V, nv, 1, i, 8, R(m.v_f[v]));
+    val(SB_V, nv, 1, i, 6, divisor(m.v_area[v]));
+    val(SB_V, nv, 1, i, 7, R(m.v_f[v]));
   }
   for (int i = 0; i < ncm; i++) {
     const int c = C.list[i];
@@ -483,8 +483,7 @@ void stage_pack(const Builder &b, const BuiltMesh &m, const Space &E, const Spac
         val(SB_CK, nck, 1, i, k, (R(0.25) * R(m.e_dc[e])) * R(m.e_dv[e]));
       }
     }
-    val(SB_CM, ncm, 1, i, 6, R(m.c_area[c]));
-    val(SB_CM, ncm, 1, i, 7, R(1) / R(m.c_area[c]));
+    val(SB_CM, ncm, 1, i, 6, divisor(m.c_area[c]));
     if (i < nck) val(SB_CK, nck, 1, i, 6, R(m.c_hs[c]));
   }
   for (int i = 0; i < nem; i++) {
@@ -498,10 +497,8 @@ void stage_pack(const Builder &b, const BuiltMesh &m, const Space &E, const Spac
       list(SB_E, nem, i, 4 + j, has ? E.local(b.eoe(e, j)) : i);
       val(SB_E, nem, 2, i, j, has ? R(m.e_w[(size_t)j * m.nE + e]) : R(0));
     }
-    val(SB_E, nem, 2, i, 10, R(m.e_dc[e]));
-    val(SB_E, nem, 2, i, 11, R(m.e_dv[e]));
-    val(SB_E, nem, 2, i, 12, R(1) / R(m.e_dc[e]));
-    val(SB_E, nem, 2, i, 13, R(1) / R(m.e_dv[e]));
+    val(SB_E, nem, 2, i, 10, divisor(m.e_dc[e]));
+    val(SB_E, nem, 2, i, 11, divisor(m.e_dv[e]));
   }
   std::memcpy(p + off[SB_GE], E.list.data(), 4 * E.list.size());
   std::memcpy(p + off[SB_GC], C.list.data(), 4 * C.list.size());
@@ -516,9 +513,6 @@ std::string build_stage_tiles(const BuiltMesh &m, int kmax, StageSetHost *o) {
     if (m.c_n[c] > kCellSlots) return "stage tiles need at most 6 edges per cell";
   for (int e = 0; e < m.nE; e++)
     if (m.e_n[e] > kEoeSlots) return "stage tiles need at most 10 edgesOnEdge";
-  for (const std::vector<double> *x : {&m.e_dc, &m.e_dv, &m.c_area, &m.v_area})
-    for (double d : *x)
-      if (!(d > 1e-50 && d < 1e50)) return "a mesh metric outside the range div_r serves";
   Builder b(m);
   *o = StageSetHost();
   int stamp = 0;

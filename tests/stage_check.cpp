@@ -81,10 +81,10 @@ extern "C" int stage_check(const int *ints, const double *cfg, const int *const 
       stage_rec(sec(SB_CM), n[S_CM], x, &q);
       if (x < n[S_CK]) {
         stage_rec(sec(SB_CK), n[S_CK], x, &k);
-        stage_ke(k, q.v[6], q.v[7], w, a, x, x < n[S_CO] ? gc[x] : -1);
+        stage_ke(k, q.v[6], w, a, x, x < n[S_CO] ? gc[x] : -1);
       }
       stage_rec(sec(SB_CX), n[S_CM], x, &y);
-      if (visc) stage_div(y, q.v[7], w, x);
+      if (visc) stage_div(y, q.v[6], w, x);
     }
     std::vector<EdgeRec<double>> er(n[S_EM]);
     std::vector<double> perp(n[S_EM]);
@@ -103,7 +103,7 @@ extern "C" int stage_check(const int *ints, const double *cfg, const int *const 
       CellXRec<double> y;
       stage_rec(sec(SB_CM), n[S_CM], x, &q);
       stage_rec(sec(SB_CX), n[S_CM], x, &y);
-      stage_thick(y, sec(SB_CO)[x], q.v[6], q.v[7], w, a, x, gc[x], 0.0, 0.0);
+      stage_thick(y, sec(SB_CO)[x], q.v[6], w, a, x, gc[x], 0.0, 0.0);
     }
     if (del4) {
       for (int x = 0; x < n[S_VA]; x++) {
@@ -116,7 +116,7 @@ extern "C" int stage_check(const int *ints, const double *cfg, const int *const 
         CellXRec<double> y;
         stage_rec(sec(SB_CM), n[S_CM], x, &q);
         stage_rec(sec(SB_CX), n[S_CM], x, &y);
-        stage_del4_cell(y, q.v[7], w, x, n[S_EM]);
+        stage_del4_cell(y, q.v[6], w, x, n[S_EM]);
       }
     }
     for (int x = 0; x < n[S_EO]; x++) stage_tend(er[x], w, a, x, ge[x], 0.0, 0.0);
