@@ -810,8 +810,18 @@ void Engine::fwd_diag(const double *u, const double *h, const Diag<double> &d, c
 // Beside the members of an overlapped sweep the tiles are taken only while they are at most two a
 // SM: their blocks hold half an SM's registers each, and on larger meshes cost the member kernels
 // more than the passes do (level 6, 8 FP64 members: sweep pair 6.5 ms with tiles, 6.0 without;
-// level 5, 64 FP32 members: 6.7 against 6.85 ms).
+// level 5, 64 FP32 members: 6.7 against 6.85 ms).  Members on tiles themselves leave them room (level 6, one
+// FP64 member, 16 steps: sweep pair 7.9 ms beside forward passes, 6.0 beside tiles).
 bool Engine::stage_tiled() const { return st64.ntiles > 0 && (!beside_members || st64.ntiles <= 2 * 148); }
+
+// FP64 members that take the tiles' tangent-linear stage.  One member gives the four passes too few
+// threads to hide their gathers; a block a member a tile does not (us a stage, passes -> tiles: level 3
+// 17.9 -> 6.4, level 5 24.5 -> 10.0, level 6 44.2 -> 31.3).  A second member has blocks of its own: 14.0
+// -> 6.6 and 22.7 -> 18.3 while both members' blocks are on the chip together, 40.7 -> 63.1 at level 6.
+// From three on the passes read whole rows of members and win (level 5, three: 27.4 against 30.8).
+bool Engine::stage_tl_tiled(int B) const {
+  return st64.ntiles > 0 && (B == 1 || (B == 2 && st64.ntiles <= 2 * 148));
+}
 
 static StageBaseOut base_out(const Diag<double> &d) {  // (u is the stage's input itself)
   StageBaseOut o{};
@@ -1128,6 +1138,11 @@ void Engine::rk4_tlm(int nsteps) {  // src/mpas_sw_module.f90:637-781
       const double *hti = k == 0 ? ht0 : tp_h[k - 1];
       RK<double, double> rut{ut0, k == 0 ? ut0 : tacc_u, k == 3 ? ut0 : tacc_u, k < 3 ? tp_u[k] : nullptr, c[k], w[k], 0.0, ph.tc1};
       RK<double, double> rht{ht0, k == 0 ? ht0 : tacc_h, k == 3 ? ht0 : tacc_h, k < 3 ? tp_h[k] : nullptr, c[k], w[k], 0.0, 0};
+      if (stage_tl_tiled(1)) {
+        L64::stage_tl(st64, StageTlArgs{uti, hti, 1, bs, ph, rut, rht, k == 3 ? dv("tend_u_tl") : nullptr,
+                                        k == 3 ? dv("tend_h_tl") : nullptr, m64.e_sc2, m64.e_sc4, m64.e_usrc}, stream);
+        continue;
+      }
       L64::tl_vertex(m64, 1, bs, uti, hti, tl_diag, stream);
       L64::tl_cell(m64, 1, bs, uti, hti, tl_diag, rht, k == 3 ? dv("tend_h_tl") : nullptr, stream);
       L64::tl_edge_diag(m64, 1, bs, uti, hti, tl_diag, ph, stream);

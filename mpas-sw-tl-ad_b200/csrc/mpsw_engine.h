@@ -217,6 +217,7 @@ struct Engine {
                  const RK<double, double> &rku, const RK<double, double> &rkh, double *tu, double *th,
                  const StageBaseOut &out);
   bool stage_tiled() const;
+  bool stage_tl_tiled(int B) const;  // FP64 members take the tiles' tangent-linear stage
   void tl_diag_run(const Base<double> &bs, const double *ut, const double *ht, const Diag<double> &d,
                    const Phys<double> &ph);
   void check_launch(const char *what);

@@ -26,6 +26,7 @@ constexpr size_t kFusedSmemMax = 227 * 1024;   // shared memory a block may use
 struct LaunchCfg {
   int grid, block;
   size_t smem = 0;  // dynamic shared memory bytes
+  int grid_y = 1;
 };
 // MPSW_BLOCK=64|128|256 overrides the starting block size.
 inline int block_threads() {
@@ -58,7 +59,7 @@ inline bool pdl_enabled() {
 template <typename... KArgs, typename... Args>
 inline void launch_k(void (*kernel)(KArgs...), LaunchCfg c, cudaStream_t s, Args &&...args) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)c.grid);
+  cfg.gridDim = dim3((unsigned)c.grid, (unsigned)c.grid_y);
   cfg.blockDim = dim3((unsigned)c.block);
   cfg.dynamicSmemBytes = c.smem;
   cfg.stream = s;
@@ -196,7 +197,22 @@ void Launch<R, A>::stage(const StageDev &ts, const StageArgs<R, A> &a, cudaStrea
   launch_k(k_stage<R, A>, LaunchCfg{ts.ntiles, kStageThreads, smem}, s, ts, a);
 }
 template <typename R, typename A>
+void Launch<R, A>::stage_tl(const StageDev &ts, const StageTlArgs &a, cudaStream_t s) {
+  if constexpr (std::is_same<R, double>::value) {
+    g_launches++;
+    launch_k(k_stage_tl<R>, LaunchCfg{ts.ntiles, kStageThreads, stage_tl_smem(a.ph.visc2 > 0.0 || a.ph.visc4 > 0.0, a.ph.visc4 > 0.0), a.B}, s, ts, a,
+             (int)g_stable_base);
+  } else {
+    throw std::invalid_argument("the tiles' tangent-linear stage runs FP64 members");
+  }
+}
+template <typename R, typename A>
 cudaError_t Launch<R, A>::stage_prepare() {
+  if constexpr (std::is_same<R, double>::value) {
+    const cudaError_t e = cudaFuncSetAttribute((const void *)k_stage_tl<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)stage_tl_smem(true, true));
+    if (e != cudaSuccess) return e;
+  }
   return cudaFuncSetAttribute((const void *)k_stage<R, A>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)stage_smem<R>(true, true));
 }

@@ -32,8 +32,54 @@ template <typename R>
 inline size_t stage_smem(bool visc, bool del4) {
   return (size_t)stage_work((int)sizeof(R), visc, del4) + StageShared<R>::END;
 }
+inline size_t stage_tl_smem(bool visc, bool del4) { return 8 * kTlBase + stage_smem<double>(visc, del4); }
 
 __device__ __forceinline__ unsigned smem_addr(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
+
+// Start the copies of a tile's records (blob g) into shared memory, one bulk copy per chunk row.
+template <typename R>
+__device__ __forceinline__ void stage_fetch(unsigned char *rec, const unsigned char *g, const int *n, const int *off,
+                                            bool visc, unsigned long long *arrived) {
+  using S = StageShared<R>;
+  const int tid = threadIdx.x;
+  if (tid < 32) {  // one bulk copy per chunk row of the records
+    const int ncx = visc ? n[S_CM] : n[S_CO];
+    if (tid == 0) {
+      asm volatile("mbarrier.init.shared.b64 [%0], 1;" ::"r"(smem_addr(arrived)) : "memory");
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+      const int bytes = 16 * (S::RV * n[S_VA] + (S::RCM - S::RV) * n[S_CM] + (S::RCX - S::RCM) * ncx +
+                              (S::RCK - S::RCX) * n[S_CK] + n[S_CO]);
+      asm volatile("mbarrier.arrive.expect_tx.shared.b64 _, [%0], %1;" ::"r"(smem_addr(arrived)), "r"(bytes)
+                   : "memory");
+    }
+    __syncwarp();
+    if (tid < S::RCO) {
+      const int k = tid < S::RV ? 0 : tid < S::RCM ? 1 : tid < S::RCX ? 2 : tid < S::RCK ? 3 : 4;
+      const int first = k == 0 ? 0 : k == 1 ? S::RV : k == 2 ? S::RCM : k == 3 ? S::RCX : S::RCK;
+      const int cnt = k == 0 ? n[S_VA] : k == 1 || k == 2 ? n[S_CM] : k == 3 ? n[S_CK] : n[S_CO];
+      const int cap = k == 0 ? kCapVA : k == 1 || k == 2 ? kCapCM : k == 3 ? kCapCK : kCapCO;
+      const int dst = k == 0 ? S::V : k == 1 ? S::CM : k == 2 ? S::CX : k == 3 ? S::CK : S::CO;
+      const int src = k == 0 ? off[SB_V] : k == 1 ? off[SB_CM] : k == 2 ? off[SB_CX] : k == 3 ? off[SB_CK] : off[SB_CO];
+      asm volatile(
+          "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+              smem_addr(rec + dst + 16 * cap * (tid - first))),
+          "l"(g + src + 16 * cnt * (tid - first)), "r"(16 * (k == 2 ? ncx : cnt)), "r"(smem_addr(arrived))
+          : "memory");
+    }
+  }
+}
+
+// Wait for them (they were issued a stage ago; a bound all the same).  The same answer for every
+// thread; false: they did not arrive.
+__device__ __forceinline__ bool stage_arrived(unsigned long long *arrived) {
+  unsigned ok = 0;
+  for (int i = 0; i < (1 << 20) && !ok; i++)
+    asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared.b64 p, [%1], 0;\nselp.u32 %0, 1, 0, p;\n}"
+                 : "=r"(ok)
+                 : "r"(smem_addr(arrived))
+                 : "memory");
+  return !__syncthreads_or(!ok);
+}
 
 template <typename R, typename A>
 __global__ void __launch_bounds__(kStageThreads, 2) k_stage(StageDev ts, StageArgs<R, A> a) {
@@ -49,31 +95,7 @@ __global__ void __launch_bounds__(kStageThreads, 2) k_stage(StageDev ts, StageAr
   for (int k = 0; k < kStageCounts; k++) n[k] = __ldg(ts.cnt + (size_t)blockIdx.x * kStageCounts + k);
   stage_layout(n, (int)sizeof(R), off);
   const unsigned char *g = ts.blob + __ldg(ts.blob_off + blockIdx.x);
-  if (tid < 32) {  // one bulk copy per chunk row of the records
-    const int ncx = visc ? n[S_CM] : n[S_CO];
-    if (tid == 0) {
-      asm volatile("mbarrier.init.shared.b64 [%0], 1;" ::"r"(smem_addr(&arrived)) : "memory");
-      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-      const int bytes = 16 * (S::RV * n[S_VA] + (S::RCM - S::RV) * n[S_CM] + (S::RCX - S::RCM) * ncx +
-                              (S::RCK - S::RCX) * n[S_CK] + n[S_CO]);
-      asm volatile("mbarrier.arrive.expect_tx.shared.b64 _, [%0], %1;" ::"r"(smem_addr(&arrived)), "r"(bytes)
-                   : "memory");
-    }
-    __syncwarp();
-    if (tid < S::RCO) {
-      const int k = tid < S::RV ? 0 : tid < S::RCM ? 1 : tid < S::RCX ? 2 : tid < S::RCK ? 3 : 4;
-      const int first = k == 0 ? 0 : k == 1 ? S::RV : k == 2 ? S::RCM : k == 3 ? S::RCX : S::RCK;
-      const int cnt = k == 0 ? n[S_VA] : k == 1 || k == 2 ? n[S_CM] : k == 3 ? n[S_CK] : n[S_CO];
-      const int cap = k == 0 ? kCapVA : k == 1 || k == 2 ? kCapCM : k == 3 ? kCapCK : kCapCO;
-      const int dst = k == 0 ? S::V : k == 1 ? S::CM : k == 2 ? S::CX : k == 3 ? S::CK : S::CO;
-      const int src = k == 0 ? off[SB_V] : k == 1 ? off[SB_CM] : k == 2 ? off[SB_CX] : k == 3 ? off[SB_CK] : off[SB_CO];
-      asm volatile(
-          "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-              smem_addr(rec + dst + 16 * cap * (tid - first))),
-          "l"(g + src + 16 * cnt * (tid - first)), "r"(16 * (k == 2 ? ncx : cnt)), "r"(smem_addr(&arrived))
-          : "memory");
-    }
-  }
+  stage_fetch<R>(rec, g, n, off, visc, &arrived);
   auto sec = [&](int o) { return reinterpret_cast<const StageChunk *>(rec + o); };
   EdgeRec<R> er;
   if (tid < n[S_EM]) stage_rec(reinterpret_cast<const StageChunk *>(g + off[SB_E]), n[S_EM], tid, &er);
@@ -105,17 +127,9 @@ __global__ void __launch_bounds__(kStageThreads, 2) k_stage(StageDev ts, StageAr
     if (tid < n[S_CA]) stage_val<R>(w, W_H + tid, 0) = h;
   }
   __syncthreads();  // (also: the barrier's initialisation is visible)
-  {
-    unsigned ok = 0;  // the copies were issued a stage ago; a bound all the same
-    for (int i = 0; i < (1 << 20) && !ok; i++)
-      asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared.b64 p, [%1], 0;\nselp.u32 %0, 1, 0, p;\n}"
-                   : "=r"(ok)
-                   : "r"(smem_addr(&arrived))
-                   : "memory");
-    if (__syncthreads_or(!ok)) {
-      if (a.ph.bad) *a.ph.bad = 1;
-      return;
-    }
+  if (!stage_arrived(&arrived)) {
+    if (a.ph.bad) *a.ph.bad = 1;
+    return;
   }
   // phase 1: vertices; from the next warp on, ke cells (with viscosity also the other divergences)
   const int nv32 = stage_up32(n[S_VA]);
@@ -179,6 +193,192 @@ __global__ void __launch_bounds__(kStageThreads, 2) k_stage(StageDev ts, StageAr
   }
   // phase 4
   if (edge) stage_tend(er, w, a, tid, own, x0, acc);
+}
+
+// RK bookkeeping of one value of a member sweep (rk_members with one member)
+struct StageTlRk {
+  double x0 = 0.0, t[3] = {0.0, 0.0, 0.0}, acc = 0.0;
+  __device__ __forceinline__ void fetch(const RK<double, double> &rk, size_t o) {
+    const bool last = rk.t_in[0] != nullptr;
+    if ((rk.next && !last) || last) x0 = __ldcg(rk.x0 + o);
+    if (last) {
+#pragma unroll
+      for (int j = 0; j < 3; j++) t[j] = __ldcg(rk.t_in[j] + o);
+    } else if (!rk.t_out && rk.acc_out) {
+      acc = __ldcg(rk.acc_in + o);
+    }
+  }
+  __device__ __forceinline__ void put(const RK<double, double> &rk, size_t o, double x) const {
+    const bool last = rk.t_in[0] != nullptr;
+    if (rk.next && !last) rk.next[o] = rk.frozen ? x0 : x0 + rk.c * x;
+    if (rk.frozen) return;
+    if (rk.t_out) {
+      rk.t_out[o] = x;
+    } else if (last) {
+      double a = x0;
+#pragma unroll
+      for (int j = 0; j < 3; j++) a = a + rk.wt[j] * t[j];
+      a = a + rk.w * x;
+      rk.acc_out[o] = a;
+      if (rk.next) rk.next[o] = a;
+    } else if (rk.acc_out) {
+      rk.acc_out[o] = acc + rk.w * x;
+    }
+  }
+};
+
+// A tangent-linear stage of FP64 members, one a block (blockIdx.y), phase by phase as k_stage and, like
+// it, bound by the chain of phases rather than by bytes or arithmetic.  early: the linearisation point is
+// stored, so its values, like the mesh, are fetched before the wait for the stage before; two blocks
+// stay on an SM (110 KB each with viscosity), so that the next stage's fetch overlaps this one.  At one
+// block an SM: 13.4 instead of 10.0 us a level-5 stage; the four passes took 24.5 (stages of a window
+// sweep of one member).
+template <typename R>  // double
+__global__ void __launch_bounds__(kStageThreads, 2) k_stage_tl(StageDev ts, StageTlArgs a, int early) {
+  static_assert(sizeof(R) == 8);
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ __align__(8) unsigned long long arrived;
+  using S = StageShared<double>;
+  constexpr int NT = kStageThreads;
+  const int tid = threadIdx.x, B = a.B, mb = blockIdx.y;
+  const bool del4 = a.ph.visc4 > 0.0, visc = del4 || a.ph.visc2 > 0.0;
+  unsigned char *const w = smem_raw + 8 * kTlBase, *const rec = w + stage_work(8, visc, del4);
+  int n[kStageCounts], off[kStageSections];
+#pragma unroll
+  for (int k = 0; k < kStageCounts; k++) n[k] = __ldg(ts.cnt + (size_t)blockIdx.x * kStageCounts + k);
+  stage_layout(n, 8, off);
+  const unsigned char *g = ts.blob + __ldg(ts.blob_off + blockIdx.x);
+  stage_fetch<double>(rec, g, n, off, visc, &arrived);
+  auto sec = [&](int o) { return reinterpret_cast<const StageChunk *>(rec + o); };
+  EdgeRec<double> er;
+  if (tid < n[S_EM]) stage_rec(reinterpret_cast<const StageChunk *>(g + off[SB_E]), n[S_EM], tid, &er);
+  const int *ids = reinterpret_cast<const int *>(g + off[SB_GE]), *idc = reinterpret_cast<const int *>(g + off[SB_GC]);
+  int ge[2] = {0, 0}, gc = 0, gv = 0;
+  if (tid < n[S_EA]) ge[0] = __ldg(ids + tid);
+  if (tid + NT < n[S_EA]) ge[1] = __ldg(ids + tid + NT);
+  if (tid < n[S_CA]) gc = __ldg(idc + tid);
+  if (tid < n[S_VA]) gv = __ldg(reinterpret_cast<const int *>(g + off[SB_GV]) + tid);
+  const int top = NT - 1 - tid;
+  const bool edge = tid < n[S_EO], cell = top < n[S_CO];
+  const int own = edge ? ge[0] : cell ? __ldg(idc + top) : 0;
+  double hv = 0.0, vo = 0.0, vb = 0.0, gpt = 0.0, gpn = 0.0;
+  auto base = [&]() {
+    double u0 = 0.0, u1 = 0.0, h0 = 0.0, h1 = 0.0, p0 = 0.0;
+    if (tid < n[S_EA]) {
+      u0 = __ldcg(a.bs.u + ge[0]);
+      h0 = __ldcg(a.bs.he + ge[0]);
+    }
+    if (tid + NT < n[S_EA]) {
+      u1 = __ldcg(a.bs.u + ge[1]);
+      h1 = __ldcg(a.bs.he + ge[1]);
+    }
+    if (tid < n[S_EM]) {
+      p0 = __ldcg(a.bs.pe + ge[0]);
+      vb = __ldcg(a.bs.v + ge[0]);
+      gpt = __ldcg(a.bs.gpt + ge[0]);
+      gpn = __ldcg(a.bs.gpn + ge[0]);
+    }
+    if (tid < n[S_VA]) {
+      hv = __ldcg(a.bs.hv + gv);
+      vo = __ldcg(a.bs.vort + gv);
+    }
+    if (tid < n[S_EA]) {
+      stage_val<double>(w, T_UB + tid, 0) = u0;
+      stage_val<double>(w, T_HB + tid, 0) = h0;
+    }
+    if (tid + NT < n[S_EA]) {
+      stage_val<double>(w, T_UB + tid + NT, 0) = u1;
+      stage_val<double>(w, T_HB + tid + NT, 0) = h1;
+    }
+    if (tid < n[S_EM]) stage_val<double>(w, T_PB + tid, 0) = p0;
+  };
+  if (early) base();
+  pdl_begin();
+  if (!early) base();
+  StageTlRk rk;
+  {
+    double u0 = 0.0, u1 = 0.0, h = 0.0;  // in flight together
+    if (tid < n[S_EA]) u0 = __ldcg(a.u + (size_t)ge[0] * B + mb);
+    if (tid + NT < n[S_EA]) u1 = __ldcg(a.u + (size_t)ge[1] * B + mb);
+    if (tid < n[S_CA]) h = __ldcg(a.h + (size_t)gc * B + mb);
+    if (edge || cell) rk.fetch(edge ? a.rku : a.rkh, (size_t)own * B + mb);
+    if (tid < n[S_EA]) stage_val<double>(w, W_U + tid, 0) = u0;
+    if (tid + NT < n[S_EA]) stage_val<double>(w, W_U + tid + NT, 0) = u1;
+    if (tid < n[S_CA]) stage_val<double>(w, W_H + tid, 0) = h;
+  }
+  __syncthreads();
+  if (!stage_arrived(&arrived)) {
+    if (a.ph.bad) *a.ph.bad = 1;
+    return;
+  }
+  // phase 1: vertices; from the next warp on, ke cells (with viscosity also the divergences)
+  const int nv32 = stage_up32(n[S_VA]);
+  if (tid < n[S_VA]) {
+    VertexRec<double> r;
+    stage_rec(sec(S::V), kCapVA, tid, &r);
+    stage_tl_vertex(r, w, tid, hv, vo, visc);
+  } else if (tid >= nv32) {
+    for (int i = tid - nv32; i < (visc ? n[S_CM] : n[S_CK]); i += NT - nv32) {
+      CellMRec<double> m;
+      stage_rec(sec(S::CM), kCapCM, i, &m);
+      if (i < n[S_CK]) {
+        CellKRec<double> r;
+        stage_rec(sec(S::CK), kCapCK, i, &r);
+        stage_tl_ke(r, m.v[6], w, i);
+      }
+      if (visc) {
+        CellXRec<double> r;
+        stage_rec(sec(S::CX), kCapCM, i, &r);
+        stage_div(r, m.v[6], w, i);
+      }
+    }
+  }
+  __syncthreads();
+  // phase 2: tangential velocity of the pv_edge layer; pv_cell on the last threads
+  double v = 0.0;
+  if (tid < n[S_EM]) {
+    v = stage_perp(er, w);
+  } else if (top < n[S_CM]) {
+    CellMRec<double> r;
+    stage_rec(sec(S::CM), kCapCM, top, &r);
+    stage_pvcell(r, w, top);
+  }
+  __syncthreads();
+  // phase 3: pv_edge; thickness of the owned cells on the last threads
+  if (tid < n[S_EM]) {
+    stage_tl_edge(er, w, a.ph, tid, v, vb, gpt, gpn, del4);
+  } else if (cell) {
+    CellMRec<double> m;
+    CellXRec<double> r;
+    stage_rec(sec(S::CM), kCapCM, top, &m);
+    stage_rec(sec(S::CX), kCapCM, top, &r);
+    const double t = stage_tl_thick(r, sec(S::CO)[top], m.v[6], w, top);
+    if (a.tend_h) a.tend_h[(size_t)own * B + mb] = t;
+    rk.put(a.rkh, (size_t)own * B + mb, t);
+  }
+  __syncthreads();
+  if (del4) {
+    if (tid < n[S_VA]) {
+      VertexRec<double> r;
+      stage_rec(sec(S::V), kCapVA, tid, &r);
+      stage_del4_vertex(r, w, tid, n[S_EM]);
+    } else if (tid - nv32 >= 0 && tid - nv32 < n[S_CK]) {
+      const int i = tid - nv32;
+      CellXRec<double> r;
+      CellMRec<double> m;
+      stage_rec(sec(S::CX), kCapCM, i, &r);
+      stage_rec(sec(S::CM), kCapCM, i, &m);
+      stage_del4_cell(r, m.v[6], w, i, n[S_EM]);
+    }
+    __syncthreads();
+  }
+  // phase 4
+  if (edge) {
+    const double t = stage_tl_tend(er, w, a, idc, tid, own);
+    flag_nonfinite(a.ph.bad, t);
+    if (a.tend_u) a.tend_u[(size_t)own * B + mb] = t;
+    rk.put(a.rku, (size_t)own * B + mb, t);
+  }
 }
 
 }  // namespace mpsw

@@ -59,6 +59,11 @@ enum StageWork {
 };
 MPSW_HD inline int stage_work(int r, bool visc, bool del4) { return r * (del4 ? W_END : visc ? W_DSQ : W_VORT); }
 
+// A tangent-linear stage exchanges the same values of the member, after the linearisation point's
+// u, h_edge (all edges) and pv_edge (pv_edge layer): negative offsets from the work area.
+enum StageTlWork { T_UB = -(2 * kCapEA + kCapEM), T_HB = T_UB + kCapEA, T_PB = T_HB + kCapEA, kTlBase = -T_UB };
+static_assert(kTlBase % 2 == 0, "the records behind start on 16 bytes");
+
 // A blob: per entity a record of 16-byte chunks, stored chunk by chunk ([chunk][n]), first chunk(s)
 // the neighbour list as byte offsets into the work arrays, then values in the stencils' precision.
 //   vertices:       edges[3] cells[3]; sign dcEdge [3], kites [3], area, f
@@ -86,7 +91,7 @@ MPSW_HD inline int stage_layout(const int *n, int r, int *off) {
   off[SB_E] = o; o += 16 * n[S_EM] * (2 + stage_chunks(kValsE, r));
   off[SB_GE] = o; o += (4 * n[S_EA] + 15) / 16 * 16;
   off[SB_GC] = o; o += (4 * n[S_CA] + 15) / 16 * 16;
-  off[SB_GV] = o; o += (4 * n[S_VO] + 15) / 16 * 16;
+  off[SB_GV] = o; o += (4 * n[S_VA] + 15) / 16 * 16;
   return o;
 }
 
@@ -354,6 +359,114 @@ MPSW_HD inline void stage_tend(const EdgeRec<R> &r, unsigned char *w, const Stag
   if (a.ph.bad && !(tu - tu == R(0))) *a.ph.bad = 1;  // NaN or infinite
   if (a.tend_u) a.tend_u[g] = tu;
   stage_rk(a.rku, g, tu, x0, acc);
+}
+
+// ---- tangent-linear stage of one FP64 member (src/mpas_sw_dyncore_tlm.f90), in the operation order
+// of the member kernels: the same phases on the same tiles -----------------------------------------
+struct StageTlArgs {
+  const double *u, *h;  // the member's stage input, rows of B members
+  int B;
+  Base<double> bs;
+  Phys<double> ph;
+  RK<double, double> rku, rkh;
+  double *tend_u, *tend_h;
+  const double *sc2, *sc4, *usrc;
+};
+
+// :255-271, :344-360; hv, vort: the linearisation point's
+MPSW_HD inline void stage_tl_vertex(const VertexRec<double> &r, unsigned char *w, int i, double hv, double vort_b,
+                                    bool visc) {
+  double circ = 0.0, hvt = 0.0;
+#pragma unroll
+  for (int k = 0; k < VDEG; k++) circ = circ + r.v[k] * stage_val<double>(w, W_U, r.at(k));
+  const double vort = circ / r.v[6];
+#pragma unroll
+  for (int k = 0; k < VDEG; k++) hvt = hvt + stage_val<double>(w, W_H, r.at(3 + k)) * r.v[3 + k];
+  hvt = hvt / r.v[6];
+  stage_val<double>(w, W_PVV + i, 0) = vort / hv - (hvt * (r.v[7] + vort_b)) / (hv * hv);
+  if (visc) stage_val<double>(w, W_VORT + i, 0) = vort;
+}
+// ke' (:274-316)
+MPSW_HD inline void stage_tl_ke(const CellKRec<double> &r, double area, unsigned char *w, int i) {
+  double ke = 0.0;
+#pragma unroll
+  for (int k = 0; k < 6; k++)
+    ke = ke + r.v[k] * ((2.0 * stage_val<double>(w, T_UB, r.at(k))) * stage_val<double>(w, W_U, r.at(k)));
+  stage_val<double>(w, W_KE + i, 0) = ke / area;
+}
+// tend_h' of an owned cell (:541-561)
+MPSW_HD inline double stage_tl_thick(const CellXRec<double> &r, const StageChunk &across, double area, unsigned char *w,
+                                     int i) {
+  const double hc = stage_val<double>(w, W_H + i, 0);
+  double th = 0.0;
+#pragma unroll
+  for (int k = 0; k < 6; k++) {
+    const double het = 0.5 * (hc + stage_val<double>(w, W_H, stage_at(&across, k)));
+    th = th - ((stage_val<double>(w, W_U, r.at(k)) * r.v[k]) * stage_val<double>(w, T_HB, r.at(k)) +
+               (stage_val<double>(w, T_UB, r.at(k)) * r.v[k]) * het);
+  }
+  return th / area;
+}
+// pv_edge', h_edge' and delsq_u' (:364-393, 425-445, 117-126, 638-652); vt: the tangential velocity;
+// vb, gpt, gpn: the linearisation point's at the edge
+MPSW_HD inline void stage_tl_edge(const EdgeRec<double> &r, unsigned char *w, const Phys<double> &ph, int i, double vt,
+                                  double vb, double gpt, double gpn, bool del4) {
+  const int c1 = r.at(0), c2 = r.at(1), v1 = r.at(2), v2 = r.at(3);
+  const double dc = r.v[10], dv = r.v[11], u = stage_val<double>(w, W_U + i, 0), ub = stage_val<double>(w, T_UB + i, 0);
+  const double pv1 = stage_val<double>(w, W_PVV, v1), pv2 = stage_val<double>(w, W_PVV, v2);
+  const double gptt = (pv2 - pv1) / dv;
+  double pet = 0.0;
+  pet = pet + 0.5 * pv1;
+  pet = pet + 0.5 * pv2;
+  pet = pet - ((ph.apvm * vt) * ph.dt) * gpt - ((ph.apvm * vb) * ph.dt) * gptt;
+  const double gpnt = (stage_val<double>(w, W_PC, c2) - stage_val<double>(w, W_PC, c1)) / dc;
+  pet = pet - ((ph.apvm * u) * ph.dt) * gpn - ((ph.apvm * ub) * ph.dt) * gpnt;
+  stage_val<double>(w, W_PE + i, 0) = pet;
+  stage_val<double>(w, W_HE + i, 0) = 0.5 * (stage_val<double>(w, W_H, c1) + stage_val<double>(w, W_H, c2));
+  if (del4)
+    stage_val<double>(w, W_DSQ + i, 0) = (stage_val<double>(w, W_DIV, c2) - stage_val<double>(w, W_DIV, c1)) / dc -
+                                         (stage_val<double>(w, W_VORT, v2) - stage_val<double>(w, W_VORT, v1)) / dv;
+}
+// tend_u' of an owned edge (:564-768); gc: internal indices of the tile's cells
+MPSW_HD inline double stage_tl_tend(const EdgeRec<double> &r, unsigned char *w, const StageTlArgs &a, const int *gc,
+                                    int i, int g) {
+  const double pet = stage_val<double>(w, W_PE + i, 0), pe = stage_val<double>(w, T_PB + i, 0);
+  double qt = 0.0;
+#pragma unroll
+  for (int j = 0; j < 10; j++) {
+    const int e = r.at(4 + j);
+    const double wt = r.v[j];
+    const double wpvt = 0.5 * (pet + stage_val<double>(w, W_PE, e)), wpv = 0.5 * (pe + stage_val<double>(w, T_PB, e));
+    const double ub = stage_val<double>(w, T_UB, e), heb = stage_val<double>(w, T_HB, e);
+    qt = qt + ((wt * stage_val<double>(w, W_U, e)) * wpv) * heb + ((wt * ub) * wpvt) * heb +
+         ((wt * ub) * wpv) * stage_val<double>(w, W_HE, e);
+  }
+  const int c1 = r.at(0), c2 = r.at(1), v1 = r.at(2), v2 = r.at(3);
+  const double dc = r.v[10], dv = r.v[11], h1 = stage_val<double>(w, W_H, c1), h2 = stage_val<double>(w, W_H, c2);
+  const double ke1 = stage_val<double>(w, W_KE, c1), ke2 = stage_val<double>(w, W_KE, c2);
+  const double grad = (ke2 - ke1) + GRAVITY * (h2 - h1);
+  double tut = qt - grad / dc;
+  if (a.ph.visc2 > 0.0) {
+    double ud = (stage_val<double>(w, W_DIV, c2) - stage_val<double>(w, W_DIV, c1)) / dc -
+                (stage_val<double>(w, W_VORT, v2) - stage_val<double>(w, W_VORT, v1)) / dv;
+    ud = (a.sc2[g] * a.ph.visc2) * ud;
+    tut = tut + ud;
+  }
+  if (a.ph.visc4 > 0.0) {
+    double ud = (stage_val<double>(w, W_C4, c2) - stage_val<double>(w, W_C4, c1)) / dc -
+                (stage_val<double>(w, W_V4, v2) - stage_val<double>(w, W_V4, v1)) / dv;
+    ud = (a.sc4[g] * a.ph.visc4) * ud;
+    tut = tut - ud;
+  }
+  const double hh = stage_val<double>(w, T_HB + i, 0), het = 0.5 * (h1 + h2);
+  if (a.ph.wind) tut = tut - ((het * a.usrc[g]) / RHO_REF) / (hh * hh);
+  if (a.ph.drag) {
+    const double ket = 0.5 * (ke1 + ke2), ke = 0.5 * (a.bs.ke[gc[c1 / 8]] + a.bs.ke[gc[c2 / 8]]);
+    const double uu = stage_val<double>(w, T_UB + i, 0), sq = sqrt(2.0 * ke);
+    tut = tut - ((1.0e-3 * stage_val<double>(w, W_U + i, 0)) * sq) / hh -
+          ((((0.5 * 1.0e-3) * uu) * (2.0 * ket)) / sq) / hh + (((1.0e-3 * uu) * sq) * het) / (hh * hh);
+  }
+  return tut;
 }
 
 }  // namespace mpsw

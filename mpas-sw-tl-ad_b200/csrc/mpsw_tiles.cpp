@@ -502,7 +502,7 @@ void stage_pack(const Builder &b, const BuiltMesh &m, const Space &E, const Spac
   }
   std::memcpy(p + off[SB_GE], E.list.data(), 4 * E.list.size());
   std::memcpy(p + off[SB_GC], C.list.data(), 4 * C.list.size());
-  std::memcpy(p + off[SB_GV], V.list.data(), 4 * (size_t)n[S_VO]);
+  std::memcpy(p + off[SB_GV], V.list.data(), 4 * (size_t)nv);
 }
 
 }  // namespace

@@ -620,6 +620,13 @@ static void tl_member_stage(Engine &E, int prec, int B, double *du, double *dh, 
     Launch<R, double>::tl_fused(E.fused, M, m, B, bs, uti, hti, ph, rut, rht, st);
     return;
   }
+  if constexpr (f64) {
+    if (E.stage_tl_tiled(B)) {
+      Launch<R, double>::stage_tl(E.st64, StageTlArgs{uti, hti, B, bs, ph, rut, rht, nullptr, nullptr, m.e_sc2, m.e_sc4,
+                                              m.e_usrc}, st);
+      return;
+    }
+  }
   const Diag<R> d = tl_rows(mb, ph);
   if (Launch<R, double>::rows_ok(E.rows, E.nE, B, ph, false)) {
     for (int part = 0; part < 3; part++) {
@@ -667,7 +674,7 @@ static void window_tl_impl(Engine &E, int prec, int Bu, double *user_u, double *
     key.p3 = W.st[prec].mem;
     key.n2 = ((long long)W.nsteps << 20) | W.every;
     StableBaseScope stable(true);  // the members read only stored stages
-    E.beside_members = true;
+    E.beside_members = prec == 1 || !E.stage_tl_tiled(B);  // (tiled members leave the tiles room)
     struct Reset {
       bool &b;
       ~Reset() { b = false; }
@@ -1031,6 +1038,13 @@ static double time_kernel_impl(Engine &E, int which, int prec, int B, int iters,
           LR::tl_fused(E.fused, M, m, B, bs, mb->pu[0], mb->ph[0], ph, rku, rkh, E.stream);
           break;
         }
+        if constexpr (sizeof(R) == 8) {
+          if (E.stage_tl_tiled(B)) {
+            LR::stage_tl(E.st64, StageTlArgs{mb->pu[0], mb->ph[0], B, bs, ph, rku, rkh, nullptr, nullptr, m.e_sc2, m.e_sc4,
+                                             m.e_usrc}, E.stream);
+            break;
+          }
+        }
         if (tl_rows_on) {
           tl(0);
           tl(1);
@@ -1103,6 +1117,7 @@ static TuneTable tune_members(Engine &E, int prec, int B) {
   const Phys<R> ph = phys_as<R>(E.phys());
   const int vs[] = {1, 2, 4, 8}, blocks[] = {64, 128, 256};
   for (int k = 0; k < K_TUNED; k++) {
+    if (sizeof(R) == 8 && k < K_AD_EDGE && E.stage_tl_tiled(B)) continue;  // the sweeps do not run it
     double tbest = 1e30;
     for (int v : vs) {
       if (B % v || (sizeof(R) == 8 && v > 4) || (sizeof(R) == 4 && v < 2 && B % 2 == 0)) continue;
