@@ -496,7 +496,7 @@ void Engine::free_device_mesh() {
   mesh_built = false;
   fused = FusedDev();
   fused_K = 0;
-  st64 = st32 = StageDev();
+  st64 = st32 = st_ad = StageDev();
   rows = RowTab();
 }
 
@@ -551,7 +551,7 @@ void Engine::build_fused() {
 // MPSW_STAGE_TILES=0 keeps the passes.
 void Engine::build_stage() {
   constexpr size_t kL2 = (size_t)110 << 20;
-  st64 = st32 = StageDev();
+  st64 = st32 = st_ad = StageDev();
   const char *off = getenv("MPSW_STAGE_TILES");
   if ((off && atoi(off) == 0) || (size_t)nC * 1200 > kL2) return;
   const int share = std::max(8, (nC + 147) / 148);
@@ -566,6 +566,12 @@ void Engine::build_stage() {
     d.cnt = cnt;
     d.blob_off = up<long long>(p ? t.off32 : t.off64, mesh_bufs);
     d.blob = up<unsigned char>(blob, mesh_bufs);
+  }
+  if (st64.ntiles && build_stage_ad_tiles(bm, share < 60 ? share : 96, &t).empty() && t.blob64.size() <= kL2) {
+    st_ad.ntiles = t.ntiles;
+    st_ad.cnt = up<int>(t.cnt, mesh_bufs);
+    st_ad.blob_off = up<long long>(t.off64, mesh_bufs);
+    st_ad.blob = up<unsigned char>(t.blob64, mesh_bufs);
   }
   cuda_check(Launch<double, double>::stage_prepare(), "nonlinear stage shared-memory limit");
   cuda_check(Launch<float, double>::stage_prepare(), "nonlinear stage shared-memory limit");
@@ -821,6 +827,14 @@ bool Engine::stage_tiled() const { return st64.ntiles > 0 && (!beside_members ||
 // From three on the passes read whole rows of members and win (level 5, three: 27.4 against 30.8).
 bool Engine::stage_tl_tiled(int B) const {
   return st64.ntiles > 0 && (B == 1 || (B == 2 && st64.ntiles <= 2 * 148));
+}
+
+// The adjoint's line is the tangent linear's, for its reasons (passes -> tiles: level 3 19.0 -> 5.2, level 4
+// 20.0 -> 6.3, level 5 24.4 -> 9.5, level 6 39.3 -> 31.2; two members 15.2 -> 6.3, 16.4 -> 7.7, 21.6 -> 17.1);
+// viscosity and drag, which add layers and terms to every phase, keep the passes.
+bool Engine::stage_ad_tiled(int B, const Phys<double> &ph) const {
+  return st_ad.ntiles > 0 && (B == 1 || (B == 2 && st_ad.ntiles <= 2 * 148)) && !(ph.visc2 > 0.0) && !(ph.visc4 > 0.0) &&
+         !ph.drag;
 }
 
 static StageBaseOut base_out(const Diag<double> &d) {  // (u is the stage's input itself)
@@ -1261,7 +1275,9 @@ void Engine::rk4_adj() {  // src/mpas_sw_module.f90:783-1002
       out.wh = w[k - 1];
       out.ch = c[k - 1];
     }
-    L64::ad_stage(m64, 1, base_of(stage[k + 1], ui), ph, in, none, adw, out, stream);
+    const Base<double> bs = base_of(stage[k + 1], ui);
+    if (stage_ad_tiled(1, ph)) L64::stage_ad(st_ad, StageAdArgs{in, 1, bs, ph, out, m64.e_usrc}, stream);
+    else L64::ad_stage(m64, 1, bs, ph, in, none, adw, out, stream);
   }
   cuda_check(cudaMemsetAsync(dv("u_ad", 1), 0, sizeof(double) * nE, stream), "memset");
   cuda_check(cudaMemsetAsync(dv("h_ad", 1), 0, sizeof(double) * nC, stream), "memset");

@@ -137,6 +137,7 @@ struct Engine {
   int fused_K = 0;             // owned cells per tile of `fused` (0: not built)
   void build_fused();
   StageDev st64, st32;         // halo tiles of the nonlinear stage, FP64 and FP32 stencils
+  StageDev st_ad;              // tiles of the FP64 adjoint stage
   void build_stage();
   RowTab rows;                 // tables of the FP32 member-row passes
   void build_row_tables();
@@ -218,6 +219,7 @@ struct Engine {
                  const StageBaseOut &out);
   bool stage_tiled() const;
   bool stage_tl_tiled(int B) const;  // FP64 members take the tiles' tangent-linear stage
+  bool stage_ad_tiled(int B, const Phys<double> &ph) const;  // and the adjoint's
   void tl_diag_run(const Base<double> &bs, const double *ut, const double *ht, const Diag<double> &d,
                    const Phys<double> &ph);
   void check_launch(const char *what);

@@ -200,10 +200,19 @@ template <typename R, typename A>
 void Launch<R, A>::stage_tl(const StageDev &ts, const StageTlArgs &a, cudaStream_t s) {
   if constexpr (std::is_same<R, double>::value) {
     g_launches++;
-    launch_k(k_stage_tl<R>, LaunchCfg{ts.ntiles, kStageThreads, stage_tl_smem(a.ph.visc2 > 0.0 || a.ph.visc4 > 0.0, a.ph.visc4 > 0.0), a.B}, s, ts, a,
-             (int)g_stable_base);
+    const size_t smem = stage_tl_smem(a.ph.visc2 > 0.0 || a.ph.visc4 > 0.0, a.ph.visc4 > 0.0);
+    launch_k(k_stage_tl<R>, LaunchCfg{ts.ntiles, kStageThreads, smem, a.B}, s, ts, a, (int)g_stable_base);
   } else {
     throw std::invalid_argument("the tiles' tangent-linear stage runs FP64 members");
+  }
+}
+template <typename R, typename A>
+void Launch<R, A>::stage_ad(const StageDev &ts, const StageAdArgs &a, cudaStream_t s) {
+  if constexpr (std::is_same<R, double>::value) {
+    g_launches++;
+    launch_k(k_stage_ad<R>, LaunchCfg{ts.ntiles, kAdThreads, kStageAdSmem, a.B}, s, ts, a, (int)g_stable_base);
+  } else {
+    throw std::invalid_argument("the tiles' adjoint stage runs FP64 members");
   }
 }
 template <typename R, typename A>
@@ -212,6 +221,9 @@ cudaError_t Launch<R, A>::stage_prepare() {
     const cudaError_t e = cudaFuncSetAttribute((const void *)k_stage_tl<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                (int)stage_tl_smem(true, true));
     if (e != cudaSuccess) return e;
+    const cudaError_t f = cudaFuncSetAttribute((const void *)k_stage_ad<double>,
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStageAdSmem);
+    if (f != cudaSuccess) return f;
   }
   return cudaFuncSetAttribute((const void *)k_stage<R, A>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)stage_smem<R>(true, true));

@@ -60,6 +60,8 @@ struct Launch {
   static cudaError_t stage_prepare();
   // a tangent-linear stage of B FP64 members on the same tiles (one member a block)
   static void stage_tl(const StageDev &ts, const StageTlArgs &a, cudaStream_t s);
+  // an adjoint stage of B FP64 members on the adjoint's tiles (no viscosity, no drag, no seeds)
+  static void stage_ad(const StageDev &ts, const StageAdArgs &a, cudaStream_t s);
   static void tend_h(const MeshDev<R> &m, const R *u, const R *he, R *out, cudaStream_t s);
   static void tracer_stage(const MeshDev<R> &m, const int *c_nb, int nT, const R *u, const R *he, const R *tr_in,
                            R *tr0, const R *h0, const R *h_next, R *tend, R *acc, R *tr_next, R c, R w, int first,

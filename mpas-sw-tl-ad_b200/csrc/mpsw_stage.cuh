@@ -381,4 +381,163 @@ __global__ void __launch_bounds__(kStageThreads, 2) k_stage_tl(StageDev ts, Stag
   }
 }
 
+// Destination bookkeeping of one value of an adjoint member sweep (ad_emit with one member)
+struct StageAdOut {
+  double x = 0.0, p[3] = {0.0, 0.0, 0.0};
+  __device__ __forceinline__ void fetch(const AdOut<double, double> &out, bool edge, size_t o) {
+    const double *x2 = edge ? out.x2u : out.x2h, *acc = edge ? out.acc_u : out.acc_h;
+    const double *const *pin = edge ? out.pad_in_u : out.pad_in_h;
+    if (x2) x = __ldcg(x2 + o);
+    if (out.mode == AD_FINAL && pin[0]) {
+#pragma unroll
+      for (int j = 0; j < 3; j++) p[j] = __ldcg(pin[j] + o);
+    } else if (out.mode == AD_FINAL || (out.mode == AD_ADD && !(edge ? out.pad_out_u : out.pad_out_h))) {
+      p[0] = __ldcg(acc + o);
+    }
+  }
+  __device__ __forceinline__ void put(const AdOut<double, double> &out, bool edge, size_t o, double pad, double area) const {
+    double *tn = edge ? out.tu_next : out.th_next;
+    const double wn = edge ? out.wu : out.wh, cn = edge ? out.cu : out.ch;
+    double next;
+    if (out.mode == AD_FINAL) {
+      double a = p[0];
+      if (out.pad_in_u[0]) a = (a + p[1]) + p[2];
+      const double d = (a + x) + pad;
+      (edge ? out.dst_u : out.dst_h)[o] = d;
+      next = wn * d;
+    } else {
+      double *pout = edge ? out.pad_out_u : out.pad_out_h;
+      if (pout) pout[o] = pad;
+      else (edge ? out.acc_u : out.acc_h)[o] = out.mode == AD_SET ? pad : p[0] + pad;
+      next = ((edge ? out.x2u : out.x2h) ? wn * x : 0.0) + cn * pad;
+    }
+    if (tn) tn[o] = edge ? next : next / area;
+  }
+};
+
+// An adjoint stage of FP64 members, one a block (blockIdx.y), on the adjoint's tiles; bound by the chain of
+// its phases, like k_stage_tl, and fetching as that does.  The divisions by dc and dv that the cells and
+// vertices each need are formed once an edge.  384 threads leave 80 registers for the edge records (two
+// weights a slot) with two blocks an SM (97 KB each).  9.5 us a level-5 stage of one member, 24.4 as four
+// passes.
+template <typename R>  // double
+__global__ void __launch_bounds__(kAdThreads, 2) k_stage_ad(StageDev ts, StageAdArgs a, int early) {
+  static_assert(sizeof(R) == 8);
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ __align__(8) unsigned long long arrived;
+  constexpr int NT = kAdThreads;
+  constexpr int RV = 0, RC = RV + 16 * kAdVA * kAdRowsV, RO = RC + 16 * kAdCM * kAdRowsC;
+  const int tid = threadIdx.x, B = a.B, mb = blockIdx.y;
+  unsigned char *const w = smem_raw, *const rec = w + 8 * Y_END;
+  int n[kTileCounts], off[kStageAdSections];
+#pragma unroll
+  for (int k = 0; k < kTileCounts; k++) n[k] = __ldg(ts.cnt + (size_t)blockIdx.x * kTileCounts + k);
+  stage_ad_layout(n, off);
+  const unsigned char *g = ts.blob + __ldg(ts.blob_off + blockIdx.x);
+  if (tid < 32) {  // one bulk copy per chunk row of the records
+    if (tid == 0) {
+      asm volatile("mbarrier.init.shared.b64 [%0], 1;" ::"r"(smem_addr(&arrived)) : "memory");
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+      const int bytes = 16 * (kAdRowsV * n[V_ALL] + kAdRowsC * n[C_MID] + kAdRowsO * n[C_OWN]);
+      asm volatile("mbarrier.arrive.expect_tx.shared.b64 _, [%0], %1;" ::"r"(smem_addr(&arrived)), "r"(bytes)
+                   : "memory");
+    }
+    __syncwarp();
+    if (tid < kAdRowsV + kAdRowsC + kAdRowsO) {
+      const int k = tid < kAdRowsV ? 0 : tid < kAdRowsV + kAdRowsC ? 1 : 2;
+      const int row = tid - (k == 0 ? 0 : k == 1 ? kAdRowsV : kAdRowsV + kAdRowsC);
+      const int cnt = k == 0 ? n[V_ALL] : k == 1 ? n[C_MID] : n[C_OWN], cap = k == 0 ? kAdVA : k == 1 ? kAdCM : kAdCO;
+      asm volatile(
+          "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+              smem_addr(rec + (k == 0 ? RV : k == 1 ? RC : RO) + 16 * cap * row)),
+          "l"(g + off[k == 0 ? YB_V : k == 1 ? YB_C : YB_O] + 16 * cnt * row), "r"(16 * cnt), "r"(smem_addr(&arrived))
+          : "memory");
+    }
+  }
+  auto sec = [&](int o) { return reinterpret_cast<const StageChunk *>(rec + o); };
+  AdEdgeRec er;
+  if (tid < n[E_MID]) stage_rec(reinterpret_cast<const StageChunk *>(g + off[YB_E]), n[E_MID], tid, &er);
+  const int *ids = reinterpret_cast<const int *>(g + off[YB_GE]), *idc = reinterpret_cast<const int *>(g + off[YB_GC]);
+  int ge[2] = {0, 0}, gc = 0, gv = 0;
+  if (tid < n[E_ALL]) ge[0] = __ldg(ids + tid);
+  if (tid + NT < n[E_ALL]) ge[1] = __ldg(ids + tid + NT);
+  if (tid < n[C_ALL]) gc = __ldg(idc + tid);
+  if (tid < n[V_ALL]) gv = __ldg(reinterpret_cast<const int *>(g + off[YB_GV]) + tid);
+  const int top = NT - 1 - tid;
+  const bool edge = tid < n[E_OWN], cell = top < n[C_OWN];
+  const int own = edge ? ge[0] : cell ? __ldg(idc + top) : 0;
+  double vb = 0.0, gpt = 0.0, gpn = 0.0, src = 0.0, hv = 1.0, vort = 0.0;
+  auto base = [&]() {
+    double b[2][3] = {};
+#pragma unroll
+    for (int k = 0; k < 2; k++)
+      if (tid + k * NT < n[E_ALL]) {
+        b[k][0] = __ldcg(a.bs.u + ge[k]);
+        b[k][1] = __ldcg(a.bs.he + ge[k]);
+        b[k][2] = __ldcg(a.bs.pe + ge[k]);
+      }
+    if (tid < n[E_MID]) {
+      vb = __ldcg(a.bs.v + ge[0]);
+      gpt = __ldcg(a.bs.gpt + ge[0]);
+      gpn = __ldcg(a.bs.gpn + ge[0]);
+    }
+    if (tid < n[V_ALL]) {
+      hv = __ldcg(a.bs.hv + gv);
+      vort = __ldcg(a.bs.vort + gv);
+    }
+#pragma unroll
+    for (int k = 0; k < 2; k++)
+      if (tid + k * NT < n[E_ALL]) {
+        stage_val<double>(w, Y_UB + tid + k * NT, 0) = b[k][0];
+        stage_val<double>(w, Y_HB + tid + k * NT, 0) = b[k][1];
+        stage_val<double>(w, Y_PB + tid + k * NT, 0) = b[k][2];
+      }
+  };
+  if (a.ph.wind && tid < n[E_MID]) src = __ldg(a.usrc + ge[0]);
+  if (early) base();
+  pdl_begin();
+  if (!early) base();
+  StageAdOut out;
+  {
+    double u0 = 0.0, u1 = 0.0, h = 0.0;  // in flight together
+    if (tid < n[E_ALL]) u0 = __ldcg(a.in.tu + (size_t)ge[0] * B + mb);
+    if (tid + NT < n[E_ALL]) u1 = __ldcg(a.in.tu + (size_t)ge[1] * B + mb);
+    if (tid < n[C_ALL]) h = __ldcg(a.in.th + (size_t)gc * B + mb);
+    if (edge || cell) out.fetch(a.out, edge, (size_t)own * B + mb);
+    if (tid < n[E_ALL]) stage_val<double>(w, Y_TU + tid, 0) = u0;
+    if (tid + NT < n[E_ALL]) stage_val<double>(w, Y_TU + tid + NT, 0) = u1;
+    if (tid < n[C_ALL]) stage_val<double>(w, Y_TH + tid, 0) = h;
+  }
+  __syncthreads();
+  if (!stage_arrived(&arrived)) {
+    if (a.ph.bad) *a.ph.bad = 1;
+    return;
+  }
+  double ud = 0.0;
+  if (tid < n[E_MID]) ud = stage_ad_edge(er, w, a, tid, vb, gpt, gpn, src);
+  __syncthreads();
+  if (tid < n[C_MID]) {
+    AdCellRec r;
+    stage_rec(sec(RC), kAdCM, tid, &r);
+    stage_ad_cell(r, w, tid);
+  }
+  __syncthreads();
+  if (tid < n[V_ALL]) {
+    AdVertexRec r;
+    stage_rec(sec(RV), kAdVA, tid, &r);
+    stage_ad_vertex(r, w, tid, hv, vort);
+  }
+  __syncthreads();
+  if (edge) {
+    const double pu = stage_ad_final(er, w, ud, stage_val<double>(w, Y_UB + tid, 0));
+    flag_nonfinite(a.ph.bad, pu);
+    out.put(a.out, true, (size_t)own * B + mb, pu, 1.0);
+  } else if (cell) {
+    AdCellRec r;
+    stage_rec(sec(RO), kAdCO, top, &r);
+    out.put(a.out, false, (size_t)own * B + mb, stage_ad_thick(r, w, top), r.v[6]);
+  }
+}
+inline constexpr size_t kStageAdSmem = 8 * Y_END + 16 * (kAdVA * kAdRowsV + kAdCM * kAdRowsC + kAdCO * kAdRowsO);
+
 }  // namespace mpsw

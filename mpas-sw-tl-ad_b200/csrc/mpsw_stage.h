@@ -469,4 +469,154 @@ MPSW_HD inline double stage_tl_tend(const EdgeRec<double> &r, unsigned char *w, 
   return tut;
 }
 
+// ---- adjoint stage of one FP64 member (src/mpas_sw_dyncore_adj.f90), no viscosity and no drag ------
+// Tiles of their own, with the fused adjoint stage's layers (TileLayer): each phase gathers what the phase
+// before formed, edges (E_MID) -> cells (C_MID) -> vertices (V_ALL) -> owned edges and cells.
+constexpr int kAdThreads = 384;  // one a pv_edge layer edge
+constexpr int kAdEM = 384, kAdEA = 672, kAdCO = 96, kAdCM = 160, kAdCA = 256, kAdVA = 256;
+MPSW_HD inline bool stage_ad_fits(const int *n) {
+  return n[E_MID] <= kAdEM && n[E_ALL] <= kAdEA && n[C_OWN] <= kAdCO && n[C_MID] <= kAdCM && n[C_ALL] <= kAdCA &&
+         n[V_ALL] <= kAdVA && stage_up32(n[E_OWN]) + stage_up32(n[C_OWN]) <= kAdThreads;
+}
+
+// Values in shared memory: u, h_edge, pv_edge of the linearisation point and the tendency adjoints; per
+// edge the adjoints of pv_edge and h_edge, gradPVn_ad / dc, tu / dc, g / dc tu, gradPVt_ad / dv, v_ad;
+// pv_cell_ad, ke_ad / area, h_ad on cells; h_vertex_ad and circulation_ad on vertices.
+enum StageAdWork {
+  Y_UB = 0,
+  Y_HB = Y_UB + kAdEA,
+  Y_PB = Y_HB + kAdEA,
+  Y_TU = Y_PB + kAdEA,
+  Y_TH = Y_TU + kAdEA,
+  Y_PE = Y_TH + kAdCA,
+  Y_HE = Y_PE + kAdEM,
+  Y_GN = Y_HE + kAdEM,
+  Y_TD = Y_GN + kAdEM,
+  Y_TG = Y_TD + kAdEM,
+  Y_GT = Y_TG + kAdEM,
+  Y_VA = Y_GT + kAdEM,
+  Y_PC = Y_VA + kAdEM,
+  Y_KE = Y_PC + kAdCM,
+  Y_HD = Y_KE + kAdCM,
+  Y_HV = Y_HD + kAdCM,
+  Y_CI = Y_HV + kAdVA,
+  Y_END = Y_CI + kAdVA
+};
+static_assert(Y_END % 2 == 0, "the records behind start on 16 bytes");
+
+// A blob, records as above:
+//   vertices:     edges[3] cells[3] edgesOnVertex[3]; sign [3], kite / areaCell [3], area, f
+//   C_MID cells:  edges[6]; sign [6] (0 past the list), area
+//   owned cells:  vertices[6]; kite / areaTriangle [6], area
+//   E_MID edges:  c1 c2 v1 v2 edgesOnEdge[10]; weights [10], transposed weights [10], dc, dv
+enum StageAdSection { YB_V, YB_C, YB_O, YB_E, YB_GE, YB_GC, YB_GV, kStageAdSections };
+constexpr int kAdValsV = 8, kAdValsC = 7, kAdValsO = 7, kAdValsE = 22;
+constexpr int kAdRowsV = 6, kAdRowsC = 5, kAdRowsO = 5;  // chunk rows
+MPSW_HD inline int stage_ad_layout(const int *n, int *off) {
+  int o = 0;
+  off[YB_V] = o; o += 16 * n[V_ALL] * kAdRowsV;
+  off[YB_C] = o; o += 16 * n[C_MID] * kAdRowsC;
+  off[YB_O] = o; o += 16 * n[C_OWN] * kAdRowsO;
+  off[YB_E] = o; o += 16 * n[E_MID] * (2 + stage_chunks(kAdValsE, 8));
+  off[YB_GE] = o; o += (4 * n[E_ALL] + 15) / 16 * 16;
+  off[YB_GC] = o; o += (4 * n[C_ALL] + 15) / 16 * 16;
+  off[YB_GV] = o; o += (4 * n[V_ALL] + 15) / 16 * 16;
+  return o;
+}
+using AdVertexRec = StageRec<double, 2, kAdValsV>;
+using AdCellRec = StageRec<double, 1, kAdValsC>;
+using AdEdgeRec = StageRec<double, 2, kAdValsE>;
+
+struct StageAdArgs {
+  AdIn<double> in;  // rows of B members
+  int B;
+  Base<double> bs;
+  Phys<double> ph;
+  AdOut<double, double> out;
+  const double *usrc;
+};
+
+// (:689-736, :567-572, :193-200, :235-242); returns the edge's direct share of u_ad
+MPSW_HD inline double stage_ad_edge(const AdEdgeRec &r, unsigned char *w, const StageAdArgs &a, int i, double vb,
+                                    double gpt, double gpn, double usrc) {
+  const double Te = stage_val<double>(w, Y_TU + i, 0), ue = stage_val<double>(w, Y_UB + i, 0);
+  const double hee = stage_val<double>(w, Y_HB + i, 0), pee = stage_val<double>(w, Y_PB + i, 0);
+  const double dc = r.v[20], dv = r.v[21];
+  double pe = 0.0, he = 0.0, ud = 0.0;
+#pragma unroll
+  for (int j = 0; j < 10; j++) {
+    const int e = r.at(4 + j);
+    const double wt = r.v[j], wr = r.v[10 + j], Tn = stage_val<double>(w, Y_TU, e);
+    pe = pe + 0.5 * (((wt * stage_val<double>(w, Y_UB, e)) * stage_val<double>(w, Y_HB, e)) * Te);
+    const double wpv = 0.5 * (stage_val<double>(w, Y_PB, e) + pee);
+    he = he + ((wr * ue) * wpv) * Tn;
+    pe = pe + 0.5 * (((wr * ue) * hee) * Tn);
+    ud = ud + ((wr * wpv) * hee) * Tn;
+  }
+  const double fa = stage_val<double>(w, Y_TH, r.at(1)) - stage_val<double>(w, Y_TH, r.at(0));
+  he = he + (ue * dv) * fa;
+  ud = ud + (dv * hee) * fa;
+  if (a.ph.wind) he = he - ((usrc / RHO_REF) / (hee * hee)) * Te;
+  const double gn = 0.0 - ((a.ph.apvm * ue) * a.ph.dt) * pe;
+  ud = ud - ((a.ph.apvm * a.ph.dt) * gpn) * pe;
+  const double gt = 0.0 - ((a.ph.apvm * vb) * a.ph.dt) * pe;
+  stage_val<double>(w, Y_PE + i, 0) = pe;
+  stage_val<double>(w, Y_HE + i, 0) = he;
+  stage_val<double>(w, Y_GN + i, 0) = gn / dc;
+  stage_val<double>(w, Y_TD + i, 0) = Te / dc;
+  stage_val<double>(w, Y_TG + i, 0) = (GRAVITY / dc) * Te;
+  stage_val<double>(w, Y_GT + i, 0) = gt / dv;
+  stage_val<double>(w, Y_VA + i, 0) = 0.0 - ((a.ph.apvm * a.ph.dt) * gpt) * pe;
+  return ud;
+}
+// (:202-213, :696-699, :358-369, :306-317)
+MPSW_HD inline void stage_ad_cell(const AdCellRec &r, unsigned char *w, int i) {
+  double pc = 0.0, ke = 0.0, hd = 0.0;
+#pragma unroll
+  for (int k = 0; k < 6; k++) {
+    const int e = r.at(k);
+    const double sg = r.v[k];
+    pc = pc + (-sg) * stage_val<double>(w, Y_GN, e);
+    ke = ke + sg * stage_val<double>(w, Y_TD, e);
+    hd = hd + sg * stage_val<double>(w, Y_TG, e);
+    hd = hd + (0.5 * fabs(sg)) * stage_val<double>(w, Y_HE, e);
+  }
+  stage_val<double>(w, Y_PC + i, 0) = pc;
+  stage_val<double>(w, Y_KE + i, 0) = ke / r.v[6];
+  stage_val<double>(w, Y_HD + i, 0) = hd;
+}
+// (:215-229, :244-262, :268-284, :343-349); hv, vort: the linearisation point's
+MPSW_HD inline void stage_ad_vertex(const AdVertexRec &r, unsigned char *w, int i, double hv, double vort) {
+  double pv = 0.0, vo = 0.0, hva = 0.0;
+#pragma unroll
+  for (int k = 0; k < VDEG; k++) pv = pv + r.v[3 + k] * stage_val<double>(w, Y_PC, r.at(3 + k));
+#pragma unroll
+  for (int k = 0; k < VDEG; k++) pv = pv + 0.5 * stage_val<double>(w, Y_PE, r.at(6 + k));
+#pragma unroll
+  for (int k = 0; k < VDEG; k++) pv = pv + r.v[k] * stage_val<double>(w, Y_GT, r.at(k));
+  hva = hva - ((r.v[7] + vort) / (hv * hv)) * pv;
+  vo = vo + pv / hv;
+  stage_val<double>(w, Y_HV + i, 0) = hva / r.v[6];
+  stage_val<double>(w, Y_CI + i, 0) = 0.0 + vo / r.v[6];
+}
+// (:296-317, :350-355); ud: stage_ad_edge's, ub: the linearisation point's u
+MPSW_HD inline double stage_ad_final(const AdEdgeRec &r, unsigned char *w, double ud, double ub) {
+  double pu = ud;
+#pragma unroll
+  for (int j = 0; j < 10; j++) pu = pu + r.v[10 + j] * stage_val<double>(w, Y_VA, r.at(4 + j));
+  const double dc = r.v[20], dv = r.v[21], kc = (((0.25 * dc) * dv) * 2.0) * ub;
+  pu = pu + kc * stage_val<double>(w, Y_KE, r.at(0));
+  pu = pu + kc * stage_val<double>(w, Y_KE, r.at(1));
+  pu = pu + dc * stage_val<double>(w, Y_CI, r.at(3));
+  pu = pu - dc * stage_val<double>(w, Y_CI, r.at(2));
+  return pu;
+}
+// (:286-289)
+MPSW_HD inline double stage_ad_thick(const AdCellRec &r, unsigned char *w, int i) {
+  double h = stage_val<double>(w, Y_HD + i, 0);
+#pragma unroll
+  for (int k = 0; k < 6; k++) h = h + r.v[k] * stage_val<double>(w, Y_HV, r.at(k));
+  return h;
+}
+
 }  // namespace mpsw

@@ -540,4 +540,100 @@ std::string build_stage_tiles(const BuiltMesh &m, int kmax, StageSetHost *o) {
   return "";
 }
 
+// ---- tiles of the FP64 adjoint stage (mpsw_stage.h) -----------------------------------------------
+namespace {
+
+void stage_ad_pack(const Builder &b, const BuiltMesh &m, const Space &E, const Space &C, const Space &V, const int *n,
+                   std::vector<unsigned char> *blob) {
+  int off[kStageAdSections];
+  const int size = stage_ad_layout(n, off);
+  const size_t base = blob->size();
+  blob->resize(base + (size_t)size, 0);
+  unsigned char *p = blob->data() + base;
+  auto list = [&](int sec, int cnt, int i, int k, int x) {
+    reinterpret_cast<uint16_t *>(p + off[sec] + 16 * ((k >> 3) * cnt + i))[k & 7] = (uint16_t)(8 * std::max(x, 0));
+  };
+  auto val = [&](int sec, int cnt, int lists, int i, int k, double x) {
+    reinterpret_cast<double *>(p + off[sec] + 16 * ((lists + k / 2) * cnt + i))[k % 2] = x;
+  };
+  const int nv = n[V_ALL], ncm = n[C_MID], nco = n[C_OWN], nem = n[E_MID];
+  for (int i = 0; i < nv; i++) {
+    const int v = V.list[i];
+    for (int k = 0; k < VDEG; k++) {
+      const size_t s = (size_t)k * m.nV + v;
+      list(YB_V, nv, i, k, E.local(m.v_es[s]));
+      list(YB_V, nv, i, 3 + k, C.local(m.v_c[s]));
+      list(YB_V, nv, i, 6 + k, E.local(m.v_e[s]));
+      val(YB_V, nv, 2, i, k, m.v_esg[s]);
+      val(YB_V, nv, 2, i, 3 + k, m.v_k[s] / m.c_area[m.v_c[s]]);
+    }
+    val(YB_V, nv, 2, i, 6, m.v_area[v]);
+    val(YB_V, nv, 2, i, 7, m.v_f[v]);
+  }
+  for (int i = 0; i < ncm; i++) {
+    const int c = C.list[i];
+    for (int k = 0; k < b.cn(c); k++) {
+      const size_t s = (size_t)k * m.nC + c;
+      list(YB_C, ncm, i, k, E.local(m.c_es[s]));
+      val(YB_C, ncm, 1, i, k, m.c_esg[s]);
+      if (i >= nco) continue;
+      list(YB_O, nco, i, k, V.local(m.c_vs[s]));
+      val(YB_O, nco, 1, i, k, m.c_vk[s]);
+    }
+    val(YB_C, ncm, 1, i, 6, m.c_area[c]);
+    if (i < nco) val(YB_O, nco, 1, i, 6, m.c_area[c]);
+  }
+  for (int i = 0; i < nem; i++) {
+    const int e = E.list[i];
+    list(YB_E, nem, i, 0, C.local(m.e_c1[e]));
+    list(YB_E, nem, i, 1, C.local(m.e_c2[e]));
+    list(YB_E, nem, i, 2, V.local(m.e_v1[e]));  // (read for owned edges only)
+    list(YB_E, nem, i, 3, V.local(m.e_v2[e]));
+    for (int j = 0; j < kEoeSlots; j++) {
+      const bool has = j < m.e_n[e];  // a padded slot weighs nothing
+      list(YB_E, nem, i, 4 + j, has ? E.local(b.eoe(e, j)) : i);
+      val(YB_E, nem, 2, i, j, has ? m.e_w[(size_t)j * m.nE + e] : 0.0);
+      val(YB_E, nem, 2, i, 10 + j, has ? m.e_wrev[(size_t)j * m.nE + e] : 0.0);
+    }
+    val(YB_E, nem, 2, i, 20, m.e_dc[e]);
+    val(YB_E, nem, 2, i, 21, m.e_dv[e]);
+  }
+  std::memcpy(p + off[YB_GE], E.list.data(), 4 * E.list.size());
+  std::memcpy(p + off[YB_GC], C.list.data(), 4 * C.list.size());
+  std::memcpy(p + off[YB_GV], V.list.data(), 4 * V.list.size());
+}
+
+}  // namespace
+
+std::string build_stage_ad_tiles(const BuiltMesh &m, int kmax, StageSetHost *o) {
+  if (kmax < 1) return "tile size must be positive";
+  for (int c = 0; c < m.nC; c++)
+    if (m.c_n[c] > kCellSlots) return "stage tiles need at most 6 edges per cell";
+  for (int e = 0; e < m.nE; e++)
+    if (m.e_n[e] > kEoeSlots) return "stage tiles need at most 10 edgesOnEdge";
+  Builder b(m);
+  *o = StageSetHost();
+  int stamp = 0;
+  for (int c0 = 0; c0 < m.nC;) {
+    int K = std::min(kmax, m.nC - c0), n[kTileCounts];
+    for (;; K = std::max(1, K - (K + 7) / 8)) {  // shorten the run while its halo is too large
+      Space E(b.se, b.le, stamp), C(b.sc, b.lc, stamp), V(b.sv, b.lv, stamp);
+      stamp++;
+      tile_spaces(b, m, c0, c0 + K, true, E, C, V, n);
+      if (!stage_ad_fits(n)) {
+        if (K == 1) return "one cell's halo exceeds a tile";
+        continue;
+      }
+      if (!validate(b, m, E, C, V, n, true)) return fail(o->ntiles, "a phase of the stage would read outside its tile");
+      o->cnt.insert(o->cnt.end(), n, n + kTileCounts);
+      o->off64.push_back((long long)o->blob64.size());
+      stage_ad_pack(b, m, E, C, V, n, &o->blob64);
+      break;
+    }
+    o->ntiles++;
+    c0 += K;
+  }
+  return "";
+}
+
 }  // namespace mpsw

@@ -70,4 +70,8 @@ struct StageSetHost {
 // grid-wide passes).
 std::string build_stage_tiles(const BuiltMesh &m, int kmax, StageSetHost *out);
 
+// Tiles of the FP64 adjoint stage (mpsw_stage.h): cnt holds kTileCounts layers a tile, blob64 / off64 the
+// blobs; at most kmax owned cells each, fewer where a layer would exceed its cap (stage_ad_fits).
+std::string build_stage_ad_tiles(const BuiltMesh &m, int kmax, StageSetHost *out);
+
 }  // namespace mpsw

@@ -767,6 +767,12 @@ static void ad_member_step(Engine &E, int prec, int B, double *au, double *ah, M
       out.wu = wu4;
       out.wh = w[3];
     }
+    if constexpr (sizeof(R) == 8) {
+      if (E.stage_ad_tiled(B, ph)) {
+        Launch<R, double>::stage_ad(E.st_ad, StageAdArgs{in, B, base(k), ph, out, m.e_usrc}, E.stream);
+        continue;
+      }
+    }
     if (const int M = fused_members<R>(E, B, ph))
       Launch<R, double>::ad_fused(E.fused, M, m, B, base(k), ph, in, out, E.stream);
     else if (Launch<R, double>::rows_ok(E.rows, E.nE, B, ph, true))
@@ -1060,6 +1066,12 @@ static double time_kernel_impl(Engine &E, int which, int prec, int B, int iters,
         break;
       case 9: {  // one whole adjoint stage, as the sweeps run it
         const AdSeeds<R> none{};
+        if constexpr (sizeof(R) == 8) {
+          if (E.stage_ad_tiled(B, ph)) {
+            LR::stage_ad(E.st_ad, StageAdArgs{in, B, bs, ph, out, m.e_usrc}, E.stream);
+            break;
+          }
+        }
         if (const int M = fused_members<R>(E, B, ph))
           LR::ad_fused(E.fused, M, m, B, bs, ph, in, out, E.stream);
         else if (ad_rows_on)
@@ -1117,7 +1129,8 @@ static TuneTable tune_members(Engine &E, int prec, int B) {
   const Phys<R> ph = phys_as<R>(E.phys());
   const int vs[] = {1, 2, 4, 8}, blocks[] = {64, 128, 256};
   for (int k = 0; k < K_TUNED; k++) {
-    if (sizeof(R) == 8 && k < K_AD_EDGE && E.stage_tl_tiled(B)) continue;  // the sweeps do not run it
+    if constexpr (sizeof(R) == 8)  // passes that the sweeps do not run
+      if (k < K_AD_EDGE ? E.stage_tl_tiled(B) : E.stage_ad_tiled(B, ph)) continue;
     double tbest = 1e30;
     for (int v : vs) {
       if (B % v || (sizeof(R) == 8 && v > 4) || (sizeof(R) == 4 && v < 2 && B % 2 == 0)) continue;
