@@ -301,7 +301,7 @@ void Launch<R, A>::tl_edge_diag(const MeshDev<R> &m, int B, const Base<R> &bs, c
   constexpr int J = BoundsNarrow::e2;
   constexpr size_t eb = eoe_stage_bytes<R, J, 1, 0>();
   if (use_staged(m, B, v, eb, bk)) {
-    MPSW_VDISPATCH(v, launch_k(tl_edge_diag_st_kernel<R, VV, J>(), staged_cfg(m.nE, B, VV, eb, bk), s, m, B, bs, ut, ht, dd, ph, (int)g_stable_base));
+    MPSW_VDISPATCH(v, launch_k(tl_edge_diag_st_kernel<R, VV, J>(beyond_two_waves((long long)m.nE * (B / VV))), staged_cfg(m.nE, B, VV, eb, bk), s, m, B, bs, ut, ht, dd, ph, (int)g_stable_base));
     return;
   }
   MPSW_VDISPATCH(v, MPSW_BDISPATCH(m, launch_k(k_tl_edge_diag<R, VV, NB>, launch_cfg((long long)(m.nE) * ((B) / (VV)), bk), s, m, B, bs, ut, ht, dd, ph)));
@@ -320,7 +320,7 @@ void Launch<R, A>::tl_edge_tend(const MeshDev<R> &m, int B, const Base<R> &bs, c
   constexpr int J = BoundsNarrow::e2;
   constexpr size_t eb = eoe_stage_bytes<R, J, 1, 3>();
   if (use_staged(m, B, v, eb, bk)) {
-    MPSW_VDISPATCH(v, launch_k(tl_edge_tend_st_kernel<R, A, VV, J>(), staged_cfg(m.nE, B, VV, eb, bk),
+    MPSW_VDISPATCH(v, launch_k(tl_edge_tend_st_kernel<R, A, VV, J>(beyond_two_waves((long long)m.nE * (B / VV))), staged_cfg(m.nE, B, VV, eb, bk),
                                s, m, B, bs, ut, ht, d, ph, rk, tend_u, (int)g_stable_base));
     return;
   }
@@ -357,7 +357,7 @@ static void ad_launch(int which, const MeshDev<R> &m, int B, const Base<R> &bs, 
       constexpr size_t eb = eoe_stage_bytes<R, J, 2, 3>();
       const int bk = tuned_block(K_AD_EDGE);
       if (use_staged(m, B, V, eb, bk))
-        launch_k(ad_edge_st_kernel<R, A, V, J>(), staged_cfg(m.nE, B, V, eb, bk), s, m, B, bs, ph, in, sd, w, (int)g_stable_base);
+        launch_k(ad_edge_st_kernel<R, A, V, J>(beyond_two_waves((long long)m.nE * (B / V))), staged_cfg(m.nE, B, V, eb, bk), s, m, B, bs, ph, in, sd, w, (int)g_stable_base);
       else
         launch_k(k_ad_edge<R, A, V, NB>, launch_cfg((long long)(m.nE) * ((B) / (V)), bk), s, m, B, bs, ph, in, sd, w);
       break;
@@ -365,7 +365,7 @@ static void ad_launch(int which, const MeshDev<R> &m, int B, const Base<R> &bs, 
     case 1: {
       const int bk = tuned_block(K_AD_CELL);
       if (use_staged(m, B, V, ad_cell_stage_bytes<R>(), bk))
-        launch_k(ad_cell_st_kernel<R, A, V>(), staged_cfg(m.nC, B, V, ad_cell_stage_bytes<R>(), bk), s, m, B, bs, ph, in, sd,
+        launch_k(ad_cell_st_kernel<R, A, V>(beyond_two_waves((long long)m.nC * (B / V))), staged_cfg(m.nC, B, V, ad_cell_stage_bytes<R>(), bk), s, m, B, bs, ph, in, sd,
                  w, (int)g_stable_base);
       else
         launch_k(k_ad_cell<R, A, V, NB>, launch_cfg((long long)(m.nC) * ((B) / (V)), bk), s, m, B, bs, ph, in, sd, w);

@@ -25,6 +25,15 @@ inline bool regcap_on() {
   static const bool on = !(std::getenv("MPSW_REGCAP") && std::atoi(std::getenv("MPSW_REGCAP")) == 0);
   return on;
 }
+
+// FP64 members, one or two a thread, beyond two waves: the compiler's 60-72 registers leave 28 of an SM's
+// warps for kernels that wait on gathers; 56 leave 36 (level 6, 8 members, us: tl_edge_diag 32.4 -> 28.6,
+// tl_edge_tend 46.0 -> 43.3, ad_edge 40.3 -> 34.4, ad_cell 23.2 -> 20.7; at 48 spills take it back: 30.9, 45.4,
+// 36.6, 24.1).  Up to two waves the cap only costs (tangent-linear stage, level 6, 4 members 50.8 -> 61.0;
+// level 5, 8 members 22.7 -> 24.6), and four members a thread spill.
+constexpr int kRegsFp64 = 56;
+inline bool beyond_two_waves(long long threads) { return regcap_on() && threads > 2 * 148LL * (65536 / 72); }
+
 #ifndef MPSW_REGS_TL_VERTEX
 #define MPSW_REGS_TL_VERTEX 32
 #endif
@@ -703,14 +712,25 @@ __global__ void __maxnreg__(MPSW_REGS_TL_EDGE_DIAG) k_tl_edge_diag_st_rc(MeshDev
   tl_edge_diag_st_run<float, V, J>(m, B, bs, ut, ht, d, ph, early);
 }
 #endif
+template <int V, int J>
+__global__ void __maxnreg__(kRegsFp64) k_tl_edge_diag_st_rd(MeshDev<double> m, int B, Base<double> bs,
+                                                                        const double *__restrict__ ut,
+                                                                        const double *__restrict__ ht, Diag<double> d,
+                                                                        Phys<double> ph, int early) {
+  tl_edge_diag_st_run<double, V, J>(m, B, bs, ut, ht, d, ph, early);
+}
 template <typename R, int V, int J>
-inline auto tl_edge_diag_st_kernel() {
+inline auto tl_edge_diag_st_kernel(bool many) {
+  if constexpr (std::is_same<R, double>::value && V <= 2) {
+    return many ? &k_tl_edge_diag_st_rd<V, J> : &k_tl_edge_diag_st<R, V, J>;
+  } else {
 #if MPSW_REGS_TL_EDGE_DIAG > 0
-  if constexpr (std::is_same<R, float>::value && V == 8) return regcap_on() ? &k_tl_edge_diag_st_rc<V, J> : &k_tl_edge_diag_st<R, V, J>;
-  else return &k_tl_edge_diag_st<R, V, J>;
+    if constexpr (std::is_same<R, float>::value && V == 8) return regcap_on() ? &k_tl_edge_diag_st_rc<V, J> : &k_tl_edge_diag_st<R, V, J>;
+    else return &k_tl_edge_diag_st<R, V, J>;
 #else
-  return &k_tl_edge_diag_st<R, V, J>;
+    return &k_tl_edge_diag_st<R, V, J>;
 #endif
+  }
 }
 
 // sw_compute_tend_tlm normal-velocity part :564-768 and the RK update.  Body for edge e,
@@ -832,14 +852,26 @@ __global__ void __maxnreg__(MPSW_REGS_TL_EDGE_TEND) k_tl_edge_tend_st_rc(MeshDev
   tl_edge_tend_st_run<float, A, V, J>(m, B, bs, ut, ht, d, ph, rk, tend_u, early);
 }
 #endif
+template <typename A, int V, int J>
+__global__ void __maxnreg__(kRegsFp64) k_tl_edge_tend_st_rd(MeshDev<double> m, int B, Base<double> bs,
+                                                                        const double *__restrict__ ut,
+                                                                        const double *__restrict__ ht, Diag<double> d,
+                                                                        Phys<double> ph, RK<double, A> rk,
+                                                                        double *tend_u, int early) {
+  tl_edge_tend_st_run<double, A, V, J>(m, B, bs, ut, ht, d, ph, rk, tend_u, early);
+}
 template <typename R, typename A, int V, int J>
-inline auto tl_edge_tend_st_kernel() {
+inline auto tl_edge_tend_st_kernel(bool many) {
+  if constexpr (std::is_same<R, double>::value && V <= 2) {
+    return many ? &k_tl_edge_tend_st_rd<A, V, J> : &k_tl_edge_tend_st<R, A, V, J>;
+  } else {
 #if MPSW_REGS_TL_EDGE_TEND > 0
-  if constexpr (std::is_same<R, float>::value && V == 8) return regcap_on() ? &k_tl_edge_tend_st_rc<A, V, J> : &k_tl_edge_tend_st<R, A, V, J>;
-  else return &k_tl_edge_tend_st<R, A, V, J>;
+    if constexpr (std::is_same<R, float>::value && V == 8) return regcap_on() ? &k_tl_edge_tend_st_rc<A, V, J> : &k_tl_edge_tend_st<R, A, V, J>;
+    else return &k_tl_edge_tend_st<R, A, V, J>;
 #else
-  return &k_tl_edge_tend_st<R, A, V, J>;
+    return &k_tl_edge_tend_st<R, A, V, J>;
 #endif
+  }
 }
 
 // ----------------------------------------------------------------------------------------
@@ -988,14 +1020,23 @@ __global__ void __maxnreg__(MPSW_REGS_AD_EDGE) k_ad_edge_st_rc(MeshDev<float> m,
   ad_edge_st_run<float, A, V, J>(m, B, bs, ph, in, sd, w, early);
 }
 #endif
+template <typename A, int V, int J>
+__global__ void __maxnreg__(kRegsFp64) k_ad_edge_st_rd(MeshDev<double> m, int B, Base<double> bs, Phys<double> ph, AdIn<double> in, AdSeeds<double> sd,
+                             AdWork<double> w, int early) {
+  ad_edge_st_run<double, A, V, J>(m, B, bs, ph, in, sd, w, early);
+}
 template <typename R, typename A, int V, int J>
-inline auto ad_edge_st_kernel() {
+inline auto ad_edge_st_kernel(bool many) {
+  if constexpr (std::is_same<R, double>::value && V <= 2) {
+    return many ? &k_ad_edge_st_rd<A, V, J> : &k_ad_edge_st<R, A, V, J>;
+  } else {
 #if MPSW_REGS_AD_EDGE > 0
-  if constexpr (std::is_same<R, float>::value && V == 8) return regcap_on() ? &k_ad_edge_st_rc<A, V, J> : &k_ad_edge_st<R, A, V, J>;
-  else return &k_ad_edge_st<R, A, V, J>;
+    if constexpr (std::is_same<R, float>::value && V == 8) return regcap_on() ? &k_ad_edge_st_rc<A, V, J> : &k_ad_edge_st<R, A, V, J>;
+    else return &k_ad_edge_st<R, A, V, J>;
 #else
-  return &k_ad_edge_st<R, A, V, J>;
+    return &k_ad_edge_st<R, A, V, J>;
 #endif
+  }
 }
 
 // del4 adjoint, first half (:588-634): delsq_vorticity/delsq_circulation adjoint on vertices
@@ -1198,14 +1239,23 @@ __global__ void __maxnreg__(MPSW_REGS_AD_CELL) k_ad_cell_st_rc(MeshDev<float> m,
   ad_cell_st_run<float, A, V>(m, B, bs, ph, in, sd, w, early);
 }
 #endif
+template <typename A, int V>
+__global__ void __maxnreg__(kRegsFp64) k_ad_cell_st_rd(MeshDev<double> m, int B, Base<double> bs, Phys<double> ph, AdIn<double> in, AdSeeds<double> sd, AdWork<double> w,
+                             int early) {
+  ad_cell_st_run<double, A, V>(m, B, bs, ph, in, sd, w, early);
+}
 template <typename R, typename A, int V>
-inline auto ad_cell_st_kernel() {
+inline auto ad_cell_st_kernel(bool many) {
+  if constexpr (std::is_same<R, double>::value && V <= 2) {
+    return many ? &k_ad_cell_st_rd<A, V> : &k_ad_cell_st<R, A, V>;
+  } else {
 #if MPSW_REGS_AD_CELL > 0
-  if constexpr (std::is_same<R, float>::value && V == 8) return regcap_on() ? &k_ad_cell_st_rc<A, V> : &k_ad_cell_st<R, A, V>;
-  else return &k_ad_cell_st<R, A, V>;
+    if constexpr (std::is_same<R, float>::value && V == 8) return regcap_on() ? &k_ad_cell_st_rc<A, V> : &k_ad_cell_st<R, A, V>;
+    else return &k_ad_cell_st<R, A, V>;
 #else
-  return &k_ad_cell_st<R, A, V>;
+    return &k_ad_cell_st<R, A, V>;
 #endif
+  }
 }
 
 // Vertex stage: pv_cell -> pv_vertex (:215-229), pv_edge -> pv_vertex (:244-252),
