@@ -376,6 +376,25 @@ def kernel_bytes(name, nC, nE, nV, sum_eoe, B, s):
     return kb[name]
 
 
+def row_bytes(name, nC, nE, nV, B, s=4):
+    """The same for the FP32 row passes, which replace the vertex kernels by folded coefficients
+    (csrc/mpsw_rows.cuh): the words a block stages per entity (indices and coefficient tables), the
+    linearisation point's fields, each member row in and out, and the RK bookkeeping (3 s)."""
+    E, C, V = nE, nC, nV
+    kb = {
+        'tl_cell': 4 * 72 * C + s * (2 * E + 2 * V) + B * s * (E + C + 2 * C + 3 * C),   # u,h in; pc,ke out; RK
+        'tl_edge_diag': 4 * 38 * E + 6 * s * E + B * s * (E + 2 * C + 2 * E),            # u,h,pc in; pv_edge, flux out
+        'tl_edge_tend': 4 * 30 * E + 3 * s * E + B * s * (2 * E + C + 3 * E),            # flux,pv_edge,ke in; RK
+        'ad_edge': 4 * 50 * E + 6 * s * E + B * s * (E + C + 3 * E),
+        'ad_cell': 4 * 48 * C + s * (2 * E + 2 * V) + B * s * (3 * E + 2 * C),
+        'ad_final': 4 * 34 * E + 4 * 24 * C + s * (2 * E + 2 * V) + B * s * (2 * E + 2 * C + 3 * (E + C)),
+        'tl_vertex': 0, 'ad_vertex': 0,
+    }
+    kb['tl_stage'] = sum(kb[k] for k in ('tl_cell', 'tl_edge_diag', 'tl_edge_tend'))
+    kb['ad_stage'] = sum(kb[k] for k in ('ad_edge', 'ad_cell', 'ad_final'))
+    return kb[name]
+
+
 def fused_bytes(name, nC, nE, nV, B, s=4, a=8):
     """Bytes a fused stage launch must move (a middle stage as the sweeps and mpsw_time_kernel run
     it; default physics): every mesh coefficient, linearisation-point value and member value it
@@ -500,7 +519,7 @@ def run_mpsw(a, rank, world):
         torch.cuda.synchronize()
         fm, fk = ctypes.c_int(), ctypes.c_int()
         eng.h.check(L.mpsw_window_fused(eng.h.ptr, FP32, B, ctypes.byref(fm), ctypes.byref(fk)), 'window_fused')
-        # the kernels the sweeps launch: the two fused stages (8, 9) or the eight split kernels
+        # the kernels the sweeps launch: the two fused stages (8, 9) or the split kernels
         which = [8, 9] if fm.value else list(range(len(KERNELS) - 2))
         torch.cuda.nvtx.range_push('mpsw_kernels')
         for i in which:
@@ -579,7 +598,7 @@ def run_mpsw(a, rank, world):
     fm, fk = ctypes.c_int(), ctypes.c_int()
     eng.h.check(L.mpsw_window_fused(eng.h.ptr, FP32, B, ctypes.byref(fm), ctypes.byref(fk)), 'window_fused')
     fused = fm.value > 0
-    # the kernels the sweeps launch: the two fused stage kernels, or the eight split ones
+    # the kernels the sweeps launch: the two fused stage kernels, or the split ones
     timed_k = ['tl_stage', 'ad_stage'] if fused else KERNELS
     kt = {}
     for name in timed_k:
@@ -587,7 +606,12 @@ def run_mpsw(a, rank, world):
         eng.h.check(L.mpsw_time_kernel(eng.h.ptr, KERNELS.index(name), FP32, B, 20, ctypes.byref(out)), 'time_kernel')
         kt[name] = out.value
 
+    # the row passes have no vertex kernel: its time is then 0
+    rows = {k: not fused and kt['tl_vertex' if k.startswith('tl') else 'ad_vertex'] == 0.0 for k in timed_k}
+
     def kbytes(k):
+        if rows[k]:
+            return row_bytes(k, nC, nE, nV, B)
         return fused_bytes(k, nC, nE, nV, B) if fused else kernel_bytes(k, nC, nE, nV, sum_eoe, B, 4)
     cand = ['tl_stage', 'ad_stage'] if fused else KERNELS[:8]
     top = max(cand, key=lambda k: kt[k])  # every candidate launches once per stage
@@ -598,9 +622,11 @@ def run_mpsw(a, rank, world):
                   'frac': kbytes(k) / (kt[k] / 1e3) / 1e9 / hbm,
                   'frac_of_M_plus_BS': s8d / (kt[k] / 1e3) / 1e9 / hbm}
               for k in ('tl_stage', 'ad_stage')}
-    roof = {'bound': 'hbm', 'kernel': ('k_tl_fused' if top == 'tl_stage' else 'k_ad_fused') if fused else top,
+    row_names = {'tl_edge_diag': 'row_tl_edge', 'tl_edge_tend': 'row_tl_tend'}
+    top_name = row_names.get(top, 'row_' + top) if rows[top] else top
+    roof = {'bound': 'hbm', 'kernel': ('k_tl_fused' if top == 'tl_stage' else 'k_ad_fused') if fused else top_name,
             'achieved': ach, 'peak': hbm, 'unit': 'GB/s', 'frac': ach / hbm, 'peak_source': peak_kind,
-            'traffic': traffic_of(('tl_fused' if top == 'tl_stage' else 'ad_fused') if fused else top, a.level, B),
+            'traffic': traffic_of(('tl_fused' if top == 'tl_stage' else 'ad_fused') if fused else top_name, a.level, B),
             'algorithmic_bytes': bytes_, 'ms_per_launch': kt[top], 'timing': 'each launch alone after a 256 MB L2 flush',
             'stage_bytes_M_plus_BS': s8d, 'kernel_ms': kt, 'stages': stages,
             'fused': {'members_per_block': fm.value, 'tile_cells': fk.value} if fused else None}
@@ -916,7 +942,10 @@ def run_costs(a, rank, world):
     out = ctypes.c_double()
     eng.h.check(L.mpsw_time_kernel(eng.h.ptr, 9, FP32, B, 10, ctypes.byref(out)), 'time_kernel')
     sum_eoe = int(unit['nEdgesOnEdge'].sum())
-    sb = kernel_bytes('ad_stage', nC, nE, nV, sum_eoe, B, 4)
+    vertex = ctypes.c_double()
+    eng.h.check(L.mpsw_time_kernel(eng.h.ptr, 6, FP32, B, 1, ctypes.byref(vertex)), 'time_kernel')
+    rows = vertex.value == 0.0  # the row passes have no vertex kernel
+    sb = row_bytes('ad_stage', nC, nE, nV, B) if rows else kernel_bytes('ad_stage', nC, nE, nV, sum_eoe, B, 4)
     ach = sb / (out.value / 1e3) / 1e9
     cpu = None
     if rank == 0:
@@ -936,7 +965,7 @@ def run_costs(a, rank, world):
             'sequential_fp64_gradients_per_s': seq,
             'batched_vs_sequential': value / world / seq,
             'rel_err_fp32_vs_fp64': rel_err,
-            'roofline': {'bound': 'hbm', 'kernel': 'one adjoint stage (ad_edge, ad_cell, ad_vertex, ad_final)',
+            'roofline': {'bound': 'hbm', 'kernel': 'one adjoint stage (%s)' % ('row_ad_edge, row_ad_cell, row_ad_final' if rows else 'ad_edge, ad_cell, ad_vertex, ad_final'),
                          'achieved': ach, 'peak': hbm, 'unit': 'GB/s', 'frac': ach / hbm, 'traffic': None,
                          'algorithmic_bytes': sb, 'ms_per_launch': out.value,
                          'peak_source': 'measured' if peaks.get('hbm_gbs') else 'fallback'},

@@ -133,7 +133,9 @@ int mpsw_window_storage(mpsw_handle *h, int mode, double max_bytes);
  * reference.  The first sweep of a window for a given (precision, B) times each kernel over the
  * pairs B allows on the window's own buffers and keeps the fastest (MPSW_TUNE=0 in the
  * environment keeps fixed defaults; MPSW_TUNE_CACHE=<file> keeps the choices in a text file
- * keyed by device, mesh size, precision and B, and reuses them). */
+ * keyed by device, mesh size, precision and B, and reuses them).  Kernels that the sweeps of this
+ * (precision, B) do not run stay at zero: tl_vertex and ad_vertex where FP32 members take the three
+ * row passes, all four of a sweep where few FP64 members take one kernel a stage. */
 int mpsw_window_tuning(mpsw_handle *h, int precision, int B, int *v_block);
 /* Checkpointing of the following mpsw_window_init calls, for windows whose stages are not
  * stored.  snapshots 0 (default): two-level checkpointing, a checkpoint every ckpt_every steps
@@ -213,7 +215,9 @@ long long mpsw_launch_count(void);
  * window sweep (same precision and B): which = 0 tl_vertex, 1 tl_cell, 2 tl_edge_diag,
  * 3 tl_edge_tend, 4 ad_edge, 5 ad_cell, 6 ad_vertex, 7 ad_final; or of a whole stage:
  * 8 tangent-linear stage, 9 adjoint stage.  Each launch is timed alone with CUDA events on the
- * engine's stream, after a 256 MiB write that evicts L2 (a cold start, as in a sweep). */
+ * engine's stream, after a 256 MiB write that evicts L2 (a cold start, as in a sweep).  Where FP32
+ * members take the row passes, 1-3 and 4, 5, 7 are those passes and 0, 6, which they do without,
+ * return 0. */
 int mpsw_time_kernel(mpsw_handle *h, int which, int precision, int B, int iters, double *ms_per_launch);
 
 #ifdef __cplusplus

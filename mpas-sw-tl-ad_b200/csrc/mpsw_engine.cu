@@ -593,7 +593,7 @@ void Engine::build_row_tables() {
   rows.c_m = F(h.c_m); rows.c_t = F(h.c_t); rows.c_q = F(h.c_q); rows.c_r = F(h.c_r); rows.c_ka = F(h.c_ka);
   rows.c_kb = F(h.c_kb); rows.c_kk = F(h.c_kk); rows.c_r2 = F(h.c_r2); rows.c_r3 = F(h.c_r3); rows.c_ra = F(h.c_ra);
   rows.e_d = F(h.e_d); rows.e_r4 = F(h.e_r4); rows.e_k = F(h.e_k); rows.e_i1 = F(h.e_i1); rows.e_i2 = F(h.e_i2);
-  rows.e_ke = F(h.e_ke); rows.e_lap = F(h.e_lap); rows.e_lapT = F(h.e_lapT); rows.e_lap0 = F(h.e_lap0);
+  rows.e_ke = F(h.e_ke); rows.e_lap = F(h.e_lap); rows.e_lap0 = F(h.e_lap0);
   rows.ok = true;
 }
 

@@ -94,7 +94,7 @@ std::string build_rows(const BuiltMesh &m, RowTabHost *t) {
   t->e_kr.assign((size_t)6 * nE, 0.0);
   t->e_t.assign((size_t)4 * nE, 0);
   for (auto *x : {&t->e_i1, &t->e_i2, &t->e_lap0}) x->assign(nE, 0.0);
-  for (auto *x : {&t->e_ke, &t->e_lap, &t->e_lapT}) x->assign((size_t)10 * nE, 0.0);
+  for (auto *x : {&t->e_ke, &t->e_lap}) x->assign((size_t)10 * nE, 0.0);
   for (int e = 0; e < nE; e++) {
     const int c1 = m.e_c1[e], c2 = m.e_c2[e];
     const double dc = m.e_dc[e], dv = m.e_dv[e];
@@ -113,15 +113,12 @@ std::string build_rows(const BuiltMesh &m, RowTabHost *t) {
       double lap = to * sign_c(c, x) * m.e_dv[x] / m.c_area[c] / dc;
       // the edge's weight in delsq_u of x: the cell's side there, and its divergence weight
       const double to_x = m.e_c2[x] == c ? 1.0 : -1.0;
-      double lapT = to_x * sign_c(c, e) * dv / m.c_area[c] / m.e_dc[x];
       for (int k = 0; k < 2; k++) {
         const int v = k ? m.e_v2[e] : m.e_v1[e];
         if (!of_vertex(v, x)) continue;
         lap -= (k ? 1.0 : -1.0) * sign_v(v, x) * m.e_dc[x] / m.v_area[v] / dv;
-        lapT -= (m.e_v2[x] == v ? 1.0 : -1.0) * sign_v(v, e) * dc / m.v_area[v] / m.e_dv[x];
       }
       t->e_lap[E(e, j)] = lap;
-      t->e_lapT[E(e, j)] = lapT;
     }
     unsigned q = 0;
     for (int k = 0; k < 2; k++) {

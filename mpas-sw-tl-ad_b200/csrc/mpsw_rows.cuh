@@ -21,7 +21,7 @@ namespace mpsw {
 
 // Words of a block's staged coefficients per entity.
 constexpr int kRowTlCellW = 6 * 12, kRowTlEdgeW = 10 * 2 + 18, kRowTlTendW = 10 * 3, kRowAdEdgeW = 10 * 5,
-              kRowAdCellW = 6 * 8, kRowAdFinalW = 10 * 2 + 14, kRowAdLastW = 6 * 4;
+              kRowAdCellW = 6 * 8, kRowAdFinalW = 10 * 2 + 14;
 
 __device__ __forceinline__ float4 *row_smem() {
   extern __shared__ __align__(16) float4 row_smem_raw[];

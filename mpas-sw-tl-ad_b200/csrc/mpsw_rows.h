@@ -41,7 +41,6 @@ struct RowTab {
   const float *e_i1, *e_i2;  // 1 / areaT(v1), 1 / areaT(v2)
   const float *e_ke;         // [10][nE] sign(c,j) / (dc(j) area(c)), c the cell that edge j shares
   const float *e_lap;        // [10][nE] weight of edge j in delsq_u of the edge, e_lap0 its own
-  const float *e_lapT;       // [10][nE] weight of the edge in delsq_u of edge j
   const float *e_lap0;
 };
 
@@ -49,7 +48,7 @@ struct RowTab {
 struct RowTabHost {
   std::vector<int> c_nb, c_sp, c_va, c_vb, e_q, e_o1, e_o2, e_t;
   std::vector<double> c_g1, c_g2, c_g3, c_n1, c_n2, c_m, c_t, c_q, c_r, c_ka, c_kb, c_kk, c_r2, c_r3, c_ra;
-  std::vector<double> e_d, e_r4, e_k, e_kr, e_i1, e_i2, e_ke, e_lap, e_lapT, e_lap0;
+  std::vector<double> e_d, e_r4, e_k, e_kr, e_i1, e_i2, e_ke, e_lap, e_lap0;
 };
 
 // Empty string, or what the mesh lacks (a vertex whose edges or cells are not those around it, an

@@ -230,15 +230,6 @@ extern "C" int row_check(const int *ints, const int *const *conn, const double *
   }
   out[2] = worst(qu, uad);
   out[3] = worst(qh2, had);
-  // delsq_u transposed: <lap u, T> = <u, lapT T>
-  double l = 0, rr = 0;
-  for (int x = 0; x < nE; x++) {
-    double s = t.e_lap0[x] * T[x];
-    for (int j = 0; j < m.e_n[x]; j++) s += t.e_lapT[E(x, j)] * T[m.e_eoe[E(x, j)]];
-    l += lap[x] * T[x];
-    rr += u[x] * s;
-  }
-  out[5] = std::fabs(l - rr) / std::fabs(l);
   // the adjoint against the tangent linear: <tu, T> + <th area, H> = <u, u_ad> + <h, h_ad>
   double a1 = 0, a2 = 0;
   for (int x = 0; x < nE; x++) {
