@@ -1224,17 +1224,17 @@ void Engine::rk4_adj() {  // src/mpas_sw_module.f90:783-1002
   double *u0 = dv("u"), *h0 = dv("h"), *u2 = dv("u", 1), *h2 = dv("h", 1);
   // forward sweep, keeping the diagnostics of every stage (:815-878)
   run_graph(graph_key(11, 0, 1, u0, h0), [&]() {
-  for (int k = 0; k < 4; k++) {
-    const double *ui = k == 0 ? u0 : sp_u[k - 1];
-    const double *hi = k == 0 ? h0 : sp_h[k - 1];
-    RK<double, double> ru{u0, k == 0 ? u0 : acc_u, acc_u, k < 3 ? sp_u[k] : nullptr, c[k], w[k], 0.0, ph.tc1};
-    RK<double, double> rh{h0, k == 0 ? h0 : acc_h, acc_h, k < 3 ? sp_h[k] : nullptr, c[k], w[k], 0.0, 0};
-    fwd_stage(ui, hi, stage[k + 1], ph, ru, rh, nullptr, nullptr, base_out(stage[k + 1]));
-  }
-  cuda_check(cudaMemcpyAsync(u2, ph.tc1 ? u0 : acc_u, sizeof(double) * nE, cudaMemcpyDeviceToDevice, stream), "u(2)");
-  cuda_check(cudaMemcpyAsync(h2, acc_h, sizeof(double) * nC, cudaMemcpyDeviceToDevice, stream), "h(2)");
-  L64::recon(m64, 1, ph.sphere, u0, dv("uReconstructX"), dv("uReconstructY"), dv("uReconstructZ"),
-             dv("uReconstructZonal"), dv("uReconstructMeridional"), stream);
+    for (int k = 0; k < 4; k++) {
+      const double *ui = k == 0 ? u0 : sp_u[k - 1];
+      const double *hi = k == 0 ? h0 : sp_h[k - 1];
+      RK<double, double> ru{u0, k == 0 ? u0 : acc_u, acc_u, k < 3 ? sp_u[k] : nullptr, c[k], w[k], 0.0, ph.tc1};
+      RK<double, double> rh{h0, k == 0 ? h0 : acc_h, acc_h, k < 3 ? sp_h[k] : nullptr, c[k], w[k], 0.0, 0};
+      fwd_stage(ui, hi, stage[k + 1], ph, ru, rh, nullptr, nullptr, base_out(stage[k + 1]));
+    }
+    cuda_check(cudaMemcpyAsync(u2, ph.tc1 ? u0 : acc_u, sizeof(double) * nE, cudaMemcpyDeviceToDevice, stream), "u(2)");
+    cuda_check(cudaMemcpyAsync(h2, acc_h, sizeof(double) * nC, cudaMemcpyDeviceToDevice, stream), "h(2)");
+    L64::recon(m64, 1, ph.sphere, u0, dv("uReconstructX"), dv("uReconstructY"), dv("uReconstructZ"),
+               dv("uReconstructZonal"), dv("uReconstructMeridional"), stream);
   });
   double *ua = dv("u_ad"), *ha = dv("h_ad");
   // adjoint of the output reconstruction and diagnostics at x(2) (:887-905)
@@ -1258,29 +1258,29 @@ void Engine::rk4_adj() {  // src/mpas_sw_module.f90:783-1002
   GraphKey key = graph_key(12, 0, 1, ua, ha);
   key.n2 = (stu ? 1 : 0) | (sth ? 2 : 0);
   run_graph(key, [&]() {
-  L64::ad_tinit(m64, 1, ua, ha, ph.tc1 ? nullptr : stu, sth, ph.tc1 ? 0.0 : w[3], w[3], tu_[0], th_[0], stream);
-  AdSeeds<double> none{};
-  for (int k = 3; k >= 0; k--) {  // :912-970
-    const double *ui = k == 0 ? u0 : sp_u[k - 1];
-    AdIn<double> in{tu_[(3 - k) & 1], th_[(3 - k) & 1]};
-    AdOut<double, double> out{};
-    out.acc_u = xacc_u; out.acc_h = xacc_h;
-    out.x2u = ua; out.x2h = ha; out.dst_u = ua; out.dst_h = ha;
-    out.mode = k == 3 ? AD_SET : k == 0 ? AD_FINAL : AD_ADD;
-    if (k > 0) {
-      out.tu_next = tu_[(4 - k) & 1];
-      out.th_next = th_[(4 - k) & 1];
-      out.wu = ph.tc1 ? 0.0 : w[k - 1];
-      out.cu = ph.tc1 ? 0.0 : c[k - 1];
-      out.wh = w[k - 1];
-      out.ch = c[k - 1];
+    L64::ad_tinit(m64, 1, ua, ha, ph.tc1 ? nullptr : stu, sth, ph.tc1 ? 0.0 : w[3], w[3], tu_[0], th_[0], stream);
+    AdSeeds<double> none{};
+    for (int k = 3; k >= 0; k--) {  // :912-970
+      const double *ui = k == 0 ? u0 : sp_u[k - 1];
+      AdIn<double> in{tu_[(3 - k) & 1], th_[(3 - k) & 1]};
+      AdOut<double, double> out{};
+      out.acc_u = xacc_u; out.acc_h = xacc_h;
+      out.x2u = ua; out.x2h = ha; out.dst_u = ua; out.dst_h = ha;
+      out.mode = k == 3 ? AD_SET : k == 0 ? AD_FINAL : AD_ADD;
+      if (k > 0) {
+        out.tu_next = tu_[(4 - k) & 1];
+        out.th_next = th_[(4 - k) & 1];
+        out.wu = ph.tc1 ? 0.0 : w[k - 1];
+        out.cu = ph.tc1 ? 0.0 : c[k - 1];
+        out.wh = w[k - 1];
+        out.ch = c[k - 1];
+      }
+      const Base<double> bs = base_of(stage[k + 1], ui);
+      if (stage_ad_tiled(1, ph)) L64::stage_ad(st_ad, StageAdArgs{in, 1, bs, ph, out, m64.e_usrc}, stream);
+      else L64::ad_stage(m64, 1, bs, ph, in, none, adw, out, stream);
     }
-    const Base<double> bs = base_of(stage[k + 1], ui);
-    if (stage_ad_tiled(1, ph)) L64::stage_ad(st_ad, StageAdArgs{in, 1, bs, ph, out, m64.e_usrc}, stream);
-    else L64::ad_stage(m64, 1, bs, ph, in, none, adw, out, stream);
-  }
-  cuda_check(cudaMemsetAsync(dv("u_ad", 1), 0, sizeof(double) * nE, stream), "memset");
-  cuda_check(cudaMemsetAsync(dv("h_ad", 1), 0, sizeof(double) * nC, stream), "memset");
+    cuda_check(cudaMemsetAsync(dv("u_ad", 1), 0, sizeof(double) * nE, stream), "memset");
+    cuda_check(cudaMemsetAsync(dv("h_ad", 1), 0, sizeof(double) * nC, stream), "memset");
   });
   zero_ad_seeds();
   cuda_check(cudaGetLastError(), "sw_rk4_adj");

@@ -126,69 +126,69 @@ __global__ void __maxnreg__(VISC ? 72 : 48) k_row_tl_edge(MeshDev<float> m, RowT
   int tile, last;
   th.run(nE, blockIdx.x, gridDim.x, &tile, &last);
   for (; tile < last; tile++) {
-  const int e0 = tile * th.epb;
-  // ten slots, the edge's own terms, the four slots that end at one of its vertices
-  for (int i = threadIdx.x; i < 15 * th.epb; i += blockDim.x) {
-    const int j = i / th.epb, le = i - j * th.epb, e = e0 + le;
-    if (j < 10) {
-      int nb = 0;
-      float p = 0.f;
-      if (e < nE && j < m.e_n[e]) {
-        nb = m.e_eoe[(size_t)j * nE + e];
-        p = row_tl_edge_slot(m.e_w[(size_t)j * nE + e], apt * bs.gpt[e]);
-      }
-      slot[le * 10 + j] = make_float2(as_f(nb), p);
-    } else if (e < nE) {
-      const RowTlEdge<float> r = row_tl_edge<float>(t, m, bs, apt, e);
-      if (j == 10) {
-        own[3 * le] = make_float4(as_f(m.e_c1[e]), as_f(m.e_c2[e]), as_f(t.e_o1[e]), as_f(t.e_o2[e]));
-        own[3 * le + 1] = make_float4(r.p0, r.h1, r.h2, r.o1);
-        own[3 * le + 2] = make_float4(r.o2, r.pc, r.he, r.uh);
-        eq[le] = t.e_q[e];
-      } else {
-        tag[(j - 11) * th.epb + le] = row_tl_edge_tag(t, nE, e, j - 11, r);
+    const int e0 = tile * th.epb;
+    // ten slots, the edge's own terms, the four slots that end at one of its vertices
+    for (int i = threadIdx.x; i < 15 * th.epb; i += blockDim.x) {
+      const int j = i / th.epb, le = i - j * th.epb, e = e0 + le;
+      if (j < 10) {
+        int nb = 0;
+        float p = 0.f;
+        if (e < nE && j < m.e_n[e]) {
+          nb = m.e_eoe[(size_t)j * nE + e];
+          p = row_tl_edge_slot(m.e_w[(size_t)j * nE + e], apt * bs.gpt[e]);
+        }
+        slot[le * 10 + j] = make_float2(as_f(nb), p);
+      } else if (e < nE) {
+        const RowTlEdge<float> r = row_tl_edge<float>(t, m, bs, apt, e);
+        if (j == 10) {
+          own[3 * le] = make_float4(as_f(m.e_c1[e]), as_f(m.e_c2[e]), as_f(t.e_o1[e]), as_f(t.e_o2[e]));
+          own[3 * le + 1] = make_float4(r.p0, r.h1, r.h2, r.o1);
+          own[3 * le + 2] = make_float4(r.o2, r.pc, r.he, r.uh);
+          eq[le] = t.e_q[e];
+        } else {
+          tag[(j - 11) * th.epb + le] = row_tl_edge_tag(t, nE, e, j - 11, r);
+        }
       }
     }
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < 4 * th.epb; i += blockDim.x) {
-    const int j = i / th.epb, le = i - j * th.epb, e = e0 + le;
-    if (e < nE) slot[le * 10 + (((unsigned)eq[le] >> (8 * j)) & 0xFF)].y += tag[i];
-  }
-  __syncthreads();
-  if (early) {
-    pdl_begin();
-    early = 0;
-  }
-  const int e = e0 + th.le;
-  if (e < nE) {
-  const size_t o = (size_t)e * B + b;
-  const M u = ldv<V>(ut + o);
-  const float4 x = own[3 * th.le], y = own[3 * th.le + 1], z = own[3 * th.le + 2];
-  const M h1 = ldv<V>(ht + (size_t)as_i(x.x) * B + b), h2 = ldv<V>(ht + (size_t)as_i(x.y) * B + b);
-  M p = y.x * u, f = z.z * u;
-  row_add(p, y.y, h1);
-  row_add(p, y.z, h2);
-  row_add(f, z.w, h1);
-  row_add(f, z.w, h2);
-  row_add(p, y.w, ldv<V>(ht + (size_t)as_i(x.z) * B + b));
-  row_add(p, z.x, ldv<V>(ht + (size_t)as_i(x.w) * B + b));
-  row_add(p, -z.y, ldv<V>(pc + (size_t)as_i(x.x) * B + b));
-  row_add(p, z.y, ldv<V>(pc + (size_t)as_i(x.y) * B + b));
-  M d = mv_fill<float, V>(0.f);
-  if (VISC) d = t.e_lap0[e] * u;
+    __syncthreads();
+    for (int i = threadIdx.x; i < 4 * th.epb; i += blockDim.x) {
+      const int j = i / th.epb, le = i - j * th.epb, e = e0 + le;
+      if (e < nE) slot[le * 10 + (((unsigned)eq[le] >> (8 * j)) & 0xFF)].y += tag[i];
+    }
+    __syncthreads();
+    if (early) {
+      pdl_begin();
+      early = 0;
+    }
+    const int e = e0 + th.le;
+    if (e < nE) {
+    const size_t o = (size_t)e * B + b;
+    const M u = ldv<V>(ut + o);
+    const float4 x = own[3 * th.le], y = own[3 * th.le + 1], z = own[3 * th.le + 2];
+    const M h1 = ldv<V>(ht + (size_t)as_i(x.x) * B + b), h2 = ldv<V>(ht + (size_t)as_i(x.y) * B + b);
+    M p = y.x * u, f = z.z * u;
+    row_add(p, y.y, h1);
+    row_add(p, y.z, h2);
+    row_add(f, z.w, h1);
+    row_add(f, z.w, h2);
+    row_add(p, y.w, ldv<V>(ht + (size_t)as_i(x.z) * B + b));
+    row_add(p, z.x, ldv<V>(ht + (size_t)as_i(x.w) * B + b));
+    row_add(p, -z.y, ldv<V>(pc + (size_t)as_i(x.x) * B + b));
+    row_add(p, z.y, ldv<V>(pc + (size_t)as_i(x.y) * B + b));
+    M d = mv_fill<float, V>(0.f);
+    if (VISC) d = t.e_lap0[e] * u;
 #pragma unroll
-  for (int j = 0; j < 10; j++) {
-    const float2 c = slot[th.le * 10 + j];
-    const M un = ldv<V>(ut + (size_t)as_i(c.x) * B + b);
-    row_add(p, c.y, un);
-    if (VISC) row_add(d, t.e_lap[(size_t)j * nE + e], un);
-  }
-  stv<V>(pe + o, p);
-  stv<V>(flux + o, f);
-  if (VISC) stv<V>(dsq + o, d);
-  }
-  __syncthreads();
+    for (int j = 0; j < 10; j++) {
+      const float2 c = slot[th.le * 10 + j];
+      const M un = ldv<V>(ut + (size_t)as_i(c.x) * B + b);
+      row_add(p, c.y, un);
+      if (VISC) row_add(d, t.e_lap[(size_t)j * nE + e], un);
+    }
+    stv<V>(pe + o, p);
+    stv<V>(flux + o, f);
+    if (VISC) stv<V>(dsq + o, d);
+    }
+    __syncthreads();
   }
 }
 
@@ -209,77 +209,77 @@ __global__ void __maxnreg__(GEN ? 72 : 48) k_row_tl_tend(MeshDev<float> m, int B
   int tile, last;
   th.run(nE, blockIdx.x, gridDim.x, &tile, &last);
   for (; tile < last; tile++) {
-  const int e0 = tile * th.epb;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    const int j = i / th.epb, le = i - j * th.epb, e = e0 + le;
-    int nb = 0;
-    RowTlTend<float> r{0.f, 0.f};
-    if (e < nE && j < m.e_n[e]) {
-      nb = m.e_eoe[(size_t)j * nE + e];
-      r = row_tl_tend<float>(bs, nb, m.e_w[(size_t)j * nE + e], bs.pe[e]);
-    }
-    nbs[i] = nb;
-    co[i] = make_float2(r.f, r.p);
-  }
-  __syncthreads();
-  if (early) {
-    pdl_begin();
-    early = 0;
-  }
-  const int e = e0 + th.le;
-  if (e < nE) {
-  const size_t o = (size_t)e * B + b;
-  const int c1 = m.e_c1[e], c2 = m.e_c2[e];
-  const float rdc = 1.f / m.e_dc[e];
-  M q = mv_fill<float, V>(0.f);
-  row_add(q, rdc, ldv<V>(d.ke + (size_t)c1 * B + b));
-  row_add(q, -rdc, ldv<V>(d.ke + (size_t)c2 * B + b));
-  float own = 0.f;
-#pragma unroll
-  for (int j = 0; j < 10; j++) {
-    const int i = j * th.epb + th.le;
-    const size_t on = (size_t)nbs[i] * B + b;
-    const float2 c = co[i];
-    row_add(q, c.x, ldv<V>(flux + on));
-    row_add(q, c.y, ldv<V>(d.pe + on));
-    own += c.y;
-  }
-  row_add(q, own, ldv<V>(d.pe + o));
-  if (GEN) {
-    if (ph.visc2 > 0.f) row_add(q, m.e_sc2[e] * ph.visc2, ldv<V>(d.dsq_u + o));
-    if (ph.visc4 > 0.f) {
-      const int v1 = m.e_v1[e], v2 = m.e_v2[e];
-      const float k = m.e_sc4[e] * ph.visc4, kv = k / m.e_dv[e], kc = k * rdc;
-      row_add(q, kc, ldv<V>(d.dsq_div + (size_t)c1 * B + b));
-      row_add(q, -kc, ldv<V>(d.dsq_div + (size_t)c2 * B + b));
-      row_add(q, -kv, ldv<V>(d.dsq_vort + (size_t)v1 * B + b));
-      row_add(q, kv, ldv<V>(d.dsq_vort + (size_t)v2 * B + b));
-    }
-    if (ph.wind || ph.drag) {
-      const float hh = bs.he[e];
-      const M h1 = ldv<V>(ht + (size_t)c1 * B + b), h2 = ldv<V>(ht + (size_t)c2 * B + b);
-      float k = ph.wind ? -(m.e_usrc[e] / float(RHO_REF)) / (hh * hh) : 0.f;
-      if (ph.drag) {  // d.ke holds ke' alone: the gravity term is added here
-        const float uu = bs.u[e], sq = sqrtf(bs.ke[c1] + bs.ke[c2]), g = float(GRAVITY) * rdc;
-        k += ((1.0e-3f * uu) * sq) / (hh * hh);
-        row_add(q, -(1.0e-3f * sq) / hh, ldv<V>(ut + o));
-        const float kk = -(((0.5f * 1.0e-3f) * uu) / sq) / hh;
-        row_add(q, kk, ldv<V>(d.ke + (size_t)c1 * B + b));
-        row_add(q, kk, ldv<V>(d.ke + (size_t)c2 * B + b));
-        row_add(q, g, h1);
-        row_add(q, -g, h2);
+    const int e0 = tile * th.epb;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+      const int j = i / th.epb, le = i - j * th.epb, e = e0 + le;
+      int nb = 0;
+      RowTlTend<float> r{0.f, 0.f};
+      if (e < nE && j < m.e_n[e]) {
+        nb = m.e_eoe[(size_t)j * nE + e];
+        r = row_tl_tend<float>(bs, nb, m.e_w[(size_t)j * nE + e], bs.pe[e]);
       }
-      row_add(q, 0.5f * k, h1);
-      row_add(q, 0.5f * k, h2);
+      nbs[i] = nb;
+      co[i] = make_float2(r.f, r.p);
     }
-  }
-  if (ph.bad) {
+    __syncthreads();
+    if (early) {
+      pdl_begin();
+      early = 0;
+    }
+    const int e = e0 + th.le;
+    if (e < nE) {
+    const size_t o = (size_t)e * B + b;
+    const int c1 = m.e_c1[e], c2 = m.e_c2[e];
+    const float rdc = 1.f / m.e_dc[e];
+    M q = mv_fill<float, V>(0.f);
+    row_add(q, rdc, ldv<V>(d.ke + (size_t)c1 * B + b));
+    row_add(q, -rdc, ldv<V>(d.ke + (size_t)c2 * B + b));
+    float own = 0.f;
 #pragma unroll
-    for (int i = 0; i < V; i++) flag_nonfinite(ph.bad, q.x[i]);
-  }
-  rk_members<float, double, V>(rk, o, q);
-  }
-  __syncthreads();
+    for (int j = 0; j < 10; j++) {
+      const int i = j * th.epb + th.le;
+      const size_t on = (size_t)nbs[i] * B + b;
+      const float2 c = co[i];
+      row_add(q, c.x, ldv<V>(flux + on));
+      row_add(q, c.y, ldv<V>(d.pe + on));
+      own += c.y;
+    }
+    row_add(q, own, ldv<V>(d.pe + o));
+    if (GEN) {
+      if (ph.visc2 > 0.f) row_add(q, m.e_sc2[e] * ph.visc2, ldv<V>(d.dsq_u + o));
+      if (ph.visc4 > 0.f) {
+        const int v1 = m.e_v1[e], v2 = m.e_v2[e];
+        const float k = m.e_sc4[e] * ph.visc4, kv = k / m.e_dv[e], kc = k * rdc;
+        row_add(q, kc, ldv<V>(d.dsq_div + (size_t)c1 * B + b));
+        row_add(q, -kc, ldv<V>(d.dsq_div + (size_t)c2 * B + b));
+        row_add(q, -kv, ldv<V>(d.dsq_vort + (size_t)v1 * B + b));
+        row_add(q, kv, ldv<V>(d.dsq_vort + (size_t)v2 * B + b));
+      }
+      if (ph.wind || ph.drag) {
+        const float hh = bs.he[e];
+        const M h1 = ldv<V>(ht + (size_t)c1 * B + b), h2 = ldv<V>(ht + (size_t)c2 * B + b);
+        float k = ph.wind ? -(m.e_usrc[e] / float(RHO_REF)) / (hh * hh) : 0.f;
+        if (ph.drag) {  // d.ke holds ke' alone: the gravity term is added here
+          const float uu = bs.u[e], sq = sqrtf(bs.ke[c1] + bs.ke[c2]), g = float(GRAVITY) * rdc;
+          k += ((1.0e-3f * uu) * sq) / (hh * hh);
+          row_add(q, -(1.0e-3f * sq) / hh, ldv<V>(ut + o));
+          const float kk = -(((0.5f * 1.0e-3f) * uu) / sq) / hh;
+          row_add(q, kk, ldv<V>(d.ke + (size_t)c1 * B + b));
+          row_add(q, kk, ldv<V>(d.ke + (size_t)c2 * B + b));
+          row_add(q, g, h1);
+          row_add(q, -g, h2);
+        }
+        row_add(q, 0.5f * k, h1);
+        row_add(q, 0.5f * k, h2);
+      }
+    }
+    if (ph.bad) {
+#pragma unroll
+      for (int i = 0; i < V; i++) flag_nonfinite(ph.bad, q.x[i]);
+    }
+    rk_members<float, double, V>(rk, o, q);
+    }
+    __syncthreads();
   }
 }
 
