@@ -61,9 +61,12 @@ int mpsw_var_info(mpsw_handle *h, const char *name, int *rank, long long dims[4]
                   int *allocated);
 int mpsw_set_var(mpsw_handle *h, const char *name, const void *src, long long count);
 int mpsw_get_var(mpsw_handle *h, const char *name, void *dst, long long count);
-/* mpsw_set_var unless src equals what was last exchanged for this variable (the caller's copy is
- * unchanged); mpsw_get_var of n variables with one wait. */
+/* mpsw_set_var, skipped where the variable already holds src: src equals what was last exchanged for
+ * it, and no routine has written it since.  mpsw_var_changed: whether src differs from what was last
+ * exchanged, whatever routines have written since (has the caller edited its copy?).  mpsw_get_vars:
+ * mpsw_get_var of n variables with one wait. */
 int mpsw_update_var(mpsw_handle *h, const char *name, const void *src, long long count);
+int mpsw_var_changed(mpsw_handle *h, const char *name, const void *src, long long count, int *changed);
 int mpsw_get_vars(mpsw_handle *h, int n, const char *const *names, void *const *dst, const long long *counts);
 
 /* ---- module subroutines (src/mpas_sw_module.f90) -------------------------------------- */

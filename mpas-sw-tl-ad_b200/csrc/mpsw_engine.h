@@ -188,6 +188,7 @@ struct Engine {
   double *d_mean = nullptr;
   void download_start(Var &v);
   void set_var(const char *name, const void *src, long long count, bool if_changed = false);
+  bool var_changed(const char *name, const void *src, long long count);
   void get_vars(int n, const char *const *names, void *const *dst, const long long *counts);
   void get_var(const char *name, void *dst, long long count);
   void mark_written(Var &v, bool maybe_nonzero);

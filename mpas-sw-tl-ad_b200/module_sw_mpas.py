@@ -78,6 +78,7 @@ class MpasSwModule:
         d['_canon'] = {n.lower(): n for n in names}
         d['_arr'] = {}         # lower name -> ndarray (Fortran order)
         d['_synced'] = set()   # lower names of allocated arrays sent only when their content changed
+        d['_assigned'] = set()  # lower names assigned since they were last sent
         d['_stale'] = set()    # lower names to refresh from the engine on next access
         d['_mesh_dirty'] = set()
 
@@ -107,7 +108,9 @@ class MpasSwModule:
                 raise ValueError(f'{name}: shape {val.shape} does not match the allocated {arr.shape}')
             arr[...] = val.reshape(arr.shape, order='F') if val.shape != arr.shape else val
             d['_stale'].discard(key)
-            if key not in d['_synced']:
+            if key in d['_synced']:
+                d['_assigned'].add(key)
+            else:
                 d['_mesh_dirty'].add(key)
             return
         if isinstance(value, (bool, np.bool_)):
@@ -122,9 +125,20 @@ class MpasSwModule:
     def _push(self, key, force=False):
         d = self.__dict__
         arr = d['_arr'][key]
-        # the engine keeps what was last exchanged and compares with it
-        routine = 'mpsw_update_var' if key in d['_synced'] and not force else 'mpsw_set_var'
-        d['_h'].call(routine, d['_canon'][key].encode(), ctypes.c_void_p(arr.ctypes.data), arr.size)
+        args = d['_canon'][key].encode(), ctypes.c_void_p(arr.ctypes.data), arr.size
+        if force or key not in d['_synced']:
+            d['_h'].call('mpsw_set_var', *args)
+        elif key in d['_assigned']:
+            # set since the last routine: the engine's value, if a routine has written it, gives way
+            d['_h'].call('mpsw_update_var', *args)
+        else:
+            # sent only where edited in place since the last exchange, so that a value written through
+            # the handle stands
+            changed = ctypes.c_int()
+            d['_h'].call('mpsw_var_changed', *args, ctypes.byref(changed))
+            if changed.value:
+                d['_h'].call('mpsw_set_var', *args)
+        d['_assigned'].discard(key)
 
     def _pull(self, *keys):
         d = self.__dict__
@@ -134,6 +148,7 @@ class MpasSwModule:
                      (ctypes.c_void_p * n)(*[a.ctypes.data for a in arrs]),
                      (ctypes.c_longlong * n)(*[a.size for a in arrs]))
         d['_stale'].difference_update(keys)
+        d['_assigned'].difference_update(keys)
 
     def _push_mesh(self, everything=False):
         d = self.__dict__
@@ -180,6 +195,7 @@ class MpasSwModule:
             shape = tuple(dims[i] for i in range(rank.value))
             d['_arr'][lname] = np.zeros(shape, dtype=np.int32 if is_int.value else np.float64, order='F')
             d['_stale'].discard(lname)
+            d['_assigned'].discard(lname)
             if lname in _TRACKED:
                 d['_synced'].add(lname)
             else:
