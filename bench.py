@@ -384,7 +384,7 @@ def row_bytes(name, nC, nE, nV, B, s=4):
     kb = {
         'tl_cell': 4 * 72 * C + s * (2 * E + 2 * V) + B * s * (E + C + 2 * C + 3 * C),   # u,h in; pc,ke out; RK
         'tl_edge_diag': 4 * 38 * E + 6 * s * E + B * s * (E + 2 * C + 2 * E),            # u,h,pc in; pv_edge, flux out
-        'tl_edge_tend': 4 * 30 * E + 3 * s * E + B * s * (2 * E + C + 3 * E),            # flux,pv_edge,ke in; RK
+        'tl_edge_tend': 4 * 30 * E + 3 * s * E + B * s * (2 * E + 2 * C + 3 * E),        # flux,pv_edge,ke,h in; RK
         'ad_edge': 4 * 50 * E + 6 * s * E + B * s * (E + C + 3 * E),
         'ad_cell': 4 * 48 * C + s * (2 * E + 2 * V) + B * s * (3 * E + 2 * C),
         'ad_final': 4 * 34 * E + 4 * 24 * C + s * (2 * E + 2 * V) + B * s * (2 * E + 2 * C + 3 * (E + C)),

@@ -563,7 +563,7 @@ void Launch<R, A>::row_tl(int part, const MeshDev<R> &m, const RowTab &t, int B,
     if (part == 0) {
       const int v = row_width(K_TL_CELL, B);
       const LaunchCfg c = row_cfg(K_TL_CELL, m.nC, B, v, kRowTlCellW, 1);
-      MPSW_ROWV(v, launch_k(k_row_tl_cell<VV>, c, s, m, t, B, bs, ut, ht, d.pc, d.ke, (int)ph.drag, rkh, early));
+      MPSW_ROWV(v, launch_k(k_row_tl_cell<VV>, c, s, m, t, B, bs, ut, ht, d.pc, d.ke, rkh, early));
     } else if (part == 1) {
       const int v = row_width(K_TL_EDGE_DIAG, B);
       const LaunchCfg c = row_cfg(K_TL_EDGE_DIAG, m.nE, B, v, kRowTlEdgeW, 2);

@@ -4,14 +4,14 @@
 //
 // A stage is bound by the member rows it moves: through the intermediate fields (mpsw_members.cuh) a
 // level-7 stage of 64 members moves 2.2 GB of rows, 53 rows a cell tangent linear and 57 adjoint;
-// folding pv_vertex, the PV flux, ke and the vertex adjoints into coefficients leaves 36 and 44, and
+// folding pv_vertex, the PV flux and the vertex adjoints into coefficients leaves 37 and 44, and
 // three kernels instead of four.  Coefficients are formed once a block in shared memory, before the
 // wait for the previous kernel where the linearisation point is a stored one, and shared by the
 // B / V threads of an entity; a thread holds V members.  The edge passes give a block two
 // neighbouring tiles of edges (the second finds rows of the first in L1: tendency pass 236 -> 214 us),
 // and each kernel is held to the registers at which occupancy and the rows a thread keeps in flight
-// balance.  Level 7, 64 members, cold, us: cells 103, edges 212, tendencies 214 (a tangent-linear stage
-// 529, through the fields 634); edges 186, cells 104, final 249 (adjoint 538, through the fields 671).
+// balance.  Level 7, 64 members, cold, us: cells 107, edges 212, tendencies 227 (a tangent-linear stage
+// 529, through the fields 634); edges 189, cells 109, final 249 (adjoint 526, through the fields 671).
 #pragma once
 
 #include "mpsw_members.cuh"
@@ -56,11 +56,11 @@ struct RowThread {
 
 // ---- tangent linear ------------------------------------------------------------------------------
 
-// pv_cell', ke' + g h' (ke' alone with bottom drag, whose term needs it), tend_h' and its RK update
+// pv_cell', ke', tend_h' and its RK update
 template <int V>
 __global__ void __maxnreg__(72) k_row_tl_cell(MeshDev<float> m, RowTab t, int B, Base<float> bs,
                                                      const float *__restrict__ ut, const float *__restrict__ ht,
-                                                     float *pc, float *ke, int drag, RK<float, double> rk, int early) {
+                                                     float *pc, float *ke, RK<float, double> rk, int early) {
   using M = Mv<float, V>;
   float4 *s = row_smem();
   if (!early) pdl_begin();
@@ -72,8 +72,8 @@ __global__ void __maxnreg__(72) k_row_tl_cell(MeshDev<float> m, RowTab t, int B,
     if (c < nC && k < m.c_n[c]) r = row_tl_cell<float>(t, m, bs, c, k);
     float4 *d = s + (size_t)(lc * 6 + k) * 3;
     d[0] = make_float4(as_f(r.e), as_f(r.nb), as_f(r.sp), r.pe);
-    d[1] = make_float4(r.te, r.ke, r.ps, r.pn);
-    d[2] = make_float4(r.tn, r.pc, 0.f, 0.f);
+    d[1] = make_float4(r.th, r.ke, r.ps, r.pn);
+    d[2] = make_float4(r.tn, r.pc, r.he, 0.f);
   }
   __syncthreads();
   if (early) pdl_begin();
@@ -86,13 +86,12 @@ __global__ void __maxnreg__(72) k_row_tl_cell(MeshDev<float> m, RowTab t, int B,
 #pragma unroll
   for (int k = 0; k < 6; k++) {
     const float4 *d = s + (size_t)(th.le * 6 + k) * 3;
-    const float4 x = d[0], y = d[1];
-    const float2 z = *reinterpret_cast<const float2 *>(d + 2);
+    const float4 x = d[0], y = d[1], z = d[2];
     const M u = ldv<V>(ut + (size_t)as_i(x.x) * B + b);
     const M hn = ldv<V>(ht + (size_t)as_i(x.y) * B + b);
     const M us = ldv<V>(ut + (size_t)as_i(x.z) * B + b);
     row_add(p, x.w, u);
-    row_add(q, y.x, u);
+    row_add(q, z.z, y.x * u);
     row_add(k2, y.y, u);
     row_add(p, y.z, us);
     row_add(p, y.w, hn);
@@ -102,7 +101,6 @@ __global__ void __maxnreg__(72) k_row_tl_cell(MeshDev<float> m, RowTab t, int B,
   }
   row_add(p, cp, hc);
   row_add(q, ct, hc);
-  if (!drag) row_add(k2, float(GRAVITY), hc);
   stv<V>(pc + o, p);
   stv<V>(ke + o, k2);
   rk_members<float, double, V>(rk, o, q);
@@ -173,8 +171,7 @@ __global__ void __maxnreg__(VISC ? 72 : 48) k_row_tl_edge(MeshDev<float> m, RowT
     row_add(f, z.w, h2);
     row_add(p, y.w, ldv<V>(ht + (size_t)as_i(x.z) * B + b));
     row_add(p, z.x, ldv<V>(ht + (size_t)as_i(x.w) * B + b));
-    row_add(p, -z.y, ldv<V>(pc + (size_t)as_i(x.x) * B + b));
-    row_add(p, z.y, ldv<V>(pc + (size_t)as_i(x.y) * B + b));
+    row_add(p, z.y, ldv<V>(pc + (size_t)as_i(x.y) * B + b) - ldv<V>(pc + (size_t)as_i(x.x) * B + b));
     M d = mv_fill<float, V>(0.f);
     if (VISC) d = t.e_lap0[e] * u;
 #pragma unroll
@@ -192,7 +189,11 @@ __global__ void __maxnreg__(VISC ? 72 : 48) k_row_tl_edge(MeshDev<float> m, RowT
   }
 }
 
-// tend_u' and its RK update; GEN: any of viscosity, wind and drag
+// tend_u' and its RK update; GEN: any of viscosity, wind and drag.  The sums run so that they round no more
+// than the general pass does: a slot's two terms meet before they join the other slots', and the gradient,
+// most of the tendency, is formed from differences of rows and comes last.  Adding gravity to the ke row
+// and the gradient's halves to the sum first, without the two h' rows, took 215 instead of 227 us (level 7,
+// 64 members) but left twice the error of a white-noise tendency and 4-12 times that of a smooth one.
 template <int V, int GEN>
 __global__ void __maxnreg__(GEN ? 72 : 48) k_row_tl_tend(MeshDev<float> m, int B, Base<float> bs,
                                                      const float *__restrict__ ut, const float *__restrict__ ht,
@@ -232,42 +233,40 @@ __global__ void __maxnreg__(GEN ? 72 : 48) k_row_tl_tend(MeshDev<float> m, int B
     const int c1 = m.e_c1[e], c2 = m.e_c2[e];
     const float rdc = 1.f / m.e_dc[e];
     M q = mv_fill<float, V>(0.f);
-    row_add(q, rdc, ldv<V>(d.ke + (size_t)c1 * B + b));
-    row_add(q, -rdc, ldv<V>(d.ke + (size_t)c2 * B + b));
     float own = 0.f;
 #pragma unroll
     for (int j = 0; j < 10; j++) {
       const int i = j * th.epb + th.le;
       const size_t on = (size_t)nbs[i] * B + b;
       const float2 c = co[i];
-      row_add(q, c.x, ldv<V>(flux + on));
-      row_add(q, c.y, ldv<V>(d.pe + on));
+      M x = c.x * ldv<V>(flux + on);
+      row_add(x, c.y, ldv<V>(d.pe + on));
+      q = q + x;
       own += c.y;
     }
     row_add(q, own, ldv<V>(d.pe + o));
+    const M h1 = ldv<V>(ht + (size_t)c1 * B + b), h2 = ldv<V>(ht + (size_t)c2 * B + b);
+    M grad = ldv<V>(d.ke + (size_t)c2 * B + b) - ldv<V>(d.ke + (size_t)c1 * B + b);
+    row_add(grad, float(GRAVITY), h2 - h1);
+    row_add(q, -rdc, grad);
     if (GEN) {
       if (ph.visc2 > 0.f) row_add(q, m.e_sc2[e] * ph.visc2, ldv<V>(d.dsq_u + o));
       if (ph.visc4 > 0.f) {
         const int v1 = m.e_v1[e], v2 = m.e_v2[e];
         const float k = m.e_sc4[e] * ph.visc4, kv = k / m.e_dv[e], kc = k * rdc;
-        row_add(q, kc, ldv<V>(d.dsq_div + (size_t)c1 * B + b));
-        row_add(q, -kc, ldv<V>(d.dsq_div + (size_t)c2 * B + b));
-        row_add(q, -kv, ldv<V>(d.dsq_vort + (size_t)v1 * B + b));
-        row_add(q, kv, ldv<V>(d.dsq_vort + (size_t)v2 * B + b));
+        row_add(q, -kc, ldv<V>(d.dsq_div + (size_t)c2 * B + b) - ldv<V>(d.dsq_div + (size_t)c1 * B + b));
+        row_add(q, kv, ldv<V>(d.dsq_vort + (size_t)v2 * B + b) - ldv<V>(d.dsq_vort + (size_t)v1 * B + b));
       }
       if (ph.wind || ph.drag) {
         const float hh = bs.he[e];
-        const M h1 = ldv<V>(ht + (size_t)c1 * B + b), h2 = ldv<V>(ht + (size_t)c2 * B + b);
         float k = ph.wind ? -(m.e_usrc[e] / float(RHO_REF)) / (hh * hh) : 0.f;
-        if (ph.drag) {  // d.ke holds ke' alone: the gravity term is added here
-          const float uu = bs.u[e], sq = sqrtf(bs.ke[c1] + bs.ke[c2]), g = float(GRAVITY) * rdc;
+        if (ph.drag) {
+          const float uu = bs.u[e], sq = sqrtf(bs.ke[c1] + bs.ke[c2]);
           k += ((1.0e-3f * uu) * sq) / (hh * hh);
           row_add(q, -(1.0e-3f * sq) / hh, ldv<V>(ut + o));
           const float kk = -(((0.5f * 1.0e-3f) * uu) / sq) / hh;
           row_add(q, kk, ldv<V>(d.ke + (size_t)c1 * B + b));
           row_add(q, kk, ldv<V>(d.ke + (size_t)c2 * B + b));
-          row_add(q, g, h1);
-          row_add(q, -g, h2);
         }
         row_add(q, 0.5f * k, h1);
         row_add(q, 0.5f * k, h2);
@@ -284,6 +283,10 @@ __global__ void __maxnreg__(GEN ? 72 : 48) k_row_tl_tend(MeshDev<float> m, int B
 }
 
 // ---- adjoint ---------------------------------------------------------------------------------------
+
+// (The adjoint passes add the small terms of a value first and its largest last, so that a sum of many
+// rows rounds no more than the general passes' shorter ones: error of one level-5 stage against 64 bits,
+// general passes = 1: u_ad 0.7, h_ad 0.9; largest first 1.1 and 1.2.)
 
 // pv_edge_ad, h_edge_ad and the edge's own part of u_ad (with the ke adjoint of both cells): three
 // sums over the slots, of the weight back, the weight times pv_edge there, and the ke weight
@@ -340,13 +343,13 @@ __global__ void __maxnreg__(72) k_row_ad_edge(MeshDev<float> m, RowTab t, int B,
       row_add(h, 0.5f * bs.pe[e], p);  // sum w (pv_edge there + here) / 2
       row_add(k, (t.c_ra[c1] - t.c_ra[c2]) / m.e_dc[e], T);  // cell 1 has sign +1, cell 2 -1
       M u = kc * k;
-      row_add(u, he, h);
-      row_add(u, dv * he, fa);
       p = (0.5f * (ue * he)) * p;
       row_add(p, own, T);
+      row_add(u, -(apt * bs.gpn[e]), p);
+      row_add(u, he, h);
+      row_add(u, dv * he, fa);
       h = ue * h;
       row_add(h, ue * dv, fa);
-      row_add(u, -(apt * bs.gpn[e]), p);
       stv<V>(w.pe_ad + o, p);
       stv<V>(w.he_ad + o, h);
       stv<V>(w.ud + o, u);
@@ -384,10 +387,11 @@ __global__ void __maxnreg__(64) k_row_ad_cell(MeshDev<float> m, RowTab t, int B,
     const size_t oe = (size_t)as_i(x.x) * B + b;
     const M pe = ldv<V>(w.pe_ad + oe);
     row_add(p, x.z, pe);
-    row_add(h, y.x, pe);
-    row_add(h, x.w, ldv<V>(in.tu + oe));
-    row_add(h, y.z, ldv<V>(w.he_ad + oe));
-    row_add(h, y.y, ldv<V>(w.pe_ad + (size_t)as_i(x.y) * B + b));
+    M q = y.x * pe;
+    row_add(q, y.y, ldv<V>(w.pe_ad + (size_t)as_i(x.y) * B + b));
+    row_add(q, y.z, ldv<V>(w.he_ad + oe));
+    row_add(q, x.w, ldv<V>(in.tu + oe));
+    h = h + q;
   }
   const size_t o = (size_t)c * B + b;
   stv<V>(w.pc_ad + o, p);
@@ -424,7 +428,7 @@ __global__ void __maxnreg__(40) k_row_ad_final(MeshDev<float> m, RowTab t, int B
       const int c = c0 + th.le;
       if (c < nC) {
         const size_t o = (size_t)c * B + b;
-        M h = ldv<V>(w.hd + o);
+        M h = mv_fill<float, V>(0.f);
         float own = 0.f;
 #pragma unroll
         for (int k = 0; k < 6; k++) {
@@ -433,6 +437,7 @@ __global__ void __maxnreg__(40) k_row_ad_final(MeshDev<float> m, RowTab t, int B
           own += x.z;
         }
         row_add(h, own, ldv<V>(w.pc_ad + o));
+        h = h + ldv<V>(w.hd + o);
         ad_emit<float, double, V>(out, 0, o, h, m.c_area[c]);
       }
       __syncthreads();
@@ -485,9 +490,8 @@ __global__ void __maxnreg__(40) k_row_ad_final(MeshDev<float> m, RowTab t, int B
     const int e = e0 + th.le;
     if (e < nE) {
       const size_t o = (size_t)e * B + b;
-      M u = ldv<V>(w.ud + o);
       const float4 x = own[2 * th.le], y = own[2 * th.le + 1];
-      row_add(u, o2[th.le], ldv<V>(w.pe_ad + o));
+      M u = o2[th.le] * ldv<V>(w.pe_ad + o);
       row_add(u, y.x, ldv<V>(w.pc_ad + (size_t)as_i(x.x) * B + b));
       row_add(u, y.y, ldv<V>(w.pc_ad + (size_t)as_i(x.y) * B + b));
       row_add(u, y.z, ldv<V>(w.pc_ad + (size_t)as_i(x.z) * B + b));
@@ -497,6 +501,7 @@ __global__ void __maxnreg__(40) k_row_ad_final(MeshDev<float> m, RowTab t, int B
         const float2 c = slot[th.le * 10 + j];
         row_add(u, c.y, ldv<V>(w.pe_ad + (size_t)as_i(c.x) * B + b));
       }
+      u = u + ldv<V>(w.ud + o);
       if (bad) {
 #pragma unroll
         for (int i = 0; i < V; i++) flag_nonfinite(bad, u.x[i]);

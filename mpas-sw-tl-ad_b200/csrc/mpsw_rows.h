@@ -65,10 +65,13 @@ std::string build_rows(const BuiltMesh &m, RowTabHost *t);
 //   pv_cell' = sum (pe u'_e + ps u'_spoke + pn h'_nb) + (sum pc) h'
 //   tend_h'  = sum (te u'_e + tn h'_nb) + (sum tn) h'
 //   ke'      = sum ke u'_e
+// te is th he.  The passes multiply by the two in turn: the rounding of their product, the same in every
+// stage of a window, would add up in h' (level 5, smooth perturbations, 24 stages: 1.2 times the general
+// passes' error, 0.85 in turn).
 template <typename R>
 struct RowTlCell {
   int e, nb, sp;
-  R pe, ps, pn, pc, te, tn, ke;
+  R pe, ps, pn, pc, te, tn, ke, th, he;
 };
 template <typename R, class T, class M, class BS>
 MPSW_HD inline RowTlCell<R> row_tl_cell(const T &t, const M &m, const BS &bs, int c, int k) {
@@ -81,13 +84,15 @@ MPSW_HD inline RowTlCell<R> row_tl_cell(const T &t, const M &m, const BS &bs, in
   const R ra = R(1) / bs.hv[a], rb = R(1) / bs.hv[b], rv = R(1) / bs.hv[v];
   const R za = ((m.v_f[a] + bs.vort[a]) * ra) * ra, zb = ((m.v_f[b] + bs.vort[b]) * rb) * rb,
           zv = ((m.v_f[v] + bs.vort[v]) * rv) * rv;
-  const R u = bs.u[r.e], he = bs.he[r.e], th = t.c_t[s];
+  const R u = bs.u[r.e];
+  r.th = t.c_t[s];
+  r.he = bs.he[r.e];
   r.pe = t.c_g1[s] * ra + t.c_g2[s] * rb;
   r.ps = t.c_g3[s] * rv;
   r.pn = -(t.c_n1[s] * za + t.c_n2[s] * zb);
   r.pc = -(t.c_m[s] * zv);
-  r.te = th * he;
-  r.tn = R(0.5) * (th * u);
+  r.te = r.th * r.he;
+  r.tn = R(0.5) * (r.th * u);
   r.ke = t.c_q[s] * u;
   return r;
 }
