@@ -73,9 +73,8 @@ struct Window {
   std::vector<double *> sn_u, sn_h;
   std::vector<long long> bin_cost;
   std::vector<int> bin_split;
-  long long forward_steps = 0;  // trajectory steps recomputed by the last adjoint sweep
   int store_now = 0;          // precisions the forward being launched stores (bit 0 FP64, bit 1 FP32)
-  Phys<double> forward_phys{}; // physics of the forward sweep that wrote the checkpoints
+  long long forward_steps = 0;  // trajectory steps recomputed by the last adjoint sweep
   int store_mode = -1;        // -1 automatic, else a mask of the precisions to store
   double store_budget = 0;    // bytes for automatic mode (0: 40% of free device memory)
   // member buffers per precision (0 FP64, 1 FP32), allocated for the largest B seen

@@ -274,6 +274,7 @@ void Engine::window_store_alloc(int nsteps) {
     if (!S.mem || S.cap < nsteps || S.slot != slot) {
       window_store_free(p);
       cuda_check(cudaMalloc(&S.mem, per * (p ? sizeof(float) : sizeof(double))), "cudaMalloc window store");
+      graphs_free();  // captured forward sweeps write the stores that were there
       S.cap = nsteps;
     }
     S.slot = slot;
@@ -497,14 +498,12 @@ static void window_forward_done(Engine &E) {
   cuda_check(cudaMemcpyAsync(W.fin_u, W.x_u, sizeof(double) * E.nE, cudaMemcpyDeviceToDevice, E.stream), "final");
   cuda_check(cudaMemcpyAsync(W.fin_h, W.x_h, sizeof(double) * E.nC, cudaMemcpyDeviceToDevice, E.stream), "final");
   cuda_check(cudaGetLastError(), "window forward");
-  for (int p = 0; p < 2; p++)
-    if ((W.store_now >> p) & 1) W.st[p].valid = W.nsteps;
+  for (int p = 0; p < 2; p++) W.st[p].valid = (W.store_now >> p) & 1 ? W.nsteps : 0;
   W.pending = false;
-  W.forward_phys = E.phys();
 }
 
-// Forward over the window from the start state in x_u, x_h, checkpointing every `every` steps and
-// writing every stage's linearisation point to the stores of the precisions in `stores` (the
+// Forward over the window from the captured start state, checkpointing every `every` steps
+// and writing every stage's linearisation point to the stores of the precisions in `stores` (the
 // whole window is then one CUDA graph, since every step writes different slots).
 void Engine::window_forward(int stores) {
   Window &W = win;
@@ -528,26 +527,23 @@ void Engine::window_forward(int stores) {
   window_forward_done(*this);
 }
 
-// The forward sweep, for a sweep of precision prec (-1: for the final state).  The store written is
-// that of the precision that asks first; a window that later sweeps in the other one as well runs
-// the forward again for its store, from the first checkpoint and with the physics of the first run.
+// The stores that the forward of a window writes whose first sweep has precision prec: FP32 sweeps
+// leave FP64 stages as well where both are kept, since only the forward could form them later; FP64
+// sweeps leave FP64 stages alone, which window_ensure rounds for a later FP32 sweep (level 6, eight
+// FP64 members: 5.6 ms a gradient, 5.9 with both).
+static int window_stores(const Window &W, int prec) {
+  const int have = (W.st[0].mem ? 1 : 0) | (W.st[1].mem ? 2 : 0);
+  return prec != 1 && (have & 1) ? 1 : have;
+}
+
+// The forward sweep, and the stored stages in precision prec (-1: the final state alone).
 void Engine::window_ensure(int prec) {
   Window &W = win;
-  const int have = (W.st[0].mem ? 1 : 0) | (W.st[1].mem ? 2 : 0), want = prec >= 0 ? have & (1 << prec) : have & 1 ? 1 : have;
-  if (W.pending) {
-    window_forward(want);
-  } else if (want && prec >= 0 && W.st[prec].valid < W.nsteps) {
-    cuda_check(cudaMemcpyAsync(W.x_u, W.ck_u[0], sizeof(double) * nE, cudaMemcpyDeviceToDevice, stream), "copy");
-    cuda_check(cudaMemcpyAsync(W.x_h, W.ck_h[0], sizeof(double) * nC, cudaMemcpyDeviceToDevice, stream), "copy");
-    const Phys<double> now = phys_cache;
-    phys_cache = W.forward_phys;
-    try {
-      window_forward(want);
-    } catch (...) {
-      phys_cache = now;
-      throw;
-    }
-    phys_cache = now;
+  if (W.pending) window_forward(window_stores(W, prec));
+  if (prec == 1 && W.st[1].mem && W.st[1].valid < W.nsteps && W.st[0].valid >= W.nsteps) {
+    convert_d2f((long long)W.nsteps * 4 * W.st[0].slot, (const double *)W.st[0].mem, (float *)W.st[1].mem, stream);
+    cuda_check(cudaGetLastError(), "window stages");
+    W.st[1].valid = W.nsteps;
   }
 }
 
@@ -679,7 +675,7 @@ static void window_tl_impl(Engine &E, int prec, int Bu, double *user_u, double *
       bool &b;
       ~Reset() { b = false; }
     } reset{E.beside_members};
-    W.store_now = 1 << prec;
+    W.store_now = window_stores(W, prec);
     E.run_graph(key, [&]() {
       cuda_check(cudaEventRecord(E.ev_fork, E.stream), "event record");
       cuda_check(cudaStreamWaitEvent(E.side, E.ev_fork, 0), "event wait");
