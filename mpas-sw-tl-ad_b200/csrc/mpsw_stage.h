@@ -74,7 +74,7 @@ static_assert(kTlBase % 2 == 0, "the records behind start on 16 bytes");
 //   pv_edge edges:  c1 c2 v1 v2 as local indices, edgesOnEdge[10]; weights [10], dc, dv
 // Areas and lengths are divisors: FP64 records hold them, FP32 ones their reciprocals (stage_over).
 // The edge records come last and go to registers; what is before them goes to shared memory.
-// Slots past a list weigh zero and point at the entity itself (cells) or at value 0.
+// Slots past a list weigh zero and repeat its first entry, so that a NaN there spreads no further.
 enum StageSection { SB_V, SB_CM, SB_CX, SB_CK, SB_CO, SB_E, SB_GE, SB_GC, SB_GV, kStageSections };
 
 MPSW_HD inline int stage_chunks(int vals, int r) { return (vals * r + 15) / 16; }

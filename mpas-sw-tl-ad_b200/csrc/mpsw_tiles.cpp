@@ -470,16 +470,17 @@ void stage_pack(const Builder &b, const BuiltMesh &m, const Space &E, const Spac
   for (int i = 0; i < ncm; i++) {
     const int c = C.list[i];
     for (int k = 0; k < kCellSlots; k++) {
-      const size_t s = (size_t)k * m.nC + c;
-      if (i < nco) list(SB_CO, nco, i, k, k < b.cn(c) ? C.local(b.cnb(c, k)) : i);
-      if (k >= b.cn(c)) continue;  // padded: value 0 with coefficient 0
+      const bool has = k < b.cn(c);  // a padded slot: the first slot's neighbours, weight 0
+      const size_t s = (size_t)(has ? k : 0) * m.nC + c;
+      if (i < nco) list(SB_CO, nco, i, k, C.local(b.cnb(c, has ? k : 0)));
       list(SB_CM, ncm, i, k, V.local(m.c_vs[s]));
-      val(SB_CM, ncm, 1, i, k, R(m.c_vk[s]));
       list(SB_CX, ncm, i, k, E.local(m.c_es[s]));
+      if (i < nck) list(SB_CK, nck, i, k, E.local(m.c_eoc[s]));
+      if (!has) continue;
+      val(SB_CM, ncm, 1, i, k, R(m.c_vk[s]));
       val(SB_CX, ncm, 1, i, k, R(m.c_esg[s]) * R(m.e_dv[m.c_es[s]]));
       if (i < nck) {
         const int e = m.c_eoc[s];
-        list(SB_CK, nck, i, k, E.local(e));
         val(SB_CK, nck, 1, i, k, (R(0.25) * R(m.e_dc[e])) * R(m.e_dv[e]));
       }
     }
@@ -494,7 +495,7 @@ void stage_pack(const Builder &b, const BuiltMesh &m, const Space &E, const Spac
     list(SB_E, nem, i, 3, V.local(m.e_v2[e]));
     for (int j = 0; j < kEoeSlots; j++) {
       const bool has = j < m.e_n[e];  // a padded slot weighs nothing
-      list(SB_E, nem, i, 4 + j, has ? E.local(b.eoe(e, j)) : i);
+      list(SB_E, nem, i, 4 + j, m.e_n[e] ? E.local(b.eoe(e, has ? j : 0)) : i);
       val(SB_E, nem, 2, i, j, has ? R(m.e_w[(size_t)j * m.nE + e]) : R(0));
     }
     val(SB_E, nem, 2, i, 10, divisor(m.e_dc[e]));
@@ -572,13 +573,14 @@ void stage_ad_pack(const Builder &b, const BuiltMesh &m, const Space &E, const S
   }
   for (int i = 0; i < ncm; i++) {
     const int c = C.list[i];
-    for (int k = 0; k < b.cn(c); k++) {
-      const size_t s = (size_t)k * m.nC + c;
+    for (int k = 0; k < kCellSlots; k++) {
+      const bool has = k < b.cn(c);  // (as above)
+      const size_t s = (size_t)(has ? k : 0) * m.nC + c;
       list(YB_C, ncm, i, k, E.local(m.c_es[s]));
+      if (i < nco) list(YB_O, nco, i, k, V.local(m.c_vs[s]));
+      if (!has) continue;
       val(YB_C, ncm, 1, i, k, m.c_esg[s]);
-      if (i >= nco) continue;
-      list(YB_O, nco, i, k, V.local(m.c_vs[s]));
-      val(YB_O, nco, 1, i, k, m.c_vk[s]);
+      if (i < nco) val(YB_O, nco, 1, i, k, m.c_vk[s]);
     }
     val(YB_C, ncm, 1, i, 6, m.c_area[c]);
     if (i < nco) val(YB_O, nco, 1, i, 6, m.c_area[c]);
@@ -591,7 +593,7 @@ void stage_ad_pack(const Builder &b, const BuiltMesh &m, const Space &E, const S
     list(YB_E, nem, i, 3, V.local(m.e_v2[e]));
     for (int j = 0; j < kEoeSlots; j++) {
       const bool has = j < m.e_n[e];  // a padded slot weighs nothing
-      list(YB_E, nem, i, 4 + j, has ? E.local(b.eoe(e, j)) : i);
+      list(YB_E, nem, i, 4 + j, m.e_n[e] ? E.local(b.eoe(e, has ? j : 0)) : i);
       val(YB_E, nem, 2, i, j, has ? m.e_w[(size_t)j * m.nE + e] : 0.0);
       val(YB_E, nem, 2, i, 10 + j, has ? m.e_wrev[(size_t)j * m.nE + e] : 0.0);
     }
