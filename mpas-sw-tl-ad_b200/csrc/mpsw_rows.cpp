@@ -155,6 +155,9 @@ std::string build_rows(const BuiltMesh &m, RowTabHost *t) {
       t->e_kr[E(e, 3 * k + 2)] = ko / ta / m.c_area[o];
       (k ? t->e_i2 : t->e_i1)[e] = 1.0 / ta;
     }
+    for (int i = 0; i < 4; i++)  // a pass adds the four terms to their slots side by side
+      for (int j = 0; j < i; j++)
+        if (((q >> (8 * i)) & 0xFF) == ((q >> (8 * j)) & 0xFF)) return "two edges between the same vertices";
     t->e_q[e] = (int)q;
   }
   return "";
