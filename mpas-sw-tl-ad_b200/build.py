@@ -38,7 +38,7 @@ UNITS = [
     ('mpsw_rows.cpp', ['--fmad=false', '-x', 'cu']),
 ]
 HEADERS = ['mpsw_internal.h', 'mpsw_kernels.cuh', 'mpsw_launch.h', 'mpsw_launch.cuh', 'mpsw_members.cuh',
-           'mpsw_fused.cuh', 'mpsw_stage.h', 'mpsw_stage.cuh', 'mpsw_rows.h', 'mpsw_rows.cuh', 'mpsw_setup.h', 'mpsw_tiles.h', 'mpsw_engine.h']
+           'mpsw_fused.cuh', 'mpsw_stage.h', 'mpsw_stage.cuh', 'mpsw_rows.h', 'mpsw_rows.cuh', 'mpsw_setup.h', 'mpsw_parts.h', 'mpsw_tiles.h', 'mpsw_engine.h']
 
 
 def _nvcc():

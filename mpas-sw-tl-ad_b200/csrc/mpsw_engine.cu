@@ -13,8 +13,6 @@
 #include <cmath>
 #include <cctype>
 #include <cstring>
-#include <system_error>
-#include <thread>
 #include <map>
 #include <memory>
 #include <stdexcept>
@@ -24,6 +22,7 @@
 #include "mpsw.h"
 #include "mpsw_engine.h"
 #include "mpsw_launch.h"
+#include "mpsw_parts.h"
 #include "mpsw_setup.h"
 
 using namespace mpsw;
@@ -353,36 +352,6 @@ void Engine::download(Var &v) {
   v.host_valid = false;
   download_start(v);
   copies_done();
-}
-
-// memcpy / memcmp of large arrays over a few threads
-template <typename F>
-static void in_parts(size_t bytes, F &&f) {
-  constexpr size_t kPart = (size_t)2 << 20;
-  const int parts = (int)std::min<size_t>(4, bytes / kPart);
-  if (parts < 2) {
-    f(0, 0, bytes);
-    return;
-  }
-  std::vector<std::thread> ts;
-  const size_t step = (bytes / parts + 63) / 64 * 64;
-  auto part = [&](int i) { f(i, i * step, i + 1 < parts ? (i + 1) * step : bytes); };
-  int i = 1;
-  try {
-    for (; i < parts; i++) ts.emplace_back(part, i);
-  } catch (const std::system_error &) {  // no more threads: the rest here
-  }
-  for (; i < parts; i++) part(i);
-  part(0);
-  for (auto &t : ts) t.join();
-}
-static void copy_bytes(void *dst, const void *src, size_t bytes) {
-  in_parts(bytes, [=](int, size_t a, size_t b) { std::memcpy((char *)dst + a, (const char *)src + a, b - a); });
-}
-static bool same_bytes(const void *x, const void *y, size_t bytes) {
-  bool eq[4] = {true, true, true, true};
-  in_parts(bytes, [&](int i, size_t a, size_t b) { eq[i] = !std::memcmp((const char *)x + a, (const char *)y + a, b - a); });
-  return eq[0] && eq[1] && eq[2] && eq[3];
 }
 
 static bool mirror_equals(const Var &v, const void *x) {
