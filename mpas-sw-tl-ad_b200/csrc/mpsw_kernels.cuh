@@ -451,7 +451,7 @@ static __global__ void k_members_resize(long long n, int Bd, double *dst, int Bs
   MPSW_GRID_LOOP(t, n * Bd) {
     const long long i = t / Bd;
     const int b = (int)(t - i * Bd);
-    dst[t] = b < Bs ? src[i * Bs + b] : 0.0;
+    dst[t] = src[i * Bs + (b < Bs ? b : Bs - 1)];
   }
 }
 

@@ -121,7 +121,7 @@ struct Launch {
 
 void convert_d2f(long long n, const double *src, float *dst, cudaStream_t s);
 void convert_d2f_off(long long n, const double *src, double off, float *dst, cudaStream_t s);
-// rows of Bd doubles from rows of Bs: the first min(Bd, Bs) copied, the rest zero
+// rows of Bd doubles from rows of Bs: the first min(Bd, Bs) copied, the last of them repeated
 void members_resize(long long n, int Bd, double *dst, int Bs, const double *src, cudaStream_t s);
 // a module variable's values, [lead] fastest in the reference layout, to and from [lead][n] internal order
 void var_to_internal(int n, int lead, const int *perm, const double *src, double *dst, cudaStream_t s);

@@ -29,13 +29,19 @@ namespace {
 using L64 = Launch<double, double>;
 
 // Members a sweep of B members runs with: counts that are no multiple of a thread's vector width
-// would move one member at a time, so the engine's own buffers hold a few zero members more.
-// Level 6, 6 steps, ms a tangent-linear / adjoint pair: FP32 members 28 -> 6.09, 32 -> 5.79; 36 ->
-// 7.63, 40 -> 7.43; 12 -> 3.80, 16 -> 3.98; 13 one at a time 6.22, padded 4.13.  FP64 3 -> 3.75, 4 -> 3.24; 10 ->
-// 6.21, 12 -> 6.06; 5 -> 4.62, 6 -> 4.79, 8 -> 4.88 (5 and 6 stay).
+// would move one member at a time, so the engine's own buffers repeat the last member a few times
+// (zeros would send every FP64 division into its slow path: level 3, seven members, an adjoint sweep
+// 0.50 -> 0.60 ms).  ms a tangent-linear / adjoint pair as given -> padded:
+//   FP64, to even counts: level 7 (2 steps) 3 -> 4 5.0 -> 4.7, 9 -> 10 9.1 -> 7.7; level 5 (6 steps) 9 -> 10
+//   1.94 -> 1.88; 10 -> 12 gains nothing (7.7 -> 8.0).
+//   FP32, to four: level 6 (4 steps) 9 -> 12 3.3 -> 2.8, 10 -> 12 2.84 -> 2.80, 18 -> 20 3.8 -> 3.6, but 12 -> 16
+//   2.80 -> 2.85; 6, which moves in pairs, 2.26 -> 2.42.  From 24 on, where the row passes take eight members a
+//   thread, to eight: 25 -> 28 4.2, -> 32 3.9; level 7 33 -> 36 9.2, -> 40 9.0.
 int padded_members(int prec, int B) {
-  if (prec == 1) return B <= 2 ? B : B <= 4 ? 4 : (B + 7) / 8 * 8;
-  return B <= 2 || B == 5 || B == 6 ? B : (B + 3) / 4 * 4;
+  if (B <= 2) return B;
+  if (prec != 1) return B + B % 2;
+  if (B == 6) return B;
+  return B < 24 ? (B + 3) / 4 * 4 : B / 8 * 8 + (B % 8 ? 8 : 0);
 }
 
 template <typename R>
@@ -639,7 +645,7 @@ static void tl_member_stage(Engine &E, int prec, int B, double *du, double *dh, 
 }
 
 // Copy members' FP64 states between a caller's buffers and the engine's (internal order): rows of
-// Bd members from rows of Bs, zeros past the source's.
+// Bd members from rows of Bs, the last of them repeated.
 static void members_copy(Engine &E, int Bd, double *dst_u, double *dst_h, int Bs, const double *src_u,
                          const double *src_h) {
   if (Bd != Bs) {
