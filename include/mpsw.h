@@ -136,7 +136,8 @@ int mpsw_window_storage(mpsw_handle *h, int mode, double max_bytes);
  * reference.  The first sweep of a window for a given (precision, B) times each kernel over the
  * pairs B allows on the window's own buffers and keeps the fastest (MPSW_TUNE=0 in the
  * environment keeps fixed defaults; MPSW_TUNE_CACHE=<file> keeps the choices in a text file
- * keyed by device, mesh size, precision and B, and reuses them).  Kernels that the sweeps of this
+ * keyed by device, mesh size, the kernels that run, precision and B, and reuses them).  Physics that
+ * brings other kernels is tuned by itself.  Kernels that the sweeps of this
  * (precision, B) do not run stay at zero: tl_vertex and ad_vertex where FP32 members take the three
  * row passes, all four of a sweep where few FP64 members take one kernel a stage. */
 int mpsw_window_tuning(mpsw_handle *h, int precision, int B, int *v_block);

@@ -88,7 +88,7 @@ struct Window {
     double *x_u = nullptr, *x_h = nullptr;
   } ms[2];
   // autotuned launch choices of the member kernels, per precision and member count
-  std::map<int, TuneTable> tune[2];
+  std::map<std::pair<int, int>, TuneTable> tune[2];  // by member count and kernel_forms()
 };
 
 // A captured CUDA graph of one window step, keyed by what its kernels bake in.
@@ -264,6 +264,7 @@ struct Engine {
   void window_ad(int prec, int B, double *au, double *ah, cudaStream_t s);
   void window_final(double *u, double *h, cudaStream_t s);
   double time_kernel(int which, int prec, int B, int iters);
+  int kernel_forms(int prec, int B) const;  // kernels that the sweeps of B members run
   const TuneTable *tuning(int prec, int B);
   const TuneTable *tuned_for(int prec, int B);
   void state_from_device(const double *u, const double *h, cudaStream_t s);

@@ -1156,8 +1156,20 @@ static TuneTable tune_members(Engine &E, int prec, int B) {
   return best;
 }
 
+// What the choices depend on besides the precision and the count: the kernels that a sweep runs follow from
+// the physics and from the tables the mesh has.  Tangent linear + 3 adjoint, each 0 general passes, 1
+// row passes, 2 tile stages.
+int Engine::kernel_forms(int prec, int B) const {
+  const Phys<double> ph = phys();
+  if (prec != 1) return (stage_tl_tiled(B) ? 2 : 0) + 3 * (stage_ad_tiled(B, ph) ? 2 : 0);
+  const Phys<float> pf = phys_as<float>(ph);
+  using L32 = Launch<float, double>;
+  return (L32::rows_ok(rows, nE, B, pf, false) ? 1 : 0) + 3 * (L32::rows_ok(rows, nE, B, pf, true) ? 1 : 0);
+}
+
 // Tuning results can be kept in a text file (MPSW_TUNE_CACHE=path), one line per key:
-// "<device name>|<nCells>|<nEdges>|<nVertices>|<precision>|<B>" then 8 pairs "v block".  A
+// "<device name>|<nCells>|<nEdges>|<nVertices>|<precision>|<B>", where a sweep runs other kernels than the
+// general passes "|<kernel_forms>" before the precision, then 8 pairs "v block".  A
 // process finding its key there skips the timing (so, for example, a profiled run uses the
 // choices of an unprofiled one).
 static std::string tune_key(const Engine &E, int prec, int B) {
@@ -1167,8 +1179,9 @@ static std::string tune_key(const Engine &E, int prec, int B) {
   std::string name(p.name);
   for (char &c : name)
     if (c == ' ' || c == '|') c = '_';
+  const int forms = E.kernel_forms(prec, B);
   return name + "|" + std::to_string(E.nC) + "|" + std::to_string(E.nE) + "|" + std::to_string(E.nV) + "|" +
-         std::to_string(prec) + "|" + std::to_string(B);
+         (forms ? std::to_string(forms) + "|" : "") + std::to_string(prec) + "|" + std::to_string(B);
 }
 
 static bool tune_cache_read(const std::string &path, const std::string &key, TuneTable *t) {
@@ -1206,7 +1219,8 @@ static void tune_cache_append(const std::string &path, const std::string &key, c
 const TuneTable *Engine::tuning(int prec, int B) {
   static const bool enabled = !(getenv("MPSW_TUNE") && atoi(getenv("MPSW_TUNE")) == 0);
   if (!enabled) return nullptr;
-  auto it = win.tune[prec].find(B);
+  const std::pair<int, int> id(B, kernel_forms(prec, B));
+  auto it = win.tune[prec].find(id);
   if (it != win.tune[prec].end()) return &it->second;
   const char *cache = getenv("MPSW_TUNE_CACHE");
   const std::string key = tune_key(*this, prec, B);
@@ -1216,12 +1230,12 @@ const TuneTable *Engine::tuning(int prec, int B) {
     if (cache && *cache) tune_cache_append(cache, key, t);
   }
   graphs_free();  // nothing captured before this point may keep the untuned choices
-  return &(win.tune[prec][B] = t);
+  return &(win.tune[prec][id] = t);
 }
 
 // The table for (prec, B) if it has been tuned, else null (defaults).
 const TuneTable *Engine::tuned_for(int prec, int B) {
-  auto it = win.tune[prec].find(B);
+  auto it = win.tune[prec].find({B, kernel_forms(prec, B)});
   return it == win.tune[prec].end() ? nullptr : &it->second;
 }
 
