@@ -806,8 +806,11 @@ bool Engine::stage_tiled() const { return st64.ntiles > 0 && (!beside_members ||
 // 17.9 -> 6.4, level 5 24.5 -> 10.0, level 6 44.2 -> 31.3).  A second member has blocks of its own: 14.0
 // -> 6.6 and 22.7 -> 18.3 while both members' blocks are on the chip together, 40.7 -> 63.1 at level 6.
 // From three on the passes read whole rows of members and win (level 5, three: 27.4 against 30.8).
-bool Engine::stage_tl_tiled(int B) const {
-  return st64.ntiles > 0 && (B == 1 || (B == 2 && st64.ntiles <= 2 * 148));
+// With del4 a block takes 118 KB and an SM one of them: tiles that run in more than two rounds lose
+// (level 6, one member, a six-step sweep: 1.47 against 1.37 ms; level 5 0.44 against 0.70).
+bool Engine::stage_tl_tiled(int B, const Phys<double> &ph) const {
+  if (st64.ntiles <= 2 * 148) return st64.ntiles > 0 && B <= 2;
+  return B == 1 && !(ph.visc4 > 0.0);
 }
 
 // The adjoint's line is the tangent linear's, for its reasons (passes -> tiles: level 3 19.0 -> 5.2, level 4
@@ -1133,7 +1136,7 @@ void Engine::rk4_tlm(int nsteps) {  // src/mpas_sw_module.f90:637-781
       const double *hti = k == 0 ? ht0 : tp_h[k - 1];
       RK<double, double> rut{ut0, k == 0 ? ut0 : tacc_u, k == 3 ? ut0 : tacc_u, k < 3 ? tp_u[k] : nullptr, c[k], w[k], 0.0, ph.tc1};
       RK<double, double> rht{ht0, k == 0 ? ht0 : tacc_h, k == 3 ? ht0 : tacc_h, k < 3 ? tp_h[k] : nullptr, c[k], w[k], 0.0, 0};
-      if (stage_tl_tiled(1)) {
+      if (stage_tl_tiled(1, ph)) {
         L64::stage_tl(st64, StageTlArgs{uti, hti, 1, bs, ph, rut, rht, k == 3 ? dv("tend_u_tl") : nullptr,
                                         k == 3 ? dv("tend_h_tl") : nullptr, m64.e_sc2, m64.e_sc4, m64.e_usrc}, stream);
         continue;

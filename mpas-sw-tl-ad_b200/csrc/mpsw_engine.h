@@ -218,7 +218,7 @@ struct Engine {
                  const RK<double, double> &rku, const RK<double, double> &rkh, double *tu, double *th,
                  const StageBaseOut &out);
   bool stage_tiled() const;
-  bool stage_tl_tiled(int B) const;  // FP64 members take the tiles' tangent-linear stage
+  bool stage_tl_tiled(int B, const Phys<double> &ph) const;  // FP64 members take the tiles' tangent-linear stage
   bool stage_ad_tiled(int B, const Phys<double> &ph) const;  // and the adjoint's
   void tl_diag_run(const Base<double> &bs, const double *ut, const double *ht, const Diag<double> &d,
                    const Phys<double> &ph);

@@ -230,9 +230,9 @@ struct StageTlRk {
 // A tangent-linear stage of FP64 members, one a block (blockIdx.y), phase by phase as k_stage and, like
 // it, bound by the chain of phases rather than by bytes or arithmetic.  early: the linearisation point is
 // stored, so its values, like the mesh, are fetched before the wait for the stage before; two blocks
-// stay on an SM (110 KB each with viscosity), so that the next stage's fetch overlaps this one.  At one
-// block an SM: 13.4 instead of 10.0 us a level-5 stage; the four passes took 24.5 (stages of a window
-// sweep of one member).
+// stay on an SM (106 KB each, 110 with del2 viscosity), so that the next stage's fetch overlaps this one;
+// del4 takes 118 KB and leaves one.  At one block an SM without viscosity: 13.4 instead of 10.0 us a level-5
+// stage; the four passes took 24.5 (stages of a window sweep of one member).
 template <typename R>  // double
 __global__ void __launch_bounds__(kStageThreads, 2) k_stage_tl(StageDev ts, StageTlArgs a, int early) {
   static_assert(sizeof(R) == 8);

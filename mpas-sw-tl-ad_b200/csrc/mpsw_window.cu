@@ -623,7 +623,7 @@ static void tl_member_stage(Engine &E, int prec, int B, double *du, double *dh, 
     return;
   }
   if constexpr (f64) {
-    if (E.stage_tl_tiled(B)) {
+    if (E.stage_tl_tiled(B, ph)) {
       Launch<R, double>::stage_tl(E.st64, StageTlArgs{uti, hti, B, bs, ph, rut, rht, nullptr, nullptr, m.e_sc2, m.e_sc4,
                                               m.e_usrc}, st);
       return;
@@ -657,6 +657,21 @@ static void members_copy(Engine &E, int Bd, double *dst_u, double *dst_h, int Bs
   cuda_check(cudaMemcpyAsync(dst_h, src_h, sizeof(double) * E.nC * Bd, cudaMemcpyDeviceToDevice, E.stream), "members");
 }
 
+struct BesideScope {  // Engine::beside_members while stages are launched
+  Engine &E;
+  const bool prev;
+  BesideScope(Engine &e, bool on) : E(e), prev(e.beside_members) { E.beside_members = on; }
+  ~BesideScope() { E.beside_members = prev; }
+};
+
+// Stages recomputed for a sweep run between its member stages, where tiles win as they do alone, but for
+// del4 (level 6, a stage, tiles against passes: 64 FP32 members 312 / 282 us, 24 188 / 185 and adjoint 196 /
+// 210, 2 95 / 110; FP64 members 2 108 / 97, 8 171 / 152).  Few tiles stay (Engine::stage_tiled): level 5, 64 FP32
+// members 88 / 107.
+static bool passes_between(int prec, int B, const Phys<double> &ph) {
+  return ph.visc4 > 0.0 && B > (prec == 1 ? 32 : 1);
+}
+
 template <typename R>
 static void window_tl_impl(Engine &E, int prec, int Bu, double *user_u, double *user_h) {
   const int B = padded_members(prec, Bu);
@@ -676,11 +691,7 @@ static void window_tl_impl(Engine &E, int prec, int Bu, double *user_u, double *
     key.p3 = W.st[prec].mem;
     key.n2 = ((long long)W.nsteps << 20) | W.every;
     StableBaseScope stable(true);  // the members read only stored stages
-    E.beside_members = prec == 1 || !E.stage_tl_tiled(B);  // (tiled members leave the tiles room)
-    struct Reset {
-      bool &b;
-      ~Reset() { b = false; }
-    } reset{E.beside_members};
+    BesideScope beside(E, prec == 1 || !E.stage_tl_tiled(B, ph64));  // (tiled members leave the tiles room)
     W.store_now = window_stores(W, prec);
     E.run_graph(key, [&]() {
       cuda_check(cudaEventRecord(E.ev_fork, E.stream), "event record");
@@ -721,6 +732,7 @@ static void window_tl_impl(Engine &E, int prec, int Bu, double *user_u, double *
     const GraphKey key = E.graph_key(2, prec, B, du, dh);
     for (int n = 0; n < W.nsteps; n++)
       E.run_graph(key, [&]() {
+        BesideScope beside(E, passes_between(prec, B, ph64));
         traj_step(E, true, prec, true, [&](int k) {
           tl_member_stage<R>(E, prec, B, du, dh, mb, ph, w, c, k, base_for<R>(W, k), E.stream, true);
         });
@@ -836,6 +848,7 @@ static void window_ad_impl(Engine &E, int prec, int Bu, double *user_u, double *
   };
   auto adjoint_step = [&]() {  // the adjoint of the step that starts at x_u, x_h
     E.run_graph(E.graph_key(3, prec, B, au, ah), [&]() {
+      BesideScope beside(E, passes_between(prec, B, ph64));
       traj_step(E, false, prec, true, [](int) {});
       ad_member_step<R>(E, prec, B, au, ah, mb, ph, w, c, [&](int k) { return base_for<R>(W, k); });
     });
@@ -1047,7 +1060,7 @@ static double time_kernel_impl(Engine &E, int which, int prec, int B, int iters,
           break;
         }
         if constexpr (sizeof(R) == 8) {
-          if (E.stage_tl_tiled(B)) {
+          if (E.stage_tl_tiled(B, ph)) {
             LR::stage_tl(E.st64, StageTlArgs{mb->pu[0], mb->ph[0], B, bs, ph, rku, rkh, nullptr, nullptr, m.e_sc2, m.e_sc4,
                                              m.e_usrc}, E.stream);
             break;
@@ -1132,7 +1145,7 @@ static TuneTable tune_members(Engine &E, int prec, int B) {
   const int vs[] = {1, 2, 4, 8}, blocks[] = {64, 128, 256};
   for (int k = 0; k < K_TUNED; k++) {
     if constexpr (sizeof(R) == 8)  // passes that the sweeps do not run
-      if (k < K_AD_EDGE ? E.stage_tl_tiled(B) : E.stage_ad_tiled(B, ph)) continue;
+      if (k < K_AD_EDGE ? E.stage_tl_tiled(B, ph) : E.stage_ad_tiled(B, ph)) continue;
     double tbest = 1e30;
     for (int v : vs) {
       if (B % v || (sizeof(R) == 8 && v > 4) || (sizeof(R) == 4 && v < 2 && B % 2 == 0)) continue;
@@ -1161,7 +1174,7 @@ static TuneTable tune_members(Engine &E, int prec, int B) {
 // row passes, 2 tile stages.
 int Engine::kernel_forms(int prec, int B) const {
   const Phys<double> ph = phys();
-  if (prec != 1) return (stage_tl_tiled(B) ? 2 : 0) + 3 * (stage_ad_tiled(B, ph) ? 2 : 0);
+  if (prec != 1) return (stage_tl_tiled(B, ph) ? 2 : 0) + 3 * (stage_ad_tiled(B, ph) ? 2 : 0);
   const Phys<float> pf = phys_as<float>(ph);
   using L32 = Launch<float, double>;
   return (L32::rows_ok(rows, nE, B, pf, false) ? 1 : 0) + 3 * (L32::rows_ok(rows, nE, B, pf, true) ? 1 : 0);
