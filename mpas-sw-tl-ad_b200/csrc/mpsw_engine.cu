@@ -416,10 +416,14 @@ void Engine::mark_written(Var &v, bool maybe_nonzero) {
 // ---- device mesh -----------------------------------------------------------------------
 template <typename T, typename S>
 const T *Engine::up(const std::vector<S> &h, std::vector<void *> &own) {
-  std::vector<T> t(h.begin(), h.end());
+  std::vector<T> as;
+  if constexpr (!std::is_same<T, S>::value) as.assign(h.begin(), h.end());
+  const T *src;
+  if constexpr (std::is_same<T, S>::value) src = h.data();
+  else src = as.data();
   void *p = nullptr;
-  cuda_check(cudaMalloc(&p, sizeof(T) * (t.empty() ? 1 : t.size())), "cudaMalloc mesh");
-  if (!t.empty()) cuda_check(cudaMemcpy(p, t.data(), sizeof(T) * t.size(), cudaMemcpyHostToDevice), "mesh upload");
+  cuda_check(cudaMalloc(&p, sizeof(T) * (h.empty() ? 1 : h.size())), "cudaMalloc mesh");
+  if (!h.empty()) cuda_check(cudaMemcpy(p, src, sizeof(T) * h.size(), cudaMemcpyHostToDevice), "mesh upload");
   own.push_back(p);
   return (const T *)p;
 }
@@ -530,29 +534,40 @@ void Engine::build_fused() {
 // level 7, beyond the line, 93.7 / 66.8 and 63.2 / 49.9.  Tiles own as many cells as give each of
 // the 148 SMs one, on meshes for which that is fewer than the layers' caps allow.
 // MPSW_STAGE_TILES=0 keeps the passes.
-void Engine::build_stage() {
-  constexpr size_t kL2 = (size_t)110 << 20;
-  st64 = st32 = st_ad = StageDev();
-  const char *off = getenv("MPSW_STAGE_TILES");
-  if ((off && atoi(off) == 0) || (size_t)nC * 1200 > kL2) return;
+static constexpr size_t kTilesL2 = (size_t)110 << 20;
+
+// The host's part of these tiles and of the row tables, side by side (level 6: 0.95 s one after the
+// other on one core, a third of it so).
+void Engine::host_tables(HostTables *h) {
+  const char *tiles = getenv("MPSW_STAGE_TILES"), *row = getenv("MPSW_ROWS");
+  const bool tiles_on = !(tiles && atoi(tiles) == 0) && (size_t)nC * 1200 <= kTilesL2;
   const int share = std::max(8, (nC + 147) / 148);
-  StageSetHost t;
-  if (!build_stage_tiles(bm, share < 60 ? share : 128, &t).empty()) return;
+  in_turns(3, [&](int i) {
+    if (i == 0) h->stage_ok = tiles_on && build_stage_tiles(bm, share < 60 ? share : 128, &h->stage).empty();
+    if (i == 1) h->adjoint_ok = tiles_on && build_stage_ad_tiles(bm, share < 60 ? share : 96, &h->adjoint).empty();
+    if (i == 2) h->rows_ok = !(row && atoi(row) == 0) && build_rows(bm, &h->rows).empty();
+  });
+}
+
+void Engine::build_stage(const HostTables &h) {
+  st64 = st32 = st_ad = StageDev();
+  if (!h.stage_ok) return;
+  const StageSetHost &t = h.stage;
   const int *cnt = up<int>(t.cnt, mesh_bufs);
   for (int p = 0; p < 2; p++) {
     const std::vector<unsigned char> &blob = p ? t.blob32 : t.blob64;
-    if (blob.size() > kL2) continue;
+    if (blob.size() > kTilesL2) continue;
     StageDev &d = p ? st32 : st64;
     d.ntiles = t.ntiles;
     d.cnt = cnt;
     d.blob_off = up<long long>(p ? t.off32 : t.off64, mesh_bufs);
     d.blob = up<unsigned char>(blob, mesh_bufs);
   }
-  if (st64.ntiles && build_stage_ad_tiles(bm, share < 60 ? share : 96, &t).empty() && t.blob64.size() <= kL2) {
-    st_ad.ntiles = t.ntiles;
-    st_ad.cnt = up<int>(t.cnt, mesh_bufs);
-    st_ad.blob_off = up<long long>(t.off64, mesh_bufs);
-    st_ad.blob = up<unsigned char>(t.blob64, mesh_bufs);
+  if (st64.ntiles && h.adjoint_ok && h.adjoint.blob64.size() <= kTilesL2) {
+    st_ad.ntiles = h.adjoint.ntiles;
+    st_ad.cnt = up<int>(h.adjoint.cnt, mesh_bufs);
+    st_ad.blob_off = up<long long>(h.adjoint.off64, mesh_bufs);
+    st_ad.blob = up<unsigned char>(h.adjoint.blob64, mesh_bufs);
   }
   cuda_check(Launch<double, double>::stage_prepare(), "nonlinear stage shared-memory limit");
   cuda_check(Launch<float, double>::stage_prepare(), "nonlinear stage shared-memory limit");
@@ -560,11 +575,10 @@ void Engine::build_stage() {
 
 // Tables of the FP32 member-row passes, for meshes whose lists are those of a closed hexagon /
 // pentagon mesh (MPSW_ROWS=0: none, the members then take the general passes).
-void Engine::build_row_tables() {
+void Engine::build_row_tables(const HostTables &tables) {
   rows = RowTab();
-  const char *off = getenv("MPSW_ROWS");
-  RowTabHost h;
-  if ((off && atoi(off) == 0) || !build_rows(bm, &h).empty()) return;
+  if (!tables.rows_ok) return;
+  const RowTabHost &h = tables.rows;
   auto &o = mesh_bufs;
   rows.c_nb = up<int>(h.c_nb, o); rows.c_sp = up<int>(h.c_sp, o); rows.c_va = up<int>(h.c_va, o);
   rows.c_vb = up<int>(h.c_vb, o); rows.e_q = up<int>(h.e_q, o); rows.e_o1 = up<int>(h.e_o1, o);
@@ -644,8 +658,12 @@ void Engine::build_device_mesh() {
   d_perm[2] = up<int>(bm.perm_v, mesh_bufs);
   cuda_check(cudaGetDevice(&mesh_device), "cudaGetDevice");
   build_fused();
-  build_stage();
-  build_row_tables();
+  {
+    HostTables h;
+    host_tables(&h);
+    build_stage(h);
+    build_row_tables(h);
+  }
   noalloc_prepare_device();
   mesh_built = true;
   mesh_dirty = false;

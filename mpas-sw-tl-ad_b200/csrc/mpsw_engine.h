@@ -137,9 +137,15 @@ struct Engine {
   void build_fused();
   StageDev st64, st32;         // halo tiles of the nonlinear stage, FP64 and FP32 stencils
   StageDev st_ad;              // tiles of the FP64 adjoint stage
-  void build_stage();
+  struct HostTables {
+    StageSetHost stage, adjoint;
+    RowTabHost rows;
+    bool stage_ok = false, adjoint_ok = false, rows_ok = false;
+  };
+  void host_tables(HostTables *h);
+  void build_stage(const HostTables &h);
   RowTab rows;                 // tables of the FP32 member-row passes
-  void build_row_tables();
+  void build_row_tables(const HostTables &h);
   bool beside_members = false; // the nonlinear stages being launched run beside member kernels
 
   // work

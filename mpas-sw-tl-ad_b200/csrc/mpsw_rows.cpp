@@ -2,8 +2,23 @@
 #include "mpsw_rows.h"
 
 #include "mpsw_internal.h"
+#include "mpsw_parts.h"
 
 namespace mpsw {
+
+// one(i) for 0 <= i < n over a few threads: null, or what the mesh lacks
+template <class One>
+static std::string side_by_side(int n, One &&one) {
+  constexpr int kParts = 16;
+  const char *bad[kParts] = {};
+  in_turns(kParts, [&](int p) {
+    const int end = (int)((long long)n * (p + 1) / kParts);
+    for (int i = (int)((long long)n * p / kParts); i < end && !bad[p]; i++) bad[p] = one(i);
+  });
+  for (const char *b : bad)
+    if (b) return b;
+  return "";
+}
 
 std::string build_rows(const BuiltMesh &m, RowTabHost *t) {
   const int nC = m.nC, nE = m.nE, nV = m.nV;
@@ -37,7 +52,7 @@ std::string build_rows(const BuiltMesh &m, RowTabHost *t) {
                   &t->c_kb, &t->c_kk, &t->c_r2, &t->c_r3})
     x->assign(S, 0.0);
   t->c_ra.resize(nC);
-  for (int c = 0; c < nC; c++) {
+  std::string bad = side_by_side(nC, [&](int c) -> const char * {
     const double area = m.c_area[c];
     t->c_ra[c] = 1.0 / area;
     for (int k = 0; k < m.c_n[c]; k++) {
@@ -87,7 +102,9 @@ std::string build_rows(const BuiltMesh &m, RowTabHost *t) {
       for (int j = 0; j < m.c_n[c]; j++) found += m.c_vs[C(c, j)] == t->c_va[C(c, k)] || m.c_vs[C(c, j)] == t->c_vb[C(c, k)];
       if (found != 2) return "a cell whose edges and vertices do not alternate";
     }
-  }
+    return nullptr;
+  });
+  if (!bad.empty()) return bad;
   for (auto *x : {&t->e_q, &t->e_o1, &t->e_o2}) x->assign(nE, 0);
   for (auto *x : {&t->e_d, &t->e_r4}) x->assign((size_t)4 * nE, 0.0);
   t->e_k.assign((size_t)6 * nE, 0.0);
@@ -95,7 +112,7 @@ std::string build_rows(const BuiltMesh &m, RowTabHost *t) {
   t->e_t.assign((size_t)4 * nE, 0);
   for (auto *x : {&t->e_i1, &t->e_i2, &t->e_lap0}) x->assign(nE, 0.0);
   for (auto *x : {&t->e_ke, &t->e_lap}) x->assign((size_t)10 * nE, 0.0);
-  for (int e = 0; e < nE; e++) {
+  return side_by_side(nE, [&](int e) -> const char * {
     const int c1 = m.e_c1[e], c2 = m.e_c2[e];
     const double dc = m.e_dc[e], dv = m.e_dv[e];
     t->e_lap0[e] = (sign_c(c2, e) * dv / m.c_area[c2] - sign_c(c1, e) * dv / m.c_area[c1]) / dc -
@@ -159,8 +176,8 @@ std::string build_rows(const BuiltMesh &m, RowTabHost *t) {
       for (int j = 0; j < i; j++)
         if (((q >> (8 * i)) & 0xFF) == ((q >> (8 * j)) & 0xFF)) return "two edges between the same vertices";
     t->e_q[e] = (int)q;
-  }
-  return "";
+    return nullptr;
+  });
 }
 
 }  // namespace mpsw

@@ -5,6 +5,8 @@
 #include <cstring>
 #include <sstream>
 
+#include "mpsw_parts.h"
+
 namespace mpsw {
 namespace {
 
@@ -506,39 +508,93 @@ void stage_pack(const Builder &b, const BuiltMesh &m, const Space &E, const Spac
   std::memcpy(p + off[SB_GV], V.list.data(), 4 * (size_t)nv);
 }
 
-}  // namespace
+// Cut the cells into runs and append one tile a run: one(b, stamp, c0, K, out) appends the tile of cells
+// [c0, c0 + K) and returns null, or kTooLarge, or what keeps the mesh from being tiled.  A run that is
+// too large is cut by 1 / shrink until it fits; neighbouring runs fit at like sizes, so the next one starts
+// three sizes above the last.  Four parts of the cells, whole multiples of kmax, are cut side by side (level 6,
+// both sets of tiles, eight cores: 865 -> 350 ms).
+const char *const kTooLarge = "one cell's halo exceeds a tile";
 
-std::string build_stage_tiles(const BuiltMesh &m, int kmax, StageSetHost *o) {
-  if (kmax < 1) return "tile size must be positive";
+template <class One>
+std::string build_runs(const BuiltMesh &m, int kmax, int shrink, StageSetHost *o, One &&one) {
+  std::vector<int> sizes(1, kmax);
+  while (sizes.back() > 1) {
+    const int K = sizes.back();
+    sizes.push_back(std::max(1, K - (K + shrink - 1) / shrink));
+  }
+  const int tiles = (m.nC + kmax - 1) / kmax, parts = std::min(tiles, 4), len = (tiles + parts - 1) / parts * kmax;
+  std::vector<StageSetHost> set(parts);
+  std::vector<std::string> err(parts);
+  auto cut = [&](int p) {
+    Builder b(m);
+    StageSetHost &out = set[p];
+    const int end = (int)std::min<long long>(m.nC, (long long)(p + 1) * len);
+    size_t at = 0;
+    int stamp = 0;
+    for (int c0 = p * len; c0 < end;) {
+      const int left = end - c0;
+      at -= std::min<size_t>(at, 3);
+      while (at + 1 < sizes.size() && sizes[at + 1] >= left) at++;  // (sizes beyond what is left are one)
+      const char *why;
+      while ((why = one(b, stamp++, c0, std::min(sizes[at], left), &out)) == kTooLarge && at + 1 < sizes.size()) at++;
+      if (why) {
+        err[p] = why == kTooLarge ? why : fail(out.ntiles, why);
+        return;
+      }
+      out.ntiles++;
+      c0 += std::min(sizes[at], left);
+    }
+  };
+  in_turns(parts, cut);
+  *o = StageSetHost();
+  for (const std::string &e : err)
+    if (!e.empty()) return e;
+  size_t n64 = 0, n32 = 0;
+  for (const StageSetHost &t : set) {
+    n64 += t.blob64.size();
+    n32 += t.blob32.size();
+  }
+  o->blob64.reserve(n64);
+  o->blob32.reserve(n32);
+  for (StageSetHost &t : set) {
+    for (long long x : t.off64) o->off64.push_back(x + (long long)o->blob64.size());
+    for (long long x : t.off32) o->off32.push_back(x + (long long)o->blob32.size());
+    o->cnt.insert(o->cnt.end(), t.cnt.begin(), t.cnt.end());
+    o->blob64.insert(o->blob64.end(), t.blob64.begin(), t.blob64.end());
+    o->blob32.insert(o->blob32.end(), t.blob32.begin(), t.blob32.end());
+    o->ntiles += t.ntiles;
+    t = StageSetHost();
+  }
+  return "";
+}
+
+std::string narrow_lists(const BuiltMesh &m) {
   for (int c = 0; c < m.nC; c++)
     if (m.c_n[c] > kCellSlots) return "stage tiles need at most 6 edges per cell";
   for (int e = 0; e < m.nE; e++)
     if (m.e_n[e] > kEoeSlots) return "stage tiles need at most 10 edgesOnEdge";
-  Builder b(m);
-  *o = StageSetHost();
-  int stamp = 0;
-  for (int c0 = 0; c0 < m.nC;) {
-    int K = std::min(kmax, m.nC - c0), n[kStageCounts];
-    for (;; K = std::max(1, K - (K + 4) / 5)) {  // shorten the run while its halo is too large
-      Space E(b.se, b.le, stamp), C(b.sc, b.lc, stamp), V(b.sv, b.lv, stamp);
-      stamp++;
-      stage_spaces(b, m, c0, c0 + K, E, C, V, n);
-      if (!stage_fits(n)) {
-        if (K == 1) return "one cell's halo exceeds a tile";
-        continue;
-      }
-      if (!stage_valid(b, m, E, C, V, n)) return fail(o->ntiles, "a phase of the stage would read outside its tile");
-      o->cnt.insert(o->cnt.end(), n, n + kStageCounts);
-      o->off64.push_back((long long)o->blob64.size());
-      o->off32.push_back((long long)o->blob32.size());
-      stage_pack<double>(b, m, E, C, V, n, &o->blob64);
-      stage_pack<float>(b, m, E, C, V, n, &o->blob32);
-      break;
-    }
-    o->ntiles++;
-    c0 += K;
-  }
   return "";
+}
+
+}  // namespace
+
+std::string build_stage_tiles(const BuiltMesh &m, int kmax, StageSetHost *o) {
+  if (kmax < 1) return "tile size must be positive";
+  const std::string wide = narrow_lists(m);
+  if (!wide.empty()) return wide;
+  return build_runs(m, kmax, 5, o, [&](Builder &b, int stamp, int c0, int K, StageSetHost *out) -> const char * {
+    int n[kStageCounts];
+    Space E(b.se, b.le, stamp), C(b.sc, b.lc, stamp), V(b.sv, b.lv, stamp);
+    stage_spaces(b, m, c0, c0 + K, E, C, V, n);
+    if (!stage_fits(n)) return kTooLarge;
+    if (!stage_valid(b, m, E, C, V, n)) return "a phase of the stage would read outside its tile";
+    out->cnt.insert(out->cnt.end(), n, n + kStageCounts);
+    out->off64.push_back((long long)out->blob64.size());
+    out->off32.push_back((long long)out->blob32.size());
+    stage_pack<double>(b, m, E, C, V, n, &out->blob64);
+    stage_pack<float>(b, m, E, C, V, n, &out->blob32);
+    return nullptr;
+  });
 }
 
 // ---- tiles of the FP64 adjoint stage (mpsw_stage.h) -----------------------------------------------
@@ -609,33 +665,19 @@ void stage_ad_pack(const Builder &b, const BuiltMesh &m, const Space &E, const S
 
 std::string build_stage_ad_tiles(const BuiltMesh &m, int kmax, StageSetHost *o) {
   if (kmax < 1) return "tile size must be positive";
-  for (int c = 0; c < m.nC; c++)
-    if (m.c_n[c] > kCellSlots) return "stage tiles need at most 6 edges per cell";
-  for (int e = 0; e < m.nE; e++)
-    if (m.e_n[e] > kEoeSlots) return "stage tiles need at most 10 edgesOnEdge";
-  Builder b(m);
-  *o = StageSetHost();
-  int stamp = 0;
-  for (int c0 = 0; c0 < m.nC;) {
-    int K = std::min(kmax, m.nC - c0), n[kTileCounts];
-    for (;; K = std::max(1, K - (K + 7) / 8)) {  // shorten the run while its halo is too large
-      Space E(b.se, b.le, stamp), C(b.sc, b.lc, stamp), V(b.sv, b.lv, stamp);
-      stamp++;
-      tile_spaces(b, m, c0, c0 + K, true, E, C, V, n);
-      if (!stage_ad_fits(n)) {
-        if (K == 1) return "one cell's halo exceeds a tile";
-        continue;
-      }
-      if (!validate(b, m, E, C, V, n, true)) return fail(o->ntiles, "a phase of the stage would read outside its tile");
-      o->cnt.insert(o->cnt.end(), n, n + kTileCounts);
-      o->off64.push_back((long long)o->blob64.size());
-      stage_ad_pack(b, m, E, C, V, n, &o->blob64);
-      break;
-    }
-    o->ntiles++;
-    c0 += K;
-  }
-  return "";
+  const std::string wide = narrow_lists(m);
+  if (!wide.empty()) return wide;
+  return build_runs(m, kmax, 8, o, [&](Builder &b, int stamp, int c0, int K, StageSetHost *out) -> const char * {
+    int n[kTileCounts];
+    Space E(b.se, b.le, stamp), C(b.sc, b.lc, stamp), V(b.sv, b.lv, stamp);
+    tile_spaces(b, m, c0, c0 + K, true, E, C, V, n);
+    if (!stage_ad_fits(n)) return kTooLarge;
+    if (!validate(b, m, E, C, V, n, true)) return "a phase of the stage would read outside its tile";
+    out->cnt.insert(out->cnt.end(), n, n + kTileCounts);
+    out->off64.push_back((long long)out->blob64.size());
+    stage_ad_pack(b, m, E, C, V, n, &out->blob64);
+    return nullptr;
+  });
 }
 
 }  // namespace mpsw
