@@ -80,6 +80,7 @@ struct Window {
   // member buffers per precision (0 FP64, 1 FP32), allocated for the largest B seen
   struct Members {
     int B = 0;
+    int short_of = 0;  // a padded count that memory did not suffice for
     std::vector<void *> mem;
     void *bufs = nullptr;  // MemberBufs<R>
     double *acc_u = nullptr, *acc_h = nullptr;

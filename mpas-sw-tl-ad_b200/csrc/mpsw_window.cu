@@ -86,6 +86,7 @@ MemberBufs<R> *members(Engine &E, int prec, int B, cudaStream_t s) {
   E.graphs_free();  // captured steps point at the buffers about to be replaced
   free_members<R>(M);
   auto *mb = new MemberBufs<R>();
+  M.bufs = mb;  // (with B 0: freed by the next call should an allocation fail)
   const size_t C = (size_t)E.nC * B, Ed = (size_t)E.nE * B, V = (size_t)E.nV * B;
   Diag<R> &d = mb->d;
   d.circ = nullptr;
@@ -120,9 +121,26 @@ MemberBufs<R> *members(Engine &E, int prec, int B, cudaStream_t s) {
   M.acc_h = walloc<double>(M, C, s);
   M.x_u = walloc<double>(M, Ed, s);
   M.x_h = walloc<double>(M, C, s);
-  M.bufs = mb;
   M.B = B;
   return mb;
+}
+
+// The count that a sweep of B members runs with: padded, or as given where memory for the padding is short.
+template <typename R>
+int sweep_members(Engine &E, int prec, int B) {
+  const int Bp = padded_members(prec, B);
+  const Window::Members &M = E.win.ms[prec];
+  int &short_of = E.win.ms[prec].short_of;
+  if (Bp == B || (short_of && Bp >= short_of && M.B < Bp)) return B;
+  try {
+    members<R>(E, prec, Bp, E.stream);
+    return Bp;
+  } catch (const EngineError &) {
+    (void)cudaGetLastError();
+    free_members<R>(E.win.ms[prec]);
+    short_of = Bp;
+    return B;
+  }
 }
 
 // The member rows a window sweep passes between its kernels.  divergence' and vorticity' feed
@@ -221,6 +239,7 @@ void Engine::window_free() {
   graphs_free();
   free_members<double>(W.ms[0]);
   free_members<float>(W.ms[1]);
+  W.ms[0].short_of = W.ms[1].short_of = 0;
   window_free_trajectory();
 }
 
@@ -673,8 +692,7 @@ static bool passes_between(int prec, int B, const Phys<double> &ph) {
 }
 
 template <typename R>
-static void window_tl_impl(Engine &E, int prec, int Bu, double *user_u, double *user_h) {
-  const int B = padded_members(prec, Bu);
+static void window_tl_impl(Engine &E, int prec, int B, int Bu, double *user_u, double *user_h) {
   Window &W = E.win;
   MemberBufs<R> *mb = members<R>(E, prec, B, E.stream);
   double *du = W.ms[prec].x_u, *dh = W.ms[prec].x_h;
@@ -798,8 +816,7 @@ static void ad_member_step(Engine &E, int prec, int B, double *au, double *ah, M
 }
 
 template <typename R>
-static void window_ad_impl(Engine &E, int prec, int Bu, double *user_u, double *user_h) {
-  const int B = padded_members(prec, Bu);
+static void window_ad_impl(Engine &E, int prec, int B, int Bu, double *user_u, double *user_h) {
   Window &W = E.win;
   MemberBufs<R> *mb = members<R>(E, prec, B, E.stream);
   double *au = W.ms[prec].x_u, *ah = W.ms[prec].x_h;
@@ -923,10 +940,11 @@ void Engine::window_tl(int prec, int B, double *du, double *dh, cudaStream_t s) 
   if (mesh_dirty) throw EngineError(MPSW_ERR_STATE, "mesh changed since mpsw_window_init");
   if (prec != 0 && prec != 1) throw EngineError(MPSW_ERR_ARG, "precision must be 0 or 1");
   join(s, stream, true);
-  TuneScope scope(tuning(prec, padded_members(prec, B)));
+  const int Bp = prec == 0 ? sweep_members<double>(*this, prec, B) : sweep_members<float>(*this, prec, B);
+  TuneScope scope(tuning(prec, Bp));
   nonfinite_clear();  // after the autotuner, whose timings run on arbitrary buffer contents
-  if (prec == 0) window_tl_impl<double>(*this, prec, B, du, dh);
-  else window_tl_impl<float>(*this, prec, B, du, dh);
+  if (prec == 0) window_tl_impl<double>(*this, prec, Bp, B, du, dh);
+  else window_tl_impl<float>(*this, prec, Bp, B, du, dh);
   nonfinite_check("window_tl");
   join(s, stream, false);
 }
@@ -938,10 +956,11 @@ void Engine::window_ad(int prec, int B, double *au, double *ah, cudaStream_t s) 
   if (prec != 0 && prec != 1) throw EngineError(MPSW_ERR_ARG, "precision must be 0 or 1");
   join(s, stream, true);
   window_ensure(prec);
-  TuneScope scope(tuning(prec, padded_members(prec, B)));
+  const int Bp = prec == 0 ? sweep_members<double>(*this, prec, B) : sweep_members<float>(*this, prec, B);
+  TuneScope scope(tuning(prec, Bp));
   nonfinite_clear();  // after the autotuner, whose timings run on arbitrary buffer contents
-  if (prec == 0) window_ad_impl<double>(*this, prec, B, au, ah);
-  else window_ad_impl<float>(*this, prec, B, au, ah);
+  if (prec == 0) window_ad_impl<double>(*this, prec, Bp, B, au, ah);
+  else window_ad_impl<float>(*this, prec, Bp, B, au, ah);
   nonfinite_check("window_ad");
   join(s, stream, false);
 }
@@ -1142,6 +1161,14 @@ template <typename R>
 static TuneTable tune_members(Engine &E, int prec, int B) {
   TuneTable best{};
   const Phys<R> ph = phys_as<R>(E.phys());
+  // rows that do not fit L2 are timed as a sweep meets them, with the kernel's inputs evicted
+  bool cold = (size_t)E.nE * B * sizeof(R) * 4 > ((size_t)126 << 20);
+  if (cold) try {
+      E.l2_flush_buffer();
+    } catch (const EngineError &) {  // no memory to spare for it
+      (void)cudaGetLastError();
+      cold = false;
+    }
   const int vs[] = {1, 2, 4, 8}, blocks[] = {64, 128, 256};
   for (int k = 0; k < K_TUNED; k++) {
     if constexpr (sizeof(R) == 8)  // passes that the sweeps do not run
@@ -1155,8 +1182,6 @@ static TuneTable tune_members(Engine &E, int prec, int B) {
         trial.k[k].v = v;
         trial.k[k].block = bl;
         TuneScope scope(&trial);
-        // rows that do not fit L2 are timed as a sweep meets them, with the kernel's inputs evicted
-        const bool cold = (size_t)E.nE * B * sizeof(R) * 4 > ((size_t)126 << 20);
         const double t = std::min(time_kernel_impl<R>(E, k, prec, B, cold ? 3 : 8, cold),
                                   time_kernel_impl<R>(E, k, prec, B, cold ? 3 : 8, cold));
         if (t < tbest) {
@@ -1239,7 +1264,12 @@ const TuneTable *Engine::tuning(int prec, int B) {
   const std::string key = tune_key(*this, prec, B);
   TuneTable t{};
   if (!(cache && *cache && tune_cache_read(cache, key, &t))) {
+    const bool held = l2_flush;
     t = prec == 1 ? tune_members<float>(*this, prec, B) : tune_members<double>(*this, prec, B);
+    if (!held && l2_flush) {
+      cudaFree(l2_flush);
+      l2_flush = nullptr;
+    }
     if (cache && *cache) tune_cache_append(cache, key, t);
   }
   graphs_free();  // nothing captured before this point may keep the untuned choices
