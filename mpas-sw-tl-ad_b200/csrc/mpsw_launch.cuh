@@ -519,12 +519,12 @@ void Launch<R, A>::ad_fused(const FusedDev &f, int M, const MeshDev<R> &m, int B
   }
 }
 // ---- member-row passes ---------------------------------------------------------------------------
-// Forming the coefficients costs the same for any member count, so few members take the general
-// passes.  ms a sweep pair (8 steps; level 6: 6 steps), row passes against general ones: 64 members
-// level 4 1.48 / 2.23, level 5 2.7 / 3.1, level 6 8.7 / 10.0; 24 members level 5 2.09 / 2.47, level 6
-// 5.03 / 5.21; 16 members level 4 1.25 / 1.30, level 5 1.89 / 2.11, but level 6 3.98 / 3.88 and its
-// adjoint with recomputed stages, where nothing hides the staging, 14.3 / 13.2; 8 members level 5
-// 1.94 / 1.75.
+// Forming the coefficients costs the same for any member count, so few members take the general passes.
+// ms a tangent-linear / adjoint sweep (6 steps), row passes against general ones.  Stored stages, 24 members: level 4
+// 0.31 / 0.32 against 0.36 / 0.42, level 6 1.99 / 2.20 against 2.12 / 2.26; 16 members: level 4 0.33 / 0.37
+// against 0.31 / 0.39, level 5 0.58 / 0.52 against 0.60 / 0.60, level 6 a pair of sweeps 3.98 against 3.88.  Recomputed
+// stages, which hide no staging, 24 members: level 6 2.99 / 3.45 against 3.19 / 3.40, level 7 (2 steps) 3.44 / 3.91
+// against 3.58 / 3.96; 16 members: level 4 0.62 / 0.79 against 0.56 / 0.79, level 5 1.04 / 1.10 against 1.00 / 1.25.
 template <typename R, typename A>
 bool Launch<R, A>::rows_ok(const RowTab &t, int nE, int B, const Phys<R> &ph, bool adjoint) {
   if (!std::is_same<R, float>::value || !t.ok || B % 4 || B > 512 || !stage_enabled()) return false;

@@ -128,8 +128,6 @@ std::string build_rows(const BuiltMesh &m, RowTabHost *t) {
       const double to = in1 ? -1.0 : 1.0;  // the side c takes in the edge's gradients
       t->e_ke[E(e, j)] = sign_c(c, x) / (m.e_dc[x] * m.c_area[c]);
       double lap = to * sign_c(c, x) * m.e_dv[x] / m.c_area[c] / dc;
-      // the edge's weight in delsq_u of x: the cell's side there, and its divergence weight
-      const double to_x = m.e_c2[x] == c ? 1.0 : -1.0;
       for (int k = 0; k < 2; k++) {
         const int v = k ? m.e_v2[e] : m.e_v1[e];
         if (!of_vertex(v, x)) continue;

@@ -160,30 +160,30 @@ __global__ void __maxnreg__(VISC ? 72 : 48) k_row_tl_edge(MeshDev<float> m, RowT
     }
     const int e = e0 + th.le;
     if (e < nE) {
-    const size_t o = (size_t)e * B + b;
-    const M u = ldv<V>(ut + o);
-    const float4 x = own[3 * th.le], y = own[3 * th.le + 1], z = own[3 * th.le + 2];
-    const M h1 = ldv<V>(ht + (size_t)as_i(x.x) * B + b), h2 = ldv<V>(ht + (size_t)as_i(x.y) * B + b);
-    M p = y.x * u, f = z.z * u;
-    row_add(p, y.y, h1);
-    row_add(p, y.z, h2);
-    row_add(f, z.w, h1);
-    row_add(f, z.w, h2);
-    row_add(p, y.w, ldv<V>(ht + (size_t)as_i(x.z) * B + b));
-    row_add(p, z.x, ldv<V>(ht + (size_t)as_i(x.w) * B + b));
-    row_add(p, z.y, ldv<V>(pc + (size_t)as_i(x.y) * B + b) - ldv<V>(pc + (size_t)as_i(x.x) * B + b));
-    M d = mv_fill<float, V>(0.f);
-    if (VISC) d = t.e_lap0[e] * u;
+      const size_t o = (size_t)e * B + b;
+      const M u = ldv<V>(ut + o);
+      const float4 x = own[3 * th.le], y = own[3 * th.le + 1], z = own[3 * th.le + 2];
+      const M h1 = ldv<V>(ht + (size_t)as_i(x.x) * B + b), h2 = ldv<V>(ht + (size_t)as_i(x.y) * B + b);
+      M p = y.x * u, f = z.z * u;
+      row_add(p, y.y, h1);
+      row_add(p, y.z, h2);
+      row_add(f, z.w, h1);
+      row_add(f, z.w, h2);
+      row_add(p, y.w, ldv<V>(ht + (size_t)as_i(x.z) * B + b));
+      row_add(p, z.x, ldv<V>(ht + (size_t)as_i(x.w) * B + b));
+      row_add(p, z.y, ldv<V>(pc + (size_t)as_i(x.y) * B + b) - ldv<V>(pc + (size_t)as_i(x.x) * B + b));
+      M d = mv_fill<float, V>(0.f);
+      if (VISC) d = t.e_lap0[e] * u;
 #pragma unroll
-    for (int j = 0; j < 10; j++) {
-      const float2 c = slot[th.le * 10 + j];
-      const M un = ldv<V>(ut + (size_t)as_i(c.x) * B + b);
-      row_add(p, c.y, un);
-      if (VISC) row_add(d, t.e_lap[(size_t)j * nE + e], un);
-    }
-    stv<V>(pe + o, p);
-    stv<V>(flux + o, f);
-    if (VISC) stv<V>(dsq + o, d);
+      for (int j = 0; j < 10; j++) {
+        const float2 c = slot[th.le * 10 + j];
+        const M un = ldv<V>(ut + (size_t)as_i(c.x) * B + b);
+        row_add(p, c.y, un);
+        if (VISC) row_add(d, t.e_lap[(size_t)j * nE + e], un);
+      }
+      stv<V>(pe + o, p);
+      stv<V>(flux + o, f);
+      if (VISC) stv<V>(dsq + o, d);
     }
     __syncthreads();
   }
@@ -229,54 +229,54 @@ __global__ void __maxnreg__(GEN ? 72 : 48) k_row_tl_tend(MeshDev<float> m, int B
     }
     const int e = e0 + th.le;
     if (e < nE) {
-    const size_t o = (size_t)e * B + b;
-    const int c1 = m.e_c1[e], c2 = m.e_c2[e];
-    const float rdc = 1.f / m.e_dc[e];
-    M q = mv_fill<float, V>(0.f);
-    float own = 0.f;
+      const size_t o = (size_t)e * B + b;
+      const int c1 = m.e_c1[e], c2 = m.e_c2[e];
+      const float rdc = 1.f / m.e_dc[e];
+      M q = mv_fill<float, V>(0.f);
+      float own = 0.f;
 #pragma unroll
-    for (int j = 0; j < 10; j++) {
-      const int i = j * th.epb + th.le;
-      const size_t on = (size_t)nbs[i] * B + b;
-      const float2 c = co[i];
-      M x = c.x * ldv<V>(flux + on);
-      row_add(x, c.y, ldv<V>(d.pe + on));
-      q = q + x;
-      own += c.y;
-    }
-    row_add(q, own, ldv<V>(d.pe + o));
-    const M h1 = ldv<V>(ht + (size_t)c1 * B + b), h2 = ldv<V>(ht + (size_t)c2 * B + b);
-    M grad = ldv<V>(d.ke + (size_t)c2 * B + b) - ldv<V>(d.ke + (size_t)c1 * B + b);
-    row_add(grad, float(GRAVITY), h2 - h1);
-    row_add(q, -rdc, grad);
-    if (GEN) {
-      if (ph.visc2 > 0.f) row_add(q, m.e_sc2[e] * ph.visc2, ldv<V>(d.dsq_u + o));
-      if (ph.visc4 > 0.f) {
-        const int v1 = m.e_v1[e], v2 = m.e_v2[e];
-        const float k = m.e_sc4[e] * ph.visc4, kv = k / m.e_dv[e], kc = k * rdc;
-        row_add(q, -kc, ldv<V>(d.dsq_div + (size_t)c2 * B + b) - ldv<V>(d.dsq_div + (size_t)c1 * B + b));
-        row_add(q, kv, ldv<V>(d.dsq_vort + (size_t)v2 * B + b) - ldv<V>(d.dsq_vort + (size_t)v1 * B + b));
+      for (int j = 0; j < 10; j++) {
+        const int i = j * th.epb + th.le;
+        const size_t on = (size_t)nbs[i] * B + b;
+        const float2 c = co[i];
+        M x = c.x * ldv<V>(flux + on);
+        row_add(x, c.y, ldv<V>(d.pe + on));
+        q = q + x;
+        own += c.y;
       }
-      if (ph.wind || ph.drag) {
-        const float hh = bs.he[e];
-        float k = ph.wind ? -(m.e_usrc[e] / float(RHO_REF)) / (hh * hh) : 0.f;
-        if (ph.drag) {
-          const float uu = bs.u[e], sq = sqrtf(bs.ke[c1] + bs.ke[c2]);
-          k += ((1.0e-3f * uu) * sq) / (hh * hh);
-          row_add(q, -(1.0e-3f * sq) / hh, ldv<V>(ut + o));
-          const float kk = -(((0.5f * 1.0e-3f) * uu) / sq) / hh;
-          row_add(q, kk, ldv<V>(d.ke + (size_t)c1 * B + b));
-          row_add(q, kk, ldv<V>(d.ke + (size_t)c2 * B + b));
+      row_add(q, own, ldv<V>(d.pe + o));
+      const M h1 = ldv<V>(ht + (size_t)c1 * B + b), h2 = ldv<V>(ht + (size_t)c2 * B + b);
+      M grad = ldv<V>(d.ke + (size_t)c2 * B + b) - ldv<V>(d.ke + (size_t)c1 * B + b);
+      row_add(grad, float(GRAVITY), h2 - h1);
+      row_add(q, -rdc, grad);
+      if (GEN) {
+        if (ph.visc2 > 0.f) row_add(q, m.e_sc2[e] * ph.visc2, ldv<V>(d.dsq_u + o));
+        if (ph.visc4 > 0.f) {
+          const int v1 = m.e_v1[e], v2 = m.e_v2[e];
+          const float k = m.e_sc4[e] * ph.visc4, kv = k / m.e_dv[e], kc = k * rdc;
+          row_add(q, -kc, ldv<V>(d.dsq_div + (size_t)c2 * B + b) - ldv<V>(d.dsq_div + (size_t)c1 * B + b));
+          row_add(q, kv, ldv<V>(d.dsq_vort + (size_t)v2 * B + b) - ldv<V>(d.dsq_vort + (size_t)v1 * B + b));
         }
-        row_add(q, 0.5f * k, h1);
-        row_add(q, 0.5f * k, h2);
+        if (ph.wind || ph.drag) {
+          const float hh = bs.he[e];
+          float k = ph.wind ? -(m.e_usrc[e] / float(RHO_REF)) / (hh * hh) : 0.f;
+          if (ph.drag) {
+            const float uu = bs.u[e], sq = sqrtf(bs.ke[c1] + bs.ke[c2]);
+            k += ((1.0e-3f * uu) * sq) / (hh * hh);
+            row_add(q, -(1.0e-3f * sq) / hh, ldv<V>(ut + o));
+            const float kk = -(((0.5f * 1.0e-3f) * uu) / sq) / hh;
+            row_add(q, kk, ldv<V>(d.ke + (size_t)c1 * B + b));
+            row_add(q, kk, ldv<V>(d.ke + (size_t)c2 * B + b));
+          }
+          row_add(q, 0.5f * k, h1);
+          row_add(q, 0.5f * k, h2);
+        }
       }
-    }
-    if (ph.bad) {
+      if (ph.bad) {
 #pragma unroll
-      for (int i = 0; i < V; i++) flag_nonfinite(ph.bad, q.x[i]);
-    }
-    rk_members<float, double, V>(rk, o, q);
+        for (int i = 0; i < V; i++) flag_nonfinite(ph.bad, q.x[i]);
+      }
+      rk_members<float, double, V>(rk, o, q);
     }
     __syncthreads();
   }
