@@ -8,10 +8,10 @@
 // three kernels instead of four.  Coefficients are formed once a block in shared memory, before the
 // wait for the previous kernel where the linearisation point is a stored one, and shared by the
 // B / V threads of an entity; a thread holds V members.  The edge passes give a block two
-// neighbouring tiles of edges (the second finds rows of the first in L1: tendency pass 236 -> 214 us),
+// neighbouring tiles of edges (the second finds rows of the first in L1: tendency pass 236 -> 214 us when it was measured, without the h' rows),
 // and each kernel is held to the registers at which occupancy and the rows a thread keeps in flight
-// balance.  Level 7, 64 members, cold, us: cells 107, edges 212, tendencies 227 (a tangent-linear stage
-// 529, through the fields 634); edges 189, cells 109, final 249 (adjoint 526, through the fields 671).
+// balance.  Level 7, 64 members, cold, us: cells 107, edges 211, tendencies 223 (a tangent-linear stage
+// 524, through the fields 634); edges 189, cells 109, final 249 (adjoint 526, through the fields 671).
 #pragma once
 
 #include "mpsw_members.cuh"
@@ -192,10 +192,12 @@ __global__ void __maxnreg__(VISC ? 72 : 48) k_row_tl_edge(MeshDev<float> m, RowT
 // tend_u' and its RK update; GEN: any of viscosity, wind and drag.  The sums run so that they round no more
 // than the general pass does: a slot's two terms meet before they join the other slots', and the gradient,
 // most of the tendency, is formed from differences of rows and comes last.  Adding gravity to the ke row
-// and the gradient's halves to the sum first, without the two h' rows, took 215 instead of 227 us (level 7,
+// and the gradient's halves to the sum first, without the two h' rows, took 215 instead of 223 us (level 7,
 // 64 members) but left twice the error of a white-noise tendency and 4-12 times that of a smooth one.
+// 40 registers spill and still lead: us at 40 / 48 / 56 / 64, level 6 70 / 76 / 80 / 76, level 7 223 / 226 / 218 / 233,
+// a level-6 sweep of 12 steps 7.4 / 7.6 / 7.8 / 7.7 ms.
 template <int V, int GEN>
-__global__ void __maxnreg__(GEN ? 72 : 48) k_row_tl_tend(MeshDev<float> m, int B, Base<float> bs,
+__global__ void __maxnreg__(GEN ? 72 : 40) k_row_tl_tend(MeshDev<float> m, int B, Base<float> bs,
                                                      const float *__restrict__ ut, const float *__restrict__ ht,
                                                      Diag<float> d, const float *__restrict__ flux, Phys<float> ph,
                                                      RK<float, double> rk, int early) {
