@@ -62,11 +62,11 @@ int mpsw_var_info(mpsw_handle *h, const char *name, int *rank, long long dims[4]
 int mpsw_set_var(mpsw_handle *h, const char *name, const void *src, long long count);
 int mpsw_get_var(mpsw_handle *h, const char *name, void *dst, long long count);
 /* mpsw_set_var, skipped where the variable already holds src: src equals what was last exchanged for
- * it, and no routine has written it since.  mpsw_var_changed: whether src differs from what was last
- * exchanged, whatever routines have written since (has the caller edited its copy?).  mpsw_get_vars:
- * mpsw_get_var of n variables with one wait. */
+ * it, and no routine has written it since.  mpsw_edit_var: mpsw_set_var, skipped where src equals what
+ * was last exchanged, whatever routines have written since (the caller has not edited its copy, and
+ * newer values stand).  mpsw_get_vars: mpsw_get_var of n variables with one wait. */
 int mpsw_update_var(mpsw_handle *h, const char *name, const void *src, long long count);
-int mpsw_var_changed(mpsw_handle *h, const char *name, const void *src, long long count, int *changed);
+int mpsw_edit_var(mpsw_handle *h, const char *name, const void *src, long long count);
 int mpsw_get_vars(mpsw_handle *h, int n, const char *const *names, void *const *dst, const long long *counts);
 
 /* ---- module subroutines (src/mpas_sw_module.f90) -------------------------------------- */

@@ -358,23 +358,13 @@ static bool mirror_equals(const Var &v, const void *x) {
   return v.is_int ? same_bytes(v.hi.data(), x, sizeof(int) * v.count) : same_bytes(v.hr.data(), x, sizeof(double) * v.count);
 }
 
-bool Engine::var_changed(const char *name, const void *src, long long count) {
+void Engine::set_var(const char *name, const void *src, long long count, Send when) {
   Var &v = var(name);
   if (!v.allocated) throw EngineError(MPSW_ERR_STATE, std::string(name) + " is not allocated");
   if (count != v.count) throw EngineError(MPSW_ERR_ARG, std::string(name) + ": element count mismatch");
   if (!src && count) throw EngineError(MPSW_ERR_ARG, "null source buffer");
   copies_done();
-  return !mirror_equals(v, src);
-}
-
-void Engine::set_var(const char *name, const void *src, long long count, bool if_changed) {
-  Var &v = var(name);
-  if (!v.allocated) throw EngineError(MPSW_ERR_STATE, std::string(name) + " is not allocated");
-  if (count != v.count) throw EngineError(MPSW_ERR_ARG, std::string(name) + ": element count mismatch");
-  if (!src && count) throw EngineError(MPSW_ERR_ARG, "null source buffer");
-  copies_done();
-  // unchanged, and no routine has written a newer value on the device
-  if (if_changed && v.host_valid && mirror_equals(v, src)) return;
+  if ((when == Send::edited || (when == Send::differs && v.host_valid)) && mirror_equals(v, src)) return;
   if (v.is_int) {
     std::memcpy(v.hi.data(), src, sizeof(int) * count);
   } else {
@@ -1445,14 +1435,11 @@ int mpsw_set_var(mpsw_handle *h, const char *name, const void *src, long long co
 }
 
 int mpsw_update_var(mpsw_handle *h, const char *name, const void *src, long long count) {
-  return mpsw::guarded(h, [&](mpsw::Engine &e) { e.set_var(name, src, count, true); });
+  return mpsw::guarded(h, [&](mpsw::Engine &e) { e.set_var(name, src, count, mpsw::Send::differs); });
 }
 
-int mpsw_var_changed(mpsw_handle *h, const char *name, const void *src, long long count, int *changed) {
-  return mpsw::guarded(h, [&](mpsw::Engine &e) {
-    if (!changed) throw mpsw::EngineError(MPSW_ERR_ARG, "null output");
-    *changed = e.var_changed(name, src, count);
-  });
+int mpsw_edit_var(mpsw_handle *h, const char *name, const void *src, long long count) {
+  return mpsw::guarded(h, [&](mpsw::Engine &e) { e.set_var(name, src, count, mpsw::Send::edited); });
 }
 
 int mpsw_get_vars(mpsw_handle *h, int n, const char *const *names, void *const *dst, const long long *counts) {

@@ -27,6 +27,11 @@ struct EngineError : std::runtime_error {
 std::string lower(const char *s);
 void cuda_check(cudaError_t e, const char *what);
 
+// When a variable's contents are taken over: always; unless the variable holds them (they equal what was last
+// exchanged, and no routine has written a newer value on the device); or only where they differ from what was
+// last exchanged.
+enum class Send { always, differs, edited };
+
 struct Var {
   std::string name, dims_spec;
   int group = 0, is_int = 0, ent = 0, mesh = 0, lead = 1;
@@ -193,8 +198,7 @@ struct Engine {
   size_t d_transfer_n = 0;
   double *d_mean = nullptr;
   void download_start(Var &v);
-  void set_var(const char *name, const void *src, long long count, bool if_changed = false);
-  bool var_changed(const char *name, const void *src, long long count);
+  void set_var(const char *name, const void *src, long long count, Send when = Send::always);
   void get_vars(int n, const char *const *names, void *const *dst, const long long *counts);
   void get_var(const char *name, void *dst, long long count);
   void mark_written(Var &v, bool maybe_nonzero);

@@ -125,20 +125,14 @@ class MpasSwModule:
     def _push(self, key, force=False):
         d = self.__dict__
         arr = d['_arr'][key]
-        args = d['_canon'][key].encode(), ctypes.c_void_p(arr.ctypes.data), arr.size
         if force or key not in d['_synced']:
-            d['_h'].call('mpsw_set_var', *args)
-        elif key in d['_assigned']:
-            # set since the last routine: the engine's value, if a routine has written it, gives way
-            d['_h'].call('mpsw_update_var', *args)
-        else:
-            # sent only where edited in place since the last exchange, so that a value written through
-            # the handle stands
-            changed = ctypes.c_int()
-            d['_h'].call('mpsw_var_changed', *args, ctypes.byref(changed))
-            if changed.value:
-                d['_h'].call('mpsw_set_var', *args)
-        d['_assigned'].discard(key)
+            routine = 'mpsw_set_var'
+        elif key in d['_assigned']:  # the engine's value, if a routine has written it since, gives way
+            routine = 'mpsw_update_var'
+            d['_assigned'].discard(key)
+        else:  # sent where edited in place, so that a value written through the handle stands
+            routine = 'mpsw_edit_var'
+        d['_h'].call(routine, d['_canon'][key].encode(), ctypes.c_void_p(arr.ctypes.data), arr.size)
 
     def _pull(self, *keys):
         d = self.__dict__

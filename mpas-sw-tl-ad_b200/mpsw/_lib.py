@@ -29,7 +29,7 @@ SIGNATURES = {
     'mpsw_set_var': (_c_int, [_vp, _cp, _vp, _ll]),
     'mpsw_get_var': (_c_int, [_vp, _cp, _vp, _ll]),
     'mpsw_update_var': (_c_int, [_vp, _cp, _vp, _ll]),
-    'mpsw_var_changed': (_c_int, [_vp, _cp, _vp, _ll, ctypes.POINTER(_c_int)]),
+    'mpsw_edit_var': (_c_int, [_vp, _cp, _vp, _ll]),
     'mpsw_get_vars': (_c_int, [_vp, _c_int, ctypes.POINTER(_cp), ctypes.POINTER(_vp), ctypes.POINTER(_ll)]),
     'mpsw_var_allocation': (_c_int, [_vp]),
     'mpsw_var_allocation_tlm': (_c_int, [_vp]),
