@@ -8,10 +8,11 @@
 // three kernels instead of four.  Coefficients are formed once a block in shared memory, before the
 // wait for the previous kernel where the linearisation point is a stored one, and shared by the
 // B / V threads of an entity; a thread holds V members.  The edge passes give a block two
-// neighbouring tiles of edges (the second finds rows of the first in L1: tendency pass 236 -> 214 us when it was measured, without the h' rows),
-// and each kernel is held to the registers at which occupancy and the rows a thread keeps in flight
-// balance.  Level 7, 64 members, cold, us: cells 107, edges 211, tendencies 223 (a tangent-linear stage
-// 524, through the fields 634); edges 189, cells 109, final 249 (adjoint 526, through the fields 671).
+// neighbouring tiles of edges (the second finds rows of the first in L1: the tendency pass, measured
+// without its two h' rows, 236 -> 214 us), and each kernel is held to the registers at which occupancy and
+// the rows a thread keeps in flight balance.  Level 7, 64 members, cold, us: cells 107, edges 211, tendencies
+// 223 (a tangent-linear stage 524, through the fields 634); edges 189, cells 109, final 248 (adjoint 524, through
+// the fields 671).
 #pragma once
 
 #include "mpsw_members.cuh"
